@@ -6,6 +6,7 @@
 #include "b2s_radix.cuh"
 #include "b2s_segsort.cuh"
 #include "b2s_segmerge.cuh"
+#include "b2s_segwarp.cuh"
 
 #include <cstdlib>
 
@@ -337,6 +338,38 @@ inline cudaError_t segmerge_cfg(int xf, const void* in, void* out, int64_t* idx_
   return cudaGetLastError();
 }
 
+// Rows of up to SW_MAX elements: one warp per 32 / group rows.
+template <int KB, bool PAIRS, int VT, int GL>
+inline cudaError_t segwarp_cfg(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
+                               unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+{
+  using K = typename KeyOf<KB>::type;
+  constexpr unsigned long long ROWS = (unsigned long long)SW_WARPS * (32 >> GL);
+  unsigned long long grid = (nseg + ROWS - 1) / ROWS;
+  if (grid > (1ull << 30)) grid = 1ull << 30;
+  {
+    prof::Scope ps(prof::K_SEGSORT, stream);
+    segwarp_kernel<KB, PAIRS, VT, GL><<<(unsigned int)grid, SW_WARPS * 32, 0, stream>>>(
+      static_cast<const K*>(in), static_cast<K*>(out), idx_out, seg_len, nseg, xf, index_offset);
+  }
+  return cudaGetLastError();
+}
+
+template <int KB, bool PAIRS>
+inline cudaError_t segwarp_any(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
+                               unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+{
+  if (seg_len <= 2) return segwarp_cfg<KB, PAIRS, 2, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 4) return segwarp_cfg<KB, PAIRS, 4, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 8) return segwarp_cfg<KB, PAIRS, 8, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 16) return segwarp_cfg<KB, PAIRS, 16, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 32) return segwarp_cfg<KB, PAIRS, 16, 1>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 64) return segwarp_cfg<KB, PAIRS, 16, 2>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 128) return segwarp_cfg<KB, PAIRS, 16, 3>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 256) return segwarp_cfg<KB, PAIRS, 16, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  return segwarp_cfg<KB, PAIRS, 16, 5>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+}
+
 inline bool seg_merge_enabled()
 {
   const char* e = std::getenv("B2S_SEG_MERGE");  // 0: keep every row on the radix kernel (comparisons)
@@ -347,11 +380,26 @@ template <int KB, bool PAIRS>
 inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
                                  unsigned long long nseg, int64_t index_offset, Ctrl* ctrl, cudaStream_t stream)
 {
+  // Short rows go to the warp kernel (2^24 float32 keys with positions, against the one-CTA-per-row radix
+  // kernel they took before: rows of 2 19.2 ms -> 0.09 ms, of 32 1.31 -> 0.16, of 100 0.47 -> 0.22, of 200
+  // 1.42 -> 0.25, of 512 0.34 -> 0.23).  One-byte rows of 65 to 128 stay with the radix kernel, which needs
+  // a single pass for them (0.140 ms against 0.146).
+  // Keys of a sort are mapped back from their images, which the complex64 image does not allow: those
+  // rows are sorted with positions and the keys fetched through them.  So are keys below 4 bytes, whose
+  // words have room for the position anyway.
+  if (KB == 1 && seg_len > 64 && seg_len <= 128)
+    return segsort_cfg<KB, PAIRS, 32, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
+  if (seg_len <= SW_MAX) {
+    if constexpr (PAIRS || KB < 4) {
+      return segwarp_any<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+    } else {
+      if (KB == 8 && xf == XF_CFLOAT) return segwarp_any<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+      return segwarp_any<KB, false>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+    }
+  }
   if constexpr (KB == 4 || KB == 8) {
-    // keys of a sort are mapped back from their images, which the complex64 image does not allow
-    if (seg_len > 256 && (PAIRS || xf != XF_CFLOAT) && seg_merge_enabled()) {
+    if ((PAIRS || xf != XF_CFLOAT) && seg_merge_enabled()) {
       constexpr int V = SM_VT;
-      if (seg_len <= 32 * V) return segmerge_cfg<KB, PAIRS, 32>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
       if (seg_len <= 64 * V) return segmerge_cfg<KB, PAIRS, 64>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
       if (seg_len <= 128 * V) return segmerge_cfg<KB, PAIRS, 128>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
       if (seg_len <= 256 * V) return segmerge_cfg<KB, PAIRS, 256>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
@@ -359,7 +407,6 @@ inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx
       if constexpr (V == 8) return segmerge_cfg<KB, PAIRS, 1024>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
     }
   }
-  if (seg_len <= 128) return segsort_cfg<KB, PAIRS, 32, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
   if (seg_len <= 1024) return segsort_cfg<KB, PAIRS, 128, 8>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
   if (seg_len <= 4096) return segsort_cfg<KB, PAIRS, 256, 16>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
   return segsort_cfg<KB, PAIRS, 512, 16>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);

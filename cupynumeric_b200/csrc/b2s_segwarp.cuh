@@ -1,0 +1,251 @@
+// Segmented sort of short rows (up to 512 elements): a group of 1 to 32 threads of one warp sorts a row, a
+// warp sorts 32 / group rows at a time, and nothing wider than the warp is ever waited for.  Every
+// thread sorts its consecutive elements in registers with Batcher's odd-even merge network (K. E.
+// Batcher, "Sorting networks and their applications", 1968), then log2(group) rounds of merge-path
+// merges run in the warp's own piece of shared memory.
+//
+// Keys travel as words that are ordered like the sort: the order-preserving image, with the element's
+// position below it where positions are wanted (a 4-byte key and its position make one 64-bit word, a
+// shorter key and its position one 32-bit word; 8-byte keys keep 16-bit positions beside them).  The
+// position makes every word of a row unique, so the network, which is not stable, sorts stably.
+//
+// Bound: instruction issue (about 40 thread instructions per key and 64-bit word in the network and the
+// merges of a row of 128), memory for the shortest rows.  A row per CTA, as the radix kernel takes
+// them, leaves a short row's CTA waiting for its barriers and four counting passes: 2^24 float32 keys
+// with positions in rows of 100 took 0.468 ms there, 0.220 ms here; float64 rows of 200 3.05 ms, 0.31 ms.
+// 16 elements per thread: the network costs 4 comparators per element, a merge round about 13
+// instructions, and 16 words are what the registers of 28 warps per SM hold.
+#pragma once
+
+#include "b2s_common.cuh"
+#include "b2s_segmerge.cuh"
+
+namespace b2s {
+
+constexpr int SW_WARPS         = 4;    // warps per CTA, independent of each other
+constexpr unsigned int SW_MAX  = 512;  // longest row: 32 threads of 16 elements
+
+template <int KB, bool PAIRS> struct SegWarpWord {
+  static constexpr bool PACK = PAIRS && KB < 8;
+  static constexpr bool SIDE = PAIRS && KB == 8;
+  static constexpr int BYTES = (KB == 8 || (PACK && KB == 4)) ? 8 : 4;
+  static constexpr int SHIFT = KB == 4 ? 32 : 16;  // PACK: the image sits above this many bits of position
+  using type                 = typename SmWord<BYTES>::type;
+};
+
+// Batcher's odd-even merge sort of N (a power of two) elements; less(i, j) orders elements i and j,
+// swap(i, j) exchanges them.
+template <int N, typename CmpSwap>
+__device__ __forceinline__ void odd_even_merge_sort(CmpSwap cmp_swap)
+{
+#pragma unroll
+  for (int p = 1; p < N; p <<= 1) {
+#pragma unroll
+    for (int k = p; k >= 1; k >>= 1) {
+#pragma unroll
+      for (int j = 0; j + k < N; ++j) {
+        // j is the lower end of a comparator where it lies in the lower half of a block of 2k that
+        // starts k % p after a multiple of 2k, and both ends lie in the same block of 2p
+        const int off = j - k % p;
+        if (off >= 0 && off % (2 * k) < k && j / (2 * p) == (j + k) / (2 * p)) cmp_swap(j, j + k);
+      }
+    }
+  }
+}
+
+// A warp sorts 32 >> GL rows at a time, 1 << GL threads of VT elements per row; seg_len <= VT << GL.
+// idx_out and out may each be null (not both).
+template <int KB, bool PAIRS, int VT, int GL>
+__global__ void __launch_bounds__(SW_WARPS * 32, KB == 8 ? (PAIRS ? 4 : 6) : PAIRS ? 7 : 8)
+segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out,
+               int64_t* idx_out, unsigned int seg_len, unsigned long long nseg, int xf, int64_t index_offset)
+{
+  using K  = typename KeyOf<KB>::type;
+  using WD = SegWarpWord<KB, PAIRS>;
+  using W  = typename WD::type;
+  constexpr bool PACK = WD::PACK, SIDE = WD::SIDE;
+  constexpr int G = 1 << GL, RT = G * VT, ROWS = 32 / G;
+  constexpr int SPAN = 32 * (VT + 1);  // one spare word per thread: blocked accesses hit all banks
+  constexpr W WMAX   = (W)~(W)0;
+  __shared__ W sw_all[SW_WARPS * SPAN];
+  __shared__ unsigned short sp_all[SIDE ? SW_WARPS * SPAN : 1];
+
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g    = lane & (G - 1);          // my place in the row's group
+  W* sw              = sw_all + warp * SPAN;
+  unsigned short* sp = sp_all + (SIDE ? warp * SPAN : 0);
+  auto at = [](int i) { return i + i / VT; };  // shared-memory index of a position of the warp's rows
+  const int mine = lane * (VT + 1);
+  const int row0 = (lane >> GL) * RT;          // first position of my row
+  const bool gather = PAIRS && (KB >= 4 || xf == XF_FLOAT);  // keys come back through the positions
+
+  const unsigned long long nblk = (nseg + ROWS - 1) / ROWS;
+  for (unsigned long long blk = (unsigned long long)blockIdx.x * SW_WARPS + warp; blk < nblk;
+       blk += (unsigned long long)gridDim.x * SW_WARPS) {
+    const unsigned long long base = blk * ROWS;
+    const int rows = (int)(nseg - base < (unsigned long long)ROWS ? nseg - base : ROWS);
+    const K* src   = in + base * seg_len;
+    // ---- load: consecutive lanes read consecutive elements ----
+    int special = 0;
+#pragma unroll
+    for (int j = 0; j < VT; ++j) {
+      const int i = j * 32 + lane, r = i / RT, c = i % RT;
+      W w = WMAX;
+      if (r < rows && (unsigned int)c < seg_len) {
+        const K raw = src[r * seg_len + c];
+        if (!PAIRS) special |= sm_is_special<KB>(raw, xf) ? 1 : 0;
+        const K o = to_ordered_rt<KB>(raw, xf);
+        w         = PACK ? (W)(((W)o << (PACK ? WD::SHIFT : 0)) | (W)(unsigned int)c) : (W)o;
+      }
+      sw[at(i)] = w;
+    }
+    if (!PAIRS) special = __any_sync(0xFFFFFFFFu, special);
+    __syncwarp();
+    W key[VT];
+    unsigned int pay[SIDE ? VT : 1];
+#pragma unroll
+    for (int j = 0; j < VT; ++j) {
+      key[j] = sw[mine + j];
+      if (SIDE) pay[j] = g * VT + j;
+    }
+    // ---- my elements in registers ----
+    odd_even_merge_sort<VT>([&](int a, int b) {
+      const W x = key[a], y = key[b];
+      if (SIDE) {
+        const unsigned int p = pay[SIDE ? a : 0], q = pay[SIDE ? b : 0];
+        const bool sw_ = y < x || (y == x && q < p);
+        key[a] = sw_ ? y : x;
+        key[b] = sw_ ? x : y;
+        pay[SIDE ? a : 0] = sw_ ? q : p;
+        pay[SIDE ? b : 0] = sw_ ? p : q;
+      } else {
+        const bool sw_ = y < x;
+        key[a] = sw_ ? y : x;
+        key[b] = sw_ ? x : y;
+      }
+    });
+    // ---- merge rounds: runs of `run` elements, pairwise; my VT outputs start at g * VT of the row ----
+#pragma unroll 1
+    for (int run = VT; run < RT; run <<= 1) {
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        sw[mine + j] = key[j];
+        if (SIDE) sp[mine + j] = (unsigned short)pay[SIDE ? j : 0];
+      }
+      __syncwarp();
+      const int first = g * VT, pbase = first & ~(2 * run - 1), diag = first - pbase;
+      const int a0 = row0 + pbase, b0 = a0 + run;
+      int lo = max(0, diag - run), hi = min(diag, run);
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (sw[at(a0 + mid)] <= sw[at(b0 + diag - 1 - mid)]) lo = mid + 1; else hi = mid;
+      }
+      int ia = lo, ib = diag - lo;
+      W ka = ia < run ? sw[at(a0 + ia)] : WMAX, kb = ib < run ? sw[at(b0 + ib)] : WMAX;
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        // an exhausted run never wins; on equal words the lower run goes first
+        const bool take_a = ib >= run || (ia < run && ka <= kb);
+        key[j]            = take_a ? ka : kb;
+        if (SIDE) pay[SIDE ? j : 0] = sp[at(take_a ? a0 + ia : b0 + ib)];
+        ia += take_a ? 1 : 0;
+        ib += take_a ? 0 : 1;
+        const bool ok = take_a ? ia < run : ib < run;
+        const W v     = ok ? sw[at(take_a ? a0 + ia : b0 + ib)] : WMAX;
+        ka = take_a ? v : ka;
+        kb = take_a ? kb : v;
+      }
+    }
+    __syncwarp();
+    // ---- results into shared memory, from there to memory with consecutive lanes on consecutive elements ----
+    if (!PAIRS) {
+#pragma unroll
+      for (int j = 0; j < VT; ++j) sw[mine + j] = (W)sm_from_ordered<KB>((K)key[j], xf);
+      if (special) {
+        // some row of the warp holds a -0.0 or an unusual NaN, which the images fold: zeros and NaNs are
+        // written again from the input, in input order
+        const W zimg = (W)to_ordered_rt<KB>((K)0, xf);
+        unsigned int z0 = 0, n0 = 0, cz = 0, cn = 0;
+        K raw[VT];
+#pragma unroll
+        for (int j = 0; j < VT; ++j) {
+          z0 += key[j] < zimg ? 1u : 0u;
+          n0 += key[j] < WMAX ? 1u : 0u;
+          const int c = g * VT + j;
+          raw[j]      = (lane >> GL) < rows && (unsigned int)c < seg_len ? src[(lane >> GL) * seg_len + c] : (K)1;
+          cz += sm_is_zero<KB>(raw[j]) ? 1u : 0u;
+          cn += sm_is_nan<KB>(raw[j]) ? 1u : 0u;
+        }
+        const unsigned int start = z0 | (n0 << 16), count = cz | (cn << 16);
+        unsigned int total = start, before = count;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+          total += __shfl_xor_sync(0xFFFFFFFFu, total, o, G);
+          const unsigned int t = __shfl_up_sync(0xFFFFFFFFu, before, o, G);
+          if (g >= o) before += t;
+        }
+        before -= count;
+        int rz = (int)((total & 0xFFFFu) + (before & 0xFFFFu)), rn = (int)((total >> 16) + (before >> 16));
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < VT; ++j) {
+          if (sm_is_zero<KB>(raw[j])) sw[at(row0 + rz++)] = (W)raw[j];
+          if (sm_is_nan<KB>(raw[j])) sw[at(row0 + rn++)] = (W)raw[j];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        if (SIDE) sp[mine + j] = (unsigned short)pay[SIDE ? j : 0];
+        else sw[mine + j] = key[j];
+      }
+    }
+    __syncwarp();
+    K* dst = out != nullptr ? out + base * seg_len : nullptr;
+    if (!PAIRS) {
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        const int i = j * 32 + lane, r = i / RT, c = i % RT;
+        if (r < rows && (unsigned int)c < seg_len) dst[r * seg_len + c] = (K)sw[at(i)];
+      }
+    } else {
+      unsigned int pos[VT];
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        const int i = j * 32 + lane;
+        pos[j]      = SIDE ? (unsigned int)sp[at(i)] : (unsigned int)sw[at(i)];
+      }
+      if (dst != nullptr) {
+        // all keys of the warp's rows are read before any is written: the output may be the input
+        K raw[VT];
+#pragma unroll
+        for (int j = 0; j < VT; ++j) {
+          const int i = j * 32 + lane, r = i / RT, c = i % RT;
+          if (r < rows && (unsigned int)c < seg_len) {
+            if (gather) raw[j] = src[r * seg_len + (KB == 4 || SIDE ? pos[j] : (pos[j] & 0xFFFFu))];
+            else raw[j] = sm_from_ordered<KB>((K)(pos[j] >> 16), xf);
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < VT; ++j) {
+          const int i = j * 32 + lane, r = i / RT, c = i % RT;
+          if (r < rows && (unsigned int)c < seg_len) dst[r * seg_len + c] = raw[j];
+        }
+      }
+      if (idx_out != nullptr) {
+        int64_t* idst = idx_out + base * seg_len;
+#pragma unroll
+        for (int j = 0; j < VT; ++j) {
+          const int i = j * 32 + lane, r = i / RT, c = i % RT;
+          if (r < rows && (unsigned int)c < seg_len)
+            idst[r * seg_len + c] = (int64_t)(KB >= 4 ? pos[j] : (pos[j] & 0xFFFFu)) + index_offset;
+        }
+      }
+    }
+    __syncwarp();  // all reads of shared memory are done before the next rows' load
+  }
+}
+
+}  // namespace b2s
