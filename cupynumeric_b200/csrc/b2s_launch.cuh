@@ -370,6 +370,17 @@ inline cudaError_t segwarp_any(int xf, const void* in, void* out, int64_t* idx_o
   return segwarp_cfg<KB, PAIRS, 16, 5>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
 }
 
+template <int KB, bool PAIRS>
+inline cudaError_t segmerge_any(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
+                                unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+{
+  constexpr int V = SM_VT;
+  if (seg_len <= 64 * V) return segmerge_cfg<KB, PAIRS, 64>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 128 * V) return segmerge_cfg<KB, PAIRS, 128>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 256 * V) return segmerge_cfg<KB, PAIRS, 256>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  return segmerge_cfg<KB, PAIRS, 512>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+}
+
 inline bool seg_merge_enabled()
 {
   const char* e = std::getenv("B2S_SEG_MERGE");  // 0: keep every row on the radix kernel (comparisons)
@@ -398,13 +409,10 @@ inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx
     }
   }
   if constexpr (KB == 4 || KB == 8) {
-    if ((PAIRS || xf != XF_CFLOAT) && seg_merge_enabled()) {
-      constexpr int V = SM_VT;
-      if (seg_len <= 64 * V) return segmerge_cfg<KB, PAIRS, 64>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-      if (seg_len <= 128 * V) return segmerge_cfg<KB, PAIRS, 128>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-      if (seg_len <= 256 * V) return segmerge_cfg<KB, PAIRS, 256>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-      if (seg_len <= 512 * V) return segmerge_cfg<KB, PAIRS, 512>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-      if constexpr (V == 8) return segmerge_cfg<KB, PAIRS, 1024>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+    if (seg_merge_enabled()) {
+      if constexpr (!PAIRS && KB == 8)
+        if (xf == XF_CFLOAT) return segmerge_any<KB, true>(xf, in, out, nullptr, seg_len, nseg, index_offset, stream);
+      return segmerge_any<KB, PAIRS>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
     }
   }
   if (seg_len <= 1024) return segsort_cfg<KB, PAIRS, 128, 8>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);

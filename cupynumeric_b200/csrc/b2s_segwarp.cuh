@@ -1,8 +1,7 @@
 // Segmented sort of short rows (up to 512 elements): a group of 1 to 32 threads of one warp sorts a row, a
 // warp sorts 32 / group rows at a time, and nothing wider than the warp is ever waited for.  Every
-// thread sorts its consecutive elements in registers with Batcher's odd-even merge network (K. E.
-// Batcher, "Sorting networks and their applications", 1968), then log2(group) rounds of merge-path
-// merges run in the warp's own piece of shared memory.
+// thread sorts its consecutive elements in registers with Batcher's odd-even merge network,
+// then log2(group) rounds of merge-path merges run in the warp's own piece of shared memory.
 //
 // Keys travel as words that are ordered like the sort: the order-preserving image, with the element's
 // position below it where positions are wanted (a 4-byte key and its position make one 64-bit word, a
@@ -32,26 +31,6 @@ template <int KB, bool PAIRS> struct SegWarpWord {
   static constexpr int SHIFT = KB == 4 ? 32 : 16;  // PACK: the image sits above this many bits of position
   using type                 = typename SmWord<BYTES>::type;
 };
-
-// Batcher's odd-even merge sort of N (a power of two) elements; less(i, j) orders elements i and j,
-// swap(i, j) exchanges them.
-template <int N, typename CmpSwap>
-__device__ __forceinline__ void odd_even_merge_sort(CmpSwap cmp_swap)
-{
-#pragma unroll
-  for (int p = 1; p < N; p <<= 1) {
-#pragma unroll
-    for (int k = p; k >= 1; k >>= 1) {
-#pragma unroll
-      for (int j = 0; j + k < N; ++j) {
-        // j is the lower end of a comparator where it lies in the lower half of a block of 2k that
-        // starts k % p after a multiple of 2k, and both ends lie in the same block of 2p
-        const int off = j - k % p;
-        if (off >= 0 && off % (2 * k) < k && j / (2 * p) == (j + k) / (2 * p)) cmp_swap(j, j + k);
-      }
-    }
-  }
-}
 
 // A warp sorts 32 >> GL rows at a time, 1 << GL threads of VT elements per row; seg_len <= VT << GL.
 // idx_out and out may each be null (not both).
@@ -109,7 +88,7 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
       if (SIDE) pay[j] = g * VT + j;
     }
     // ---- my elements in registers ----
-    odd_even_merge_sort<VT>([&](int a, int b) {
+    odd_even_merge_sort<VT, 1>([&](int a, int b) {
       const W x = key[a], y = key[b];
       if (SIDE) {
         const unsigned int p = pay[SIDE ? a : 0], q = pay[SIDE ? b : 0];

@@ -39,3 +39,50 @@ def test_short_complex_rows(cuda_device):
         assert_bit_equal(out, a[np.arange(37).repeat(seg) * seg + idx], f"sort 37x{seg}")
         _, got = cabi_local_sort(a, seg, True, ndim_is_1=False)
         assert np.array_equal(got, idx), f"argsort 37x{seg}"
+
+
+def _long_rows(rng, dtype, nseg, seg, how):
+    """Rows by how their keys spread: evenly, by a bell curve with special values, with one far outlier,
+    over a handful of values, or in a narrow cluster far from zero."""
+    dt, n = np.dtype(dtype), nseg * seg
+    if how == "full":
+        return random_keys(rng, dt, n, "full")
+    if how == "few":
+        return random_keys(rng, dt, n, "small")
+    x = rng.standard_normal(n)
+    if how == "outlier":
+        x[::seg] = 1e6
+    if dt.kind == "f":
+        a = (x + (1e5 if how == "cluster" else 0.0)).astype(dt)
+        if how == "bell":
+            for v in (np.nan, -np.nan, np.inf, -np.inf, -0.0, 0.0):
+                a[rng.integers(0, n, n // 300)] = v
+        return a
+    a = np.round(x * 50_000).astype(np.int64)
+    return (a + (1 << 30) if how == "cluster" else np.abs(a)).astype(dt)
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.uint32, np.float32, np.int64, np.float64])
+@pytest.mark.parametrize("how", ["full", "bell", "outlier", "few", "cluster"])
+def test_rows_of_one_block(cuda_device, dtype, how):
+    rng = np.random.default_rng(9)
+    for seg in (513, 1000, 1024, 1025, 2047, 2048, 2049, 4096, 4097, 8191, 8192):
+        a = _long_rows(rng, dtype, 5, seg, how)
+        if a.dtype.kind == "f":
+            a[seg:2 * seg] = np.nan if how == "few" else 2.5   # a row of one value
+        idx = np_task_sort(a, seg, True, 0, False)
+        want = a[np.arange(5).repeat(seg) * seg + idx]
+        out, _ = cabi_local_sort(a, seg, False, ndim_is_1=False)
+        assert_bit_equal(out, want, f"sort {dtype} {how} 5x{seg}")
+        out, got = cabi_local_sort(a, seg, True, ndim_is_1=False, want_keys_too=True, inplace=True)
+        assert np.array_equal(got, idx), f"argsort {dtype} {how} 5x{seg}"
+        assert_bit_equal(out, want, f"keys beside the indices {dtype} {how} 5x{seg}")
+
+
+def test_complex_rows_of_one_block(cuda_device):
+    rng = np.random.default_rng(10)
+    for seg in (600, 2000, 4097):
+        a = (np.round(rng.standard_normal(5 * seg), 2) + 1j * rng.standard_normal(5 * seg)).astype(np.complex64)
+        idx = complex_lex_argsort(a, seg)
+        out, _ = cabi_local_sort(a, seg, False, ndim_is_1=False)
+        assert_bit_equal(out, a[np.arange(5).repeat(seg) * seg + idx], f"sort 5x{seg}")
