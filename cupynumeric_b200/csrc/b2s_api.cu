@@ -334,7 +334,7 @@ __global__ void selftest_fill_kernel(uint32_t* keys, unsigned int n)
 
 int b2s_selftest_wait_timeout(void* ws, size_t ws_bytes, void* cuda_stream)
 {
-  constexpr unsigned int N = 1u << 16;  // a dozen tiles
+  constexpr unsigned int N = 1u << 16;  // 32 small tiles
   const auto lay           = radix_1d_layout<4>(N, false);
   const size_t need        = lay.total + 2 * (size_t)N * 4;
   if (ws == nullptr || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u) != 0) return B2S_ERR_WORKSPACE;
@@ -361,7 +361,7 @@ int b2s_selftest_wait_timeout(void* ws, size_t ws_bytes, void* cuda_stream)
   if (cudaMemcpyAsync(&ctrl->tile_counter[0], &one, 4, cudaMemcpyHostToDevice, stream) != cudaSuccess) return B2S_ERR_CUDA;
   if (cudaMemcpyAsync(&ctrl->spin_limit, &limit, 4, cudaMemcpyHostToDevice, stream) != cudaSuccess) return B2S_ERR_CUDA;
   const SegGeom geo{N, lay.tiles, 1u, 4, nullptr};
-  const cudaError_t e = launch_sweeps<4, XF_UNSIGNED, false>(ctrl, lb, lay.tiles, geo, 0, stream);
+  const cudaError_t e = launch_sweeps<4, XF_UNSIGNED, false, SWEEP_SMALL>(ctrl, lb, lay.tiles, geo, 0, stream);
   return e == cudaSuccess ? B2S_OK : B2S_ERR_CUDA;
 }
 

@@ -9,69 +9,49 @@
 #include "b2s_segwarp.cuh"
 
 #include <cstdlib>
+#include <type_traits>
 
 namespace b2s {
 
 // Largest segment the on-chip segmented kernel takes.
 constexpr unsigned int SEG_CAP = 8192;
 
-// Tile shape of the onesweep pass per key width / payload.
-// Tile shapes found by sweeps on B200 (2^28 keys): more keys per thread amortise the per-tile
-// work (counter zeroing, row scan, look-back); pairs run three CTAs per SM.
-// -DB2S_CFG_<group>_{THREADS,ITEMS,MINCTAS} override a group for tuning sweeps; groups are
-// K4 (keys only, <= 4-byte keys), K8 (keys only, 8-byte keys), P4 / P8 (key + index).
-#ifndef B2S_CFG_CHAINS
-#define B2S_CFG_CHAINS 1
-#endif
-#ifndef B2S_CFG_K4_THREADS
-#define B2S_CFG_K4_THREADS 256
-#endif
-#ifndef B2S_CFG_K4_ITEMS
-#define B2S_CFG_K4_ITEMS 20
-#endif
-#ifndef B2S_CFG_K4_MINCTAS
-#define B2S_CFG_K4_MINCTAS 4
-#endif
-#ifndef B2S_CFG_K8_THREADS
-#define B2S_CFG_K8_THREADS 256
-#endif
-#ifndef B2S_CFG_K8_ITEMS
-#define B2S_CFG_K8_ITEMS 28
-#endif
-#ifndef B2S_CFG_K8_MINCTAS
-#define B2S_CFG_K8_MINCTAS 3
-#endif
-#ifndef B2S_CFG_P4_THREADS
-#define B2S_CFG_P4_THREADS 256
-#endif
-#ifndef B2S_CFG_P4_ITEMS
-#define B2S_CFG_P4_ITEMS 32
-#endif
-#ifndef B2S_CFG_P4_MINCTAS
-#define B2S_CFG_P4_MINCTAS 3
-#endif
-#ifndef B2S_CFG_P8_THREADS
-#define B2S_CFG_P8_THREADS 256
-#endif
-#ifndef B2S_CFG_P8_ITEMS
-#define B2S_CFG_P8_ITEMS 20
-#endif
-#ifndef B2S_CFG_P8_MINCTAS
-#define B2S_CFG_P8_MINCTAS 3
-#endif
-template <int KB, bool PAIRS> struct SweepCfg {
-  static constexpr int THREADS = PAIRS ? (KB == 8 ? B2S_CFG_P8_THREADS : B2S_CFG_P4_THREADS)
-                                       : (KB == 8 ? B2S_CFG_K8_THREADS : B2S_CFG_K4_THREADS);
-  static constexpr int ITEMS   = PAIRS ? (KB == 8 ? B2S_CFG_P8_ITEMS : B2S_CFG_P4_ITEMS)
-                                       : (KB == 8 ? B2S_CFG_K8_ITEMS : B2S_CFG_K4_ITEMS);
-  static constexpr int MINCTAS = PAIRS ? (KB == 8 ? B2S_CFG_P8_MINCTAS : B2S_CFG_P4_MINCTAS)
-                                       : (KB == 8 ? B2S_CFG_K8_MINCTAS : B2S_CFG_K4_MINCTAS);
-  static constexpr int CHAINS  = B2S_CFG_CHAINS;
+// Tile shapes of the onesweep pass: threads, keys per thread, CTAs per SM and look-back window by key
+// width, payload and size class, found by sweeps on B200.
+//
+// Short arrays (1-D sorts of up to SMALL_MAX keys) take small tiles: with the others 10^5 keys are 13 to 20
+// tiles on 148 SMs, and a pass lasts as long as one tile's chain of loading, ranking and looking back.
+// Their walks read 16 entries per round trip, since most tiles run at once and few prefixes are ready.
+// Measured, medium -> small tiles: float32 argsort of 20000 116 -> 63 us, of 100003 106 -> 65, of 400000 122 ->
+// 73; int64 argsort of 20000 169 -> 110 us; int32 sort of 400000 73 -> 67; at 2^20 keys the medium tiles win
+// (float32 argsort 95 against 124 us).  4 keys per thread lose to 8 from 4-byte keys on, 12 at the short end.
+//
+// Long arrays (1-D sorts of more than MEDIUM_MAX keys), medium -> large tiles: int32 sort of 2^28 4.94 -> 4.71
+// ms (24 keys per thread amortise the work per tile better), float16 sort of 2^27 1.66 -> 1.54 (384
+// threads), int64 sort of 2^28 Zipf keys 7.45 -> 7.33 and float64 sort of 2^27 6.52 -> 6.24 (20 keys leave
+// the registers of a fourth CTA per SM), int64 argsort of 2^27 7.67 -> 7.44 (longer digit runs).  The border
+// is where the scratch of b2s_local_sort_noalloc ends: the smaller tiles need a larger look-back table,
+// and what fits that scratch has to go on fitting.  Segments keep the medium tiles, whose last tile wastes least.
+enum : int { SWEEP_SMALL = 0, SWEEP_MEDIUM = 1, SWEEP_LARGE = 2 };
+constexpr size_t SMALL_TILE = 256 * 8;
+constexpr size_t SMALL_MAX  = 240 * SMALL_TILE;
+constexpr size_t MEDIUM_MAX = (size_t)1 << 21;
+template <int KB, bool PAIRS, int SIZE = SWEEP_MEDIUM> struct SweepCfg {
+  static constexpr bool LARGE  = SIZE == SWEEP_LARGE && !(PAIRS && KB < 8);
+  static constexpr int THREADS = SIZE == SWEEP_SMALL || !LARGE ? 256 : PAIRS ? 512 : KB == 2 ? 384 : 256;
+  static constexpr int ITEMS   = SIZE == SWEEP_SMALL ? (int)(SMALL_TILE / 256)
+                               : LARGE               ? (PAIRS ? 14 : KB == 8 || KB == 2 ? 20 : 24)
+                                                     : (PAIRS ? (KB == 8 ? 20 : 32) : (KB == 8 ? 28 : 20));
+  static constexpr int MINCTAS = SIZE == SWEEP_SMALL ? 4
+                               : LARGE               ? (PAIRS ? 2 : KB == 2 ? 3 : 4)
+                                                     : (PAIRS ? 3 : (KB == 8 ? 3 : 4));
+  static constexpr int CHAINS  = 1;
   static constexpr int TILE    = THREADS * ITEMS;
+  static constexpr int WINDOW  = SIZE == SWEEP_SMALL ? 16 : LB_WINDOW;
 };
 
 struct Radix1dLayout {
-  size_t off_lookback, off_keys[2], off_idx[2], total;
+  size_t off_lookback, lookback_used, off_keys[2], off_idx[2], total;
   unsigned int tiles;
 };
 
@@ -79,11 +59,21 @@ template <int KB>
 inline Radix1dLayout radix_1d_layout(size_t n, bool pairs)
 {
   Radix1dLayout l{};
-  const unsigned int tile = pairs ? SweepCfg<KB, true>::TILE : SweepCfg<KB, false>::TILE;
-  l.tiles                 = (unsigned int)((n + tile - 1) / tile);
-  size_t off              = align_up(sizeof(Ctrl), 256);
-  l.off_lookback          = off;
-  off += align_up((size_t)KB * l.tiles * RADIX * sizeof(unsigned int), 256);
+  const size_t small = SMALL_TILE, medium = pairs ? SweepCfg<KB, true>::TILE : SweepCfg<KB, false>::TILE,
+               large = pairs ? SweepCfg<KB, true, SWEEP_LARGE>::TILE : SweepCfg<KB, false, SWEEP_LARGE>::TILE;
+  auto tiles_of = [&](size_t m) {
+    const size_t tile = m <= SMALL_MAX ? small : m <= MEDIUM_MAX ? medium : large;
+    return (m + tile - 1) / tile;
+  };
+  l.tiles = (unsigned int)tiles_of(n);
+  // room for the table of every shorter sort too, so that a workspace serves any length below its own
+  size_t rows = tiles_of(n);
+  if (n > SMALL_MAX && tiles_of(SMALL_MAX) > rows) rows = tiles_of(SMALL_MAX);
+  if (n > MEDIUM_MAX && tiles_of(MEDIUM_MAX) > rows) rows = tiles_of(MEDIUM_MAX);
+  size_t off           = align_up(sizeof(Ctrl), 256);
+  l.off_lookback       = off;
+  l.lookback_used      = align_up((size_t)KB * l.tiles * RADIX * sizeof(unsigned int), 256);
+  off += align_up((size_t)KB * rows * RADIX * sizeof(unsigned int), 256);
   for (int i = 0; i < 2; ++i) {
     l.off_keys[i] = off;
     off += align_up(n * KB, 256);
@@ -96,13 +86,13 @@ inline Radix1dLayout radix_1d_layout(size_t n, bool pairs)
   return l;
 }
 
-template <int KB, int XF, bool PAIRS>
+template <int KB, int XF, bool PAIRS, int SIZE = SWEEP_MEDIUM>
 inline cudaError_t launch_sweeps(Ctrl* ctrl, unsigned int* lookback, unsigned int tiles, SegGeom geo,
                                  int64_t index_offset, cudaStream_t stream)
 {
-  using C   = SweepCfg<KB, PAIRS>;
+  using C   = SweepCfg<KB, PAIRS, SIZE>;
   using S   = SweepSmem<KB, PAIRS, C::THREADS, C::ITEMS, C::CHAINS>;
-  auto kern = onesweep_kernel<KB, XF, PAIRS, C::THREADS, C::ITEMS, C::CHAINS, C::MINCTAS>;
+  auto kern = onesweep_kernel<KB, XF, PAIRS, C::THREADS, C::ITEMS, C::CHAINS, C::MINCTAS, C::WINDOW>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::BYTES);
   if (e != cudaSuccess) return e;
   for (int pass = 0; pass < KB; ++pass) {
@@ -129,7 +119,7 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
   unsigned int* lb   = reinterpret_cast<unsigned int*>(ws + lay.off_lookback);
   // control block; the look-back tables too unless the histogram kernel clears them
   const bool own_hist = hist_parts == nullptr;
-  cudaError_t e       = cudaMemsetAsync(ws, 0, own_hist ? lay.off_lookback : lay.off_keys[0], stream);
+  cudaError_t e       = cudaMemsetAsync(ws, 0, lay.off_lookback + (own_hist ? 0 : lay.lookback_used), stream);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -151,7 +141,7 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
   ra.npass       = KB;
   ra.key_bytes   = KB;
   ra.zero_ptr    = own_hist ? reinterpret_cast<uint4*>(ws + lay.off_lookback) : nullptr;
-  ra.zero_vecs   = own_hist ? (lay.off_keys[0] - lay.off_lookback) / 16 : 0;
+  ra.zero_vecs   = own_hist ? lay.lookback_used / 16 : 0;
   if (hist_parts != nullptr) {
     // the histograms were counted elsewhere (by the ranks that sent this GPU its keys)
     prof::Scope ps(prof::K_SCAN, stream);
@@ -172,8 +162,14 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
     hist_kernel<KB, XF><<<hgrid, HIST_THREADS, 0, stream>>>(static_cast<const K*>(in), n, ctrl, ra);
   }
   const SegGeom geo{n, lay.tiles, 1u, KB, nullptr};
-  e = pairs ? launch_sweeps<KB, XF, true>(ctrl, lb, lay.tiles, geo, index_offset, stream)
-            : launch_sweeps<KB, XF, false>(ctrl, lb, lay.tiles, geo, index_offset, stream);
+  auto sweeps = [&](auto size) {
+    constexpr int SIZE = decltype(size)::value;
+    return pairs ? launch_sweeps<KB, XF, true, SIZE>(ctrl, lb, lay.tiles, geo, index_offset, stream)
+                 : launch_sweeps<KB, XF, false, SIZE>(ctrl, lb, lay.tiles, geo, index_offset, stream);
+  };
+  e = n <= SMALL_MAX    ? sweeps(std::integral_constant<int, SWEEP_SMALL>{})
+      : n <= MEDIUM_MAX ? sweeps(std::integral_constant<int, SWEEP_MEDIUM>{})
+                        : sweeps(std::integral_constant<int, SWEEP_LARGE>{});
   if (e != cudaSuccess) return e;
   unsigned int fgrid = (n + 256 * 16 - 1) / (256 * 16);
   if (fgrid > (unsigned int)sms * 8) fgrid = sms * 8;

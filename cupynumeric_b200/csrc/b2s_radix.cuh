@@ -423,10 +423,56 @@ constexpr unsigned int LB_FLAG_AGG  = 1u << 30;  // tile count published
 constexpr unsigned int LB_FLAG_INCL = 2u << 30;  // inclusive prefix published
 constexpr unsigned int LB_VALUE     = (1u << 30) - 1;
 constexpr unsigned int MAX_N_1D     = 1u << 30;  // counts must fit 30 bits
-#ifndef B2S_CFG_LB_WINDOW
-#define B2S_CFG_LB_WINDOW 4
-#endif
-constexpr int LB_WINDOW             = B2S_CFG_LB_WINDOW;  // predecessors inspected per round trip
+constexpr int LB_WINDOW             = 4;         // predecessors inspected per round trip
+
+// Decoupled look-back of one thread for one digit: adds up the predecessors' entries from `entry` (the
+// tile before the caller's) downwards until one holds an inclusive prefix; the segment's first tile
+// always does, so the walk never leaves the segment.  WINDOW entries are loaded per round trip: the
+// loads are independent, so a run of tiles that have only published their counts costs one memory
+// latency per window.  A window may reach beyond the segment's first tile, `left` entries further down: it
+// then reads what lies in front (another segment's or pass's entries, or the control block, which is as
+// large as a short window), never to be counted; a longer window reads the first tile's entry again.
+// The walk is on the critical path of every tile, and its instructions cost more of that than its loads:
+// hence the straight-line form (2^28 float32 argsort 5.92 -> 5.84 ms, Zipf int64 sort 7.50 -> 7.38 against a
+// branch per entry; windows of 8 and 16 were slower on long arrays).
+// Returns false when the poll limit ran out.
+static_assert(sizeof(Ctrl) >= (LB_WINDOW - 1) * RADIX * sizeof(unsigned int), "a short window may read the control block");
+template <int WINDOW>
+__device__ __forceinline__ bool look_back(const Ctrl* ctrl, const unsigned int* entry, int left, unsigned int* excl_out)
+{
+  unsigned int excl  = 0;
+  unsigned int spins = 0, spin_cap = SPIN_LIMIT;
+  bool ok            = true;
+  while (true) {
+    unsigned int v[WINDOW];
+#pragma unroll
+    for (int j = 0; j < WINDOW; ++j) v[j] = ld_relaxed(entry - (WINDOW > LB_WINDOW ? min(j, left) : j) * RADIX);
+    bool go             = true;   // no gap and no inclusive entry so far
+    bool done           = false;
+    int used            = 0;
+#pragma unroll
+    for (int j = 0; j < WINDOW; ++j) {
+      const bool take = go && v[j] != 0;   // (an entry without a flag is all zero)
+      excl += take ? v[j] & LB_VALUE : 0u;
+      used += take ? 1 : 0;
+      done = done || (take && (int)v[j] < 0);
+      go   = take && (int)v[j] >= 0;
+    }
+    if (done) break;
+    entry -= used * RADIX;
+    if (WINDOW > LB_WINDOW) left -= used;
+    if (used == 0) {
+      if (spins == 0 && ctrl->spin_limit != 0) spin_cap = ctrl->spin_limit;
+      if (++spins > spin_cap || ((spins & 1023u) == 0 && ld_relaxed(&ctrl->abort))) {
+        ok = false;
+        break;
+      }
+      if (spins > 4) __nanosleep(64);  // leave the issue slots to the other CTAs of the SM
+    }
+  }
+  *excl_out = excl;
+  return ok;
+}
 
 template <int KB, bool PAIRS, int THREADS, int ITEMS, int CHAINS>
 struct SweepSmem {
@@ -458,7 +504,7 @@ struct SegGeom {
   const unsigned int* seg_bases;  // [nseg][npass][RADIX] exclusive digit bases, or null
 };
 
-template <int KB, int XF, bool PAIRS, int THREADS, int ITEMS, int CHAINS, int MIN_CTAS>
+template <int KB, int XF, bool PAIRS, int THREADS, int ITEMS, int CHAINS, int MIN_CTAS, int WINDOW>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS)
 onesweep_kernel(Ctrl* ctrl, unsigned int* __restrict__ lookback, int pass, SegGeom geo, int64_t index_offset)
 {
@@ -671,49 +717,13 @@ onesweep_kernel(Ctrl* ctrl, unsigned int* __restrict__ lookback, int pass, SegGe
     for (int i = 0; i < ITEMS; ++i) stage_vals[pos[i]] = val[i];
   }
 
-  // ---- chained prefix over tiles (decoupled look-back), one thread per digit ----
+  // ---- chained prefix over tiles (decoupled look-back).  It runs this late so that most
+  // predecessors have published by then and the walk rarely has to poll ----
   if (tid < RADIX) {
     unsigned int excl = 0;
     if (t_in != 0) {
-      // Walk back over the predecessors (the segment's first tile always holds an inclusive
-      // prefix, so the walk never leaves the segment), LB_WINDOW of them per round trip: the loads of one
-      // window are independent, so a run of tiles that have only published their counts costs
-      // one memory latency per window instead of one per tile.
-      int t              = (int)tile - 1;
-      unsigned int spins = 0, spin_cap = SPIN_LIMIT;
-      bool gave_up       = false;
-      bool done          = false;
-      while (!done) {
-        unsigned int v[LB_WINDOW];
-#pragma unroll
-        for (int j = 0; j < LB_WINDOW; ++j) {
-          const int tj = t - j;
-          v[j]         = tj >= 0 ? ld_relaxed(lookback + (size_t)tj * RADIX + tid) : LB_FLAG_INCL;
-        }
-        int used = 0;
-#pragma unroll
-        for (int j = 0; j < LB_WINDOW; ++j) {
-          if (!done && used == j) {
-            const unsigned int f = v[j] >> 30;
-            if (f != 0) {
-              excl += v[j] & LB_VALUE;
-              ++used;
-              if (f == 2) done = true;
-            }
-          }
-        }
-        t -= used;
-        if (!done && used == 0) {
-          if (spins == 0 && ctrl->spin_limit != 0) spin_cap = ctrl->spin_limit;
-          if (++spins > spin_cap || ((spins & 1023u) == 0 && ld_relaxed(&ctrl->abort))) {
-            gave_up = true;
-            break;
-          }
-          if (spins > 4) __nanosleep(64);  // leave the issue slots to the other CTAs of the SM
-        }
-      }
-      if (gave_up) raise_timeout(ctrl);
-      st_relaxed(mine, LB_FLAG_INCL | ((excl + my_count) & LB_VALUE));
+      if (!look_back<WINDOW>(ctrl, lookback + (size_t)(tile - 1) * RADIX + tid, (int)t_in - 1, &excl)) raise_timeout(ctrl);
+      st_relaxed(lookback + (size_t)tile * RADIX + tid, LB_FLAG_INCL | ((excl + my_count) & LB_VALUE));
     }
     // global index of a staged element = base_ml[digit] + its position in the staged tile
     const unsigned int* bases =
