@@ -309,13 +309,13 @@ inline cudaError_t segsort_cfg(int xf, const void* in, void* out, int64_t* idx_o
 }
 
 // The merge-sort form of the on-chip row sort (4- and 8-byte keys, rows of more than 256 elements).
-template <int KB, bool PAIRS, int THREADS>
+template <int KB, bool PAIRS, int THREADS, int FORM>
 inline cudaError_t segmerge_cfg(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
                                 unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
 {
   using K   = typename KeyOf<KB>::type;
   using S   = SegMergeSmem<KB, PAIRS, THREADS>;
-  auto kern = segmerge_kernel<KB, PAIRS, THREADS>;
+  auto kern = segmerge_kernel<KB, PAIRS, THREADS, FORM>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::BYTES);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 148;
@@ -366,15 +366,25 @@ inline cudaError_t segwarp_any(int xf, const void* in, void* out, int64_t* idx_o
   return segwarp_cfg<KB, PAIRS, 16, 5>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
 }
 
+template <int KB, bool PAIRS, int FORM>
+inline cudaError_t segmerge_form(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
+                                 unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+{
+  constexpr int V = SM_VT;
+  if (seg_len <= 64 * V) return segmerge_cfg<KB, PAIRS, 64, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 128 * V) return segmerge_cfg<KB, PAIRS, 128, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 256 * V) return segmerge_cfg<KB, PAIRS, 256, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  return segmerge_cfg<KB, PAIRS, 512, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+}
+
 template <int KB, bool PAIRS>
 inline cudaError_t segmerge_any(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
                                 unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
 {
-  constexpr int V = SM_VT;
-  if (seg_len <= 64 * V) return segmerge_cfg<KB, PAIRS, 64>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 128 * V) return segmerge_cfg<KB, PAIRS, 128>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 256 * V) return segmerge_cfg<KB, PAIRS, 256>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  return segmerge_cfg<KB, PAIRS, 512>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (xf == XF_FLOAT) return segmerge_form<KB, PAIRS, SM_FLOAT>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if constexpr (KB == 8 && PAIRS)
+    if (xf == XF_CFLOAT) return segmerge_form<KB, PAIRS, SM_COMPLEX>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  return segmerge_form<KB, PAIRS, SM_INT>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
 }
 
 inline bool seg_merge_enabled()

@@ -150,9 +150,11 @@ template <int KB, int NB> struct RowBuckets {
     ok        = lo <= hi && fscale > (F)0 && fscale < (F)(KB == 8 ? 1e300 : 1e37f);
     exact     = false;
   }
-  __device__ __forceinline__ unsigned int bucket_float(K raw, K o) const
+  __device__ __forceinline__ unsigned int bucket_float(K o) const
   {
     const unsigned int u = upper(o);
+    const K flip         = (K)((K)1 << (8 * KB - 1)) | (K)~(K)((typename std::make_signed<K>::type)o >> (8 * KB - 1));
+    const K raw          = (K)(o ^ flip);  // the key's bits, but for signed zeros and NaNs
     unsigned int b;
     // the addition of 2^23 (2^52) leaves the rounded product in the low bits
     if constexpr (KB == 8) b = (unsigned int)__double_as_longlong(fma(value(raw) - fmin, fscale, 4503599627370496.0));
@@ -177,8 +179,11 @@ template <int KB, int NB> struct RowBuckets {
   }
 };
 
+// How a kernel turns keys into images: integers share one form (flip is the sign bit or nothing).
+enum : int { SM_INT = 0, SM_FLOAT = 1, SM_COMPLEX = 2 };
+
 // One CTA sorts one row at a time (grid-stride over rows); seg_len <= THREADS * 16.
-template <int KB, bool PAIRS, int THREADS>
+template <int KB, bool PAIRS, int THREADS, int FORM>
 __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : THREADS == 256 ? 3 : THREADS == 128 ? 5 : 10)
 segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out /* may be `in`: no __restrict__ */, int64_t* idx_out, unsigned int seg_len, unsigned long long nseg, int xf, int64_t index_offset)
 {
@@ -198,21 +203,38 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int first = tid * SM_VT;
   constexpr W WMAX = (W)~(W)0;
+  const K flip = xf == XF_SIGNED ? (K)((K)1 << (8 * KB - 1)) : (K)0;
+  auto image = [&](K raw) {
+    if constexpr (FORM == SM_FLOAT) return to_ordered<KB, XF_FLOAT>(raw);
+    else if constexpr (FORM == SM_COMPLEX) return to_ordered<8, XF_CFLOAT>(raw);
+    else return (K)(raw ^ flip);
+  };
+  auto from_image = [&](K o) {
+    if constexpr (FORM == SM_FLOAT) return sm_from_ordered<KB>(o, XF_FLOAT);
+    else return (K)(o ^ flip);
+  };
 
   for (unsigned long long seg = blockIdx.x; seg < nseg; seg += gridDim.x) {
     const K* src = in + seg * seg_len;
     // ---- load: consecutive threads read consecutive elements ----
     int special = 0;
-    K raw_in[SM_VT];
+    K img[SM_VT];
 #pragma unroll
     for (int j = 0; j < SM_VT; ++j) {
       const int e = j * THREADS + tid;
-      raw_in[j]   = (unsigned int)e < seg_len ? src[e] : (K)0;
+      img[j]      = (unsigned int)e < seg_len ? src[e] : (K)0;
     }
-    auto word_of = [&](K raw, int e) {
-      const K o = to_ordered_rt<KB>(raw, xf);
-      return PACK ? (W)(((unsigned long long)o << 32) | (unsigned int)e) : (W)o;
-    };
+#pragma unroll
+    for (int j = 0; j < SM_VT; ++j) {
+      const K raw = img[j];
+      img[j]      = image(raw);
+      if constexpr (FORM == SM_FLOAT && !PAIRS) {
+        // only zeros and NaNs can be special
+        const unsigned int u = RowBuckets<KB, S::NB>::upper(img[j]);
+        if (u == 0xFFFFFFFFu || u == 0x80000000u) special |= sm_is_special<KB>(raw, XF_FLOAT) ? 1 : 0;
+      }
+    }
+    auto word_of = [&](K o, int e) { return PACK ? (W)(((unsigned long long)o << 32) | (unsigned int)e) : (W)o; };
     W key[SM_VT];
     unsigned int pay[SIDE ? SM_VT : 1];
     auto cmp_swap = [&](int a, int b) {
@@ -251,13 +273,12 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
       constexpr int NB = S::NB;
       RowBuckets<KB, NB> rb;
       for (int i = tid; i < (int)(S::CNT_BYTES / 16); i += THREADS) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (xf == XF_FLOAT) {
+      if constexpr (FORM == SM_FLOAT) {
         unsigned int lo = 0xFFFFFFFFu, hi = 0;
 #pragma unroll
         for (int j = 0; j < SM_VT; ++j) {
           if ((unsigned int)(j * THREADS + tid) < seg_len) {
-            special |= sm_is_special<KB>(raw_in[j], xf) ? 1 : 0;
-            const unsigned int u = RowBuckets<KB, NB>::upper(to_ordered<KB, XF_FLOAT>(raw_in[j]));
+            const unsigned int u = RowBuckets<KB, NB>::upper(img[j]);
             if (u - RowBuckets<KB, NB>::FIN_LO < RowBuckets<KB, NB>::FIN_N) {
               lo = min(lo, u);
               hi = max(hi, u);
@@ -281,9 +302,8 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
 #pragma unroll
         for (int j = 0; j < SM_VT; ++j) {
           if ((unsigned int)(j * THREADS + tid) < seg_len) {
-            const K o = to_ordered_rt<KB>(raw_in[j], xf);
-            lo        = o < lo ? o : lo;
-            hi        = o > hi ? o : hi;
+            lo = img[j] < lo ? img[j] : lo;
+            hi = img[j] > hi ? img[j] : hi;
           }
         }
 #pragma unroll
@@ -308,18 +328,18 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
       // equal keys of a sort need no order among themselves: a row with fewer values than buckets is
       // done once it is counted
       const bool counted = !PAIRS && rb.exact;
-      unsigned int br[SM_VT];  // bucket | rank inside it << 16
+      unsigned int br[SM_VT];  // where the bucket's counter is | rank in the bucket << 16
       int over = rb.ok ? 0 : 1;
       if (rb.ok) {
 #pragma unroll
         for (int j = 0; j < SM_VT; ++j) {
           if ((unsigned int)(j * THREADS + tid) < seg_len) {
-            const K o            = to_ordered_rt<KB>(raw_in[j], xf);
-            const unsigned int b = xf == XF_FLOAT ? rb.bucket_float(raw_in[j], o) : rb.bucket_image(o);
-            const unsigned int h = (b & 1u) * 16u;
-            const unsigned int r = (atomicAdd(reinterpret_cast<unsigned int*>(cnt + (b >> 1) * 4 + (b >> 6) * 16), 1u << h) >> h) & 0xFFFFu;
+            const unsigned int b  = FORM == SM_FLOAT ? rb.bucket_float(img[j]) : rb.bucket_image(img[j]);
+            const unsigned int at = b * 2 + (b >> 6) * 16;  // of the bucket's 16 bits
+            const unsigned int h  = (b & 1u) * 16u;
+            const unsigned int r  = (atomicAdd(reinterpret_cast<unsigned int*>(cnt + (at & ~3u)), 1u << h) >> h) & 0xFFFFu;
             over |= r >= (unsigned int)SM_BUCKET ? 1 : 0;
-            br[j] = b | (r << 16);
+            br[j] = at | (r << 16);
           }
         }
       }
@@ -364,9 +384,8 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
         for (int j = 0; j < SM_VT; ++j) {
           const int e = j * THREADS + tid;
           if ((unsigned int)e < seg_len) {
-            const unsigned int b = br[j] & 0xFFFFu;
-            const unsigned int p = *reinterpret_cast<const unsigned short*>(cnt + (b >> 1) * 4 + (b >> 6) * 16 + (b & 1u) * 2) + (br[j] >> 16);
-            sw[smpad(p)] = word_of(raw_in[j], e);
+            const unsigned int p = *reinterpret_cast<const unsigned short*>(cnt + (br[j] & 0xFFFFu)) + (br[j] >> 16);
+            sw[smpad(p)] = word_of(img[j], e);
             if (SIDE) sp[smpad(p)] = (unsigned short)e;
           } else {
             sw[smpad(e)] = WMAX;
@@ -397,7 +416,7 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
 #pragma unroll
       for (int j = 0; j < SM_VT; ++j) {
         const int e  = j * THREADS + tid;
-        sw[smpad(e)] = (unsigned int)e < seg_len ? word_of(raw_in[j], e) : WMAX;
+        sw[smpad(e)] = (unsigned int)e < seg_len ? word_of(img[j], e) : WMAX;
         if (SIDE) sp[smpad(e)] = (unsigned short)e;
       }
       __syncthreads();
@@ -444,13 +463,13 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
 
     // ---- rows with -0.0 or unusual NaNs (sorts of keys): the elements the image folded are
     // fetched from the input in input order, to be written over their blocks after the store ----
-    K fix_raw[SM_VT];
-    int fix_at[SM_VT];
+    K fix_raw[FORM == SM_FLOAT && !PAIRS ? SM_VT : 1];
+    int fix_at[FORM == SM_FLOAT && !PAIRS ? SM_VT : 1];
     int nfix = 0;
-    if (!PAIRS && special) {
+    if constexpr (FORM == SM_FLOAT && !PAIRS) if (special) {
       if (tid == 0) {
         // block of zeros [z0, z1) and start of the NaN block in the sorted images
-        const W zimg = (W)to_ordered_rt<KB>((K)0, xf);
+        const W zimg = (W)image((K)0);
         int a = 0, b = (int)seg_len;
         while (a < b) { const int m = (a + b) >> 1; if (sw[smpad(m)] < zimg) a = m + 1; else b = m; }
         misc[0] = a;
@@ -494,7 +513,7 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
     // ---- store (coalesced) ----
     K* dst = out ? out + seg * seg_len : nullptr;
     if (!PAIRS) {
-      for (int e = tid; e < (int)seg_len; e += THREADS) dst[e] = sm_from_ordered<KB>((K)sw[smpad(e)], xf);
+      for (int e = tid; e < (int)seg_len; e += THREADS) dst[e] = from_image((K)sw[smpad(e)]);
       if (special) {
         __syncthreads();  // the plain store of the row is complete
         for (int f = 0; f < nfix; ++f) dst[fix_at[f]] = fix_raw[f];
