@@ -9,121 +9,138 @@
 namespace b2s {
 
 constexpr int UQ_THREADS = 256;
+constexpr int UQ_WARPS   = UQ_THREADS / 32;
 constexpr int UQ_ITEMS   = 16;
 constexpr int UQ_TILE    = UQ_THREADS * UQ_ITEMS;
 
-template <int KB>
-__device__ __forceinline__ bool is_head(const typename KeyOf<KB>::type* a, long long i, int xf)
+// Head of the workspace; one state word per tile follows (0: nothing yet).
+struct UniqueCtrl {
+  unsigned long long total;  // heads in the whole array, written by the last tile
+  unsigned int ticket;       // next tile
+  unsigned int status;       // 0 or DEV_ERR_TIMEOUT
+};
+constexpr unsigned long long UQ_AGG = 1ull << 62, UQ_INCL = 2ull << 62, UQ_VALUE = UQ_AGG - 1;
+
+__device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long long* p)
 {
-  return i == 0 || to_ordered_rt<KB>(a[i], xf) != to_ordered_rt<KB>(a[i - 1], xf);
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned long long v)
+{
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// pass 1: heads per tile
-template <int KB>
-__global__ void __launch_bounds__(UQ_THREADS)
-unique_count_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int xf,
-                    unsigned int* __restrict__ tile_counts)
-{
-  const long long base = (long long)blockIdx.x * UQ_TILE;
-  unsigned int c       = 0;
-  for (int j = 0; j < UQ_ITEMS; ++j) {
-    const long long i = base + j * UQ_THREADS + threadIdx.x;
-    if (i < n && is_head<KB>(a, i, xf)) ++c;
-  }
-  c = __reduce_add_sync(0xFFFFFFFFu, c);
-  __shared__ unsigned int w[UQ_THREADS / 32];
-  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int t = 0;
-    for (int k = 0; k < UQ_THREADS / 32; ++k) t += w[k];
-    tile_counts[blockIdx.x] = t;
-  }
-}
-
-// pass 2 (one CTA): exclusive scan of the tile counts into 64-bit offsets; total at [ntiles]
-static __global__ void __launch_bounds__(1024)
-unique_scan_kernel(const unsigned int* __restrict__ tile_counts, long long ntiles, unsigned long long* __restrict__ offsets)
-{
-  __shared__ unsigned long long warp_tot[32];
-  __shared__ unsigned long long carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (long long base = 0; base < ntiles; base += 1024) {
-    const long long i      = base + threadIdx.x;
-    const unsigned long long c = i < ntiles ? tile_counts[i] : 0;
-    unsigned long long incl    = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) warp_tot[w] = incl;
-    __syncthreads();
-    unsigned long long before = carry;
-    for (int k = 0; k < w; ++k) before += warp_tot[k];
-    if (i < ntiles) offsets[i] = before + incl - c;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry = before + incl;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) offsets[ntiles] = carry;
-}
-
-// pass 3: write the heads of a tile to its offset, in order
+// One pass over the sorted keys: a CTA takes the next tile (ticket), counts its heads, chains the count
+// to its predecessors (decoupled look-back, 32 tiles per round trip, one lane each) and writes its heads
+// in order.  Bound by memory: every key is read once from HBM (its left neighbour comes from the L1),
+// every head written once; counting, scanning and writing in three launches read the keys twice
+// (33.5 M int64 keys, an eighth of them heads: see the figures at unique_launch).
 template <int KB>
 __global__ void __launch_bounds__(UQ_THREADS)
-unique_write_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int xf,
-                    const unsigned long long* __restrict__ offsets, typename KeyOf<KB>::type* __restrict__ out)
+unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int xf, UniqueCtrl* ctrl,
+              unsigned long long* __restrict__ state, typename KeyOf<KB>::type* __restrict__ out)
 {
   using K = typename KeyOf<KB>::type;
-  __shared__ unsigned int warp_tot[UQ_THREADS / 32];
-  __shared__ unsigned int running;
-  if (threadIdx.x == 0) running = 0;
+  __shared__ unsigned int heads[UQ_ITEMS * UQ_WARPS];  // per group of 32 keys, in key order; then their prefix
+  __shared__ unsigned int tile_sh;
+  __shared__ unsigned long long before_sh;
+  if (threadIdx.x == 0) tile_sh = atomicAdd(&ctrl->ticket, 1u);
   __syncthreads();
-  const long long base           = (long long)blockIdx.x * UQ_TILE;
-  const unsigned long long tile0 = offsets[blockIdx.x];
+  const unsigned int tile = tile_sh;
+  const long long base    = (long long)tile * UQ_TILE;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  K key[UQ_ITEMS];
+  unsigned int bal[UQ_ITEMS];
+#pragma unroll
   for (int j = 0; j < UQ_ITEMS; ++j) {
     const long long i = base + j * UQ_THREADS + threadIdx.x;
-    const bool head   = i < n && is_head<KB>(a, i, xf);
-    const unsigned int bal = __ballot_sync(0xFFFFFFFFu, head);
-    if (lane == 0) warp_tot[w] = __popc(bal);
-    __syncthreads();
-    unsigned int before = running;
-    for (int k = 0; k < w; ++k) before += warp_tot[k];
-    if (head) out[tile0 + before + __popc(bal & ((1u << lane) - 1))] = a[i];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned int t = 0;
-      for (int k = 0; k < UQ_THREADS / 32; ++k) t += warp_tot[k];
-      running += t;
-    }
-    __syncthreads();
+    key[j]            = i < n ? a[i] : (K)0;
   }
+#pragma unroll
+  for (int j = 0; j < UQ_ITEMS; ++j) {
+    const long long i = base + j * UQ_THREADS + threadIdx.x;
+    const bool head   = i < n && (i == 0 || to_ordered_rt<KB>(key[j], xf) != to_ordered_rt<KB>(a[i - 1], xf));
+    bal[j]            = __ballot_sync(0xFFFFFFFFu, head);
+    if (lane == 0) heads[j * UQ_WARPS + w] = __popc(bal[j]);
+  }
+  __syncthreads();
+  if (w == 0) {
+    // 128 counts, four consecutive ones per lane
+    constexpr int PER = UQ_ITEMS * UQ_WARPS / 32;
+    unsigned int c[PER], sum = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      c[j] = heads[lane * PER + j];
+      sum += c[j];
+    }
+    unsigned int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    unsigned int run = incl - sum;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      heads[lane * PER + j] = run;
+      run += c[j];
+    }
+    const unsigned long long mine = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    unsigned long long before     = 0;
+    if (tile != 0) {
+      if (lane == 0) st_relaxed64(state + tile, UQ_AGG | mine);
+      long long t        = (long long)tile - 1 - lane;
+      unsigned int spins = 0;
+      while (true) {
+        const unsigned long long v  = t >= 0 ? ld_relaxed64(state + t) : UQ_INCL;
+        const unsigned int missing  = __ballot_sync(0xFFFFFFFFu, v == 0);
+        const unsigned int inclusive = __ballot_sync(0xFFFFFFFFu, (v >> 62) == 2);
+        // the nearest entries up to the first gap; up to and with the first inclusive one
+        const int gap   = missing ? __ffs(missing) - 1 : 32;
+        const int stop  = inclusive ? __ffs(inclusive) - 1 : 32;
+        const int used  = stop < gap ? stop + 1 : gap;
+        unsigned long long add = lane < used ? v & UQ_VALUE : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xFFFFFFFFu, add, o);
+        before += add;
+        t -= used;
+        if (stop < gap) break;
+        if (used == 0) {
+          if (++spins > SPIN_LIMIT || ((spins & 1023u) == 0 && ld_relaxed(&ctrl->status) != 0)) {
+            if (lane == 0) atomicMax(&ctrl->status, DEV_ERR_TIMEOUT);
+            break;
+          }
+          if (spins > 4) __nanosleep(64);
+        }
+      }
+    }
+    if (lane == 0) {
+      st_relaxed64(state + tile, UQ_INCL | (before + mine));
+      before_sh = before;
+      if (base + UQ_TILE >= n) ctrl->total = before + mine;
+    }
+  }
+  __syncthreads();
+  K* dst = out + before_sh;
+#pragma unroll
+  for (int j = 0; j < UQ_ITEMS; ++j)
+    if ((bal[j] >> lane) & 1u) dst[heads[j * UQ_WARPS + w] + __popc(bal[j] & ((1u << lane) - 1))] = key[j];
 }
 
 template <int KB>
 static cudaError_t unique_launch(const void* a, long long n, int xf, void* out, unsigned char* ws, cudaStream_t stream)
 {
   using K = typename KeyOf<KB>::type;
-  const long long ntiles        = (n + UQ_TILE - 1) / UQ_TILE;
-  unsigned int* counts          = reinterpret_cast<unsigned int*>(ws);
-  unsigned long long* offsets   = reinterpret_cast<unsigned long long*>(ws + align_up((size_t)ntiles * 4, 256));
-  {
-    prof::Scope ps(prof::K_DIST, stream);
-    unique_count_kernel<KB><<<(unsigned int)ntiles, UQ_THREADS, 0, stream>>>(static_cast<const K*>(a), n, xf, counts);
-  }
-  {
-    prof::Scope ps(prof::K_DIST, stream);
-    unique_scan_kernel<<<1, 1024, 0, stream>>>(counts, ntiles, offsets);
-  }
-  {
-    prof::Scope ps(prof::K_DIST, stream);
-    unique_write_kernel<KB><<<(unsigned int)ntiles, UQ_THREADS, 0, stream>>>(static_cast<const K*>(a), n, xf, offsets,
-                                                                          static_cast<K*>(out));
-  }
+  const long long ntiles = (n + UQ_TILE - 1) / UQ_TILE;
+  UniqueCtrl* ctrl          = reinterpret_cast<UniqueCtrl*>(ws);
+  unsigned long long* state = reinterpret_cast<unsigned long long*>(ws + 256);
+  const cudaError_t e       = cudaMemsetAsync(ws, 0, 256 + (size_t)ntiles * 8, stream);
+  if (e != cudaSuccess) return e;
+  prof::Scope ps(prof::K_DIST, stream);
+  unique_kernel<KB><<<(unsigned int)ntiles, UQ_THREADS, 0, stream>>>(static_cast<const K*>(a), n, xf, ctrl, state,
+                                                                    static_cast<K*>(out));
   return cudaGetLastError();
 }
 
@@ -137,7 +154,7 @@ int b2s_unique_workspace_bytes(size_t n, size_t* bytes)
 {
   if (bytes == nullptr) return B2S_ERR_INVALID_ARG;
   const size_t ntiles = (n + UQ_TILE - 1) / UQ_TILE;
-  *bytes              = align_up(ntiles * 4, 256) + align_up((ntiles + 1) * 8, 256);
+  *bytes              = 256 + align_up(ntiles * 8, 256);
   return B2S_OK;
 }
 
@@ -177,12 +194,11 @@ int b2s_unique_sorted(int dtype, const void* sorted, size_t n, void* out, size_t
     default: e = unique_launch<8>(sorted, (long long)n, xf, out, w, stream); break;
   }
   if (e != cudaSuccess) return B2S_ERR_CUDA;
-  const size_t ntiles = (n + UQ_TILE - 1) / UQ_TILE;
-  unsigned long long total = 0;
-  const unsigned long long* offsets = reinterpret_cast<const unsigned long long*>(w + align_up(ntiles * 4, 256));
-  if (cudaMemcpyAsync(&total, offsets + ntiles, 8, cudaMemcpyDeviceToHost, stream) != cudaSuccess) return B2S_ERR_CUDA;
+  UniqueCtrl done{};
+  if (cudaMemcpyAsync(&done, w, sizeof(done), cudaMemcpyDeviceToHost, stream) != cudaSuccess) return B2S_ERR_CUDA;
   if (cudaStreamSynchronize(stream) != cudaSuccess) return B2S_ERR_CUDA;
-  *out_len = (size_t)total;
+  if (done.status != 0) return (int)done.status;
+  *out_len = (size_t)done.total;
   return B2S_OK;
 }
 }
