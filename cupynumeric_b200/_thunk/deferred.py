@@ -118,6 +118,16 @@ class DeferredArray:
         vals = v.base.contiguous()
         assert vals.dtype == tile.dtype, "searchsorted: the caller brings both arrays to one dtype"
         global_size = tile.numel()
+        if runtime.num_procs == 1 and rhs.global_lo == 0:
+            # the tile is the whole array: positions are stored, there is nothing to combine
+            out = torch.empty(vals.shape, dtype=torch.int64, device=tile.device)
+            _lib.check(lib.b2s_searchsorted_whole(_lib.DTYPE_CODE[to_numpy_dtype(tile.dtype)],
+                                                  tile.data_ptr() if tile.numel() else None, tile.numel(),
+                                                  vals.data_ptr() if vals.numel() else None, vals.numel(), int(is_left),
+                                                  out.data_ptr() if out.numel() else None, runtime.stream_handle()),
+                       "b2s_searchsorted_whole")
+            self.base = out
+            return
         if runtime.num_procs > 1:
             t = torch.tensor([global_size], dtype=torch.int64, device=tile.device)
             dist.all_reduce(t)

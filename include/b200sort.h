@@ -286,6 +286,11 @@ int b2s_searchsorted(int dtype, const void* sorted_tile, size_t n_tile, int64_t 
                      const void* values, size_t num_values, int left, int64_t* positions,
                      void* cuda_stream);
 
+/* The same for a tile that is the whole array (one process): the positions are stored as they are, so
+ * `positions` needs no pre-fill and nothing is combined. */
+int b2s_searchsorted_whole(int dtype, const void* sorted, size_t n, const void* values, size_t num_values, int left,
+                           int64_t* positions, void* cuda_stream);
+
 /* ---- UNIQUE on sorted data ------------------------------------------------------------------- */
 
 /* Writes the first element of every run of equal keys of `sorted` (n elements, ascending) to
