@@ -129,6 +129,7 @@ SIGNATURES = {
     "b2s_host_bucket_of": (_I, [_P, _I, _I, ctypes.c_ulonglong, ctypes.c_ulonglong, ctypes.c_longlong]),
     "b2s_searchsorted": (_I, [_I, _P, _SZ, _I64, _P, _SZ, _I, _P, _P]),
     "b2s_searchsorted_whole": (_I, [_I, _P, _SZ, _P, _SZ, _I, _P, _P]),
+    "b2s_transpose": (_I, [_SZ, _P, _P, _SZ, _SZ, _SZ, _P]),
     "b2s_unique_workspace_bytes": (_I, [_SZ, ctypes.POINTER(_SZ)]),
     "b2s_unique_sorted": (_I, [_I, _P, _SZ, _P, ctypes.POINTER(_SZ), _P, _SZ, _P]),
     "b2s_profile_enable": (_I, [_I]),

@@ -59,12 +59,38 @@ def sort_flattened(output: DeferredArray, input: DeferredArray, argsort: bool, s
     output.base, output.global_lo, output.tiled_axis = result.base, result.global_lo, result.tiled_axis
 
 
+# Shorter sides than this leave most of a transposed tile empty: torch's strided copy takes those.
+TRANSPOSE_MIN = 32
+
+
+def _transpose(moved: DeferredArray, input: DeferredArray, sort_axis: int) -> bool:
+    """Fills ``moved`` with the dense copy of ``input`` whose last two axes are swapped, tile by tile
+    through shared memory.  False (nothing done) where that is not the copy that is wanted: other axes, a
+    strided or conjugated input, 16-byte elements, short sides, more tiles than a grid holds."""
+    t = input.base
+    if sort_axis != input.ndim - 2 or not t.is_contiguous() or t.is_conj() or t.is_neg() or not t.is_cuda:
+        return False
+    rows, cols = t.shape[-2:]
+    size = t.element_size()
+    if size > 8 or min(rows, cols) < TRANSPOSE_MIN or t.numel() >= 1 << 40:
+        return False
+    swapped = input.swapaxes(sort_axis, input.ndim - 1)
+    out = torch.empty(swapped.shape, dtype=t.dtype, device=t.device)
+    batch = t.numel() // (rows * cols)
+    _lib.check(_lib.lib().b2s_transpose(size, t.data_ptr(), out.data_ptr(), batch, rows, cols, runtime.stream_handle()),
+               "b2s_transpose")
+    moved.base = out
+    moved.global_lo, moved.tiled_axis = swapped.global_lo, swapped.tiled_axis
+    return True
+
+
 def sort_swapped(output: DeferredArray, input: DeferredArray, argsort: bool, sort_axis: int,
                  stable: bool) -> None:
     sort_axis = normalize_axis_index(sort_axis, input.ndim)
     last = input.ndim - 1
     moved = create_deferred_thunk(input.swapaxes(sort_axis, last).shape, dtype=input.dtype)
-    moved.copy(input.swapaxes(sort_axis, last), deep=True)
+    if not _transpose(moved, input, sort_axis):
+        moved.copy(input.swapaxes(sort_axis, last), deep=True)
     if argsort:
         result = create_deferred_thunk(moved.shape, dtype=output.dtype)
         sort_deferred(result, moved, argsort, stable=stable)

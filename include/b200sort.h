@@ -291,6 +291,11 @@ int b2s_searchsorted(int dtype, const void* sorted_tile, size_t n_tile, int64_t 
 int b2s_searchsorted_whole(int dtype, const void* sorted, size_t n, const void* values, size_t num_values, int left,
                            int64_t* positions, void* cuda_stream);
 
+/* out[b][c][r] = in[b][r][c] for `batch` dense matrices of rows x cols elements of 1, 2, 4 or 8 bytes (out must
+ * not overlap in; both aligned to the element): the copy that brings another axis than the last to the end
+ * (cupynumeric/_thunk/_sort.py:50-76 of the reference). */
+int b2s_transpose(size_t elem_bytes, const void* in, void* out, size_t batch, size_t rows, size_t cols, void* cuda_stream);
+
 /* ---- UNIQUE on sorted data ------------------------------------------------------------------- */
 
 /* Writes the first element of every run of equal keys of `sorted` (n elements, ascending) to
