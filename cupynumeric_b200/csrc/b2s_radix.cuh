@@ -322,7 +322,22 @@ seg_hist_kernel(const typename KeyOf<KB>::type* __restrict__ keys, unsigned int 
   const unsigned int lo  = chunk * SEG_HIST_CHUNK;
   const unsigned int hi  = min(seg_len, lo + SEG_HIST_CHUNK);
   const auto* base       = keys + (size_t)seg * seg_len;
-  for (unsigned int i = lo + threadIdx.x; i < hi; i += 256) {
+  // eight loads in flight per thread: with one the kernel waited for memory most of the time (segments
+  // start at any element, so the loads are one element wide)
+  constexpr int AHEAD = 8;
+  unsigned int i      = lo + threadIdx.x;
+  for (; i + (AHEAD - 1) * 256 < hi; i += AHEAD * 256) {
+    typename KeyOf<KB>::type raw[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) raw[j] = base[i + j * 256];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) {
+      const auto k = to_ordered<KB, XF>(raw[j]);
+#pragma unroll
+      for (int p = 0; p < KB; ++p) atomicAdd(&sh[p][(unsigned int)(k >> (8 * p)) & 0xFFu], 1u);
+    }
+  }
+  for (; i < hi; i += 256) {
     const auto k = to_ordered<KB, XF>(base[i]);
 #pragma unroll
     for (int p = 0; p < KB; ++p) atomicAdd(&sh[p][(unsigned int)(k >> (8 * p)) & 0xFFu], 1u);
