@@ -22,6 +22,11 @@ from ..runtime import runtime
 from .deferred import DeferredArray, create_deferred_thunk, to_numpy_dtype
 
 
+# Segments of up to this many elements are sorted on chip (SEG_CAP in csrc/b2s_launch.cuh) by kernels
+# that wait for nothing: there is no status to collect.
+ON_CHIP = 8192
+
+
 def local_sort_tile(tile: torch.Tensor, argsort: bool, stable: bool, index_offset: int = 0,
                     out: torch.Tensor | None = None) -> torch.Tensor:
     """Runs the point task body on one dense row-major tile: sorts along the last axis.
@@ -47,7 +52,7 @@ def local_sort_tile(tile: torch.Tensor, argsort: bool, stable: bool, index_offse
                             int(tile.ndim == 1), int(stable), ws.data_ptr(), ws.numel(),
                             runtime.stream_handle())
     _lib.check(st, "b2s_local_sort")
-    if tile.dtype != torch.complex128:  # (its inner sorts keep their control blocks elsewhere)
+    if segment > ON_CHIP and tile.dtype != torch.complex128:  # (its inner sorts keep their control blocks elsewhere)
         runtime.note_sort(ws)
     return out
 

@@ -76,22 +76,23 @@ inline cudaError_t radix_seg_any(int kb, int xf, const void* in, void* out, int6
 }
 
 inline cudaError_t seg_any(int kb, int xf, const void* in, void* out, int64_t* idx, unsigned int L,
-                           unsigned long long nseg, int64_t off, Ctrl* ctrl, cudaStream_t s)
+                           unsigned long long nseg, int64_t off, unsigned int* status, cudaStream_t s)
 {
   switch (kb) {
-    case 1: return launch_segsort<1>(xf, in, out, idx, L, nseg, off, ctrl, s);
-    case 2: return launch_segsort<2>(xf, in, out, idx, L, nseg, off, ctrl, s);
-    case 4: return launch_segsort<4>(xf, in, out, idx, L, nseg, off, ctrl, s);
-    default: return launch_segsort<8>(xf, in, out, idx, L, nseg, off, ctrl, s);
+    case 1: return launch_segsort<1>(xf, in, out, idx, L, nseg, off, status, s);
+    case 2: return launch_segsort<2>(xf, in, out, idx, L, nseg, off, status, s);
+    case 4: return launch_segsort<4>(xf, in, out, idx, L, nseg, off, status, s);
+    default: return launch_segsort<8>(xf, in, out, idx, L, nseg, off, status, s);
   }
 }
 
 // Segments of one element: the output is the input, every index is index_offset.
 __global__ void unit_segment_kernel(const unsigned char* in, unsigned char* out, int64_t* idx, size_t volume,
-                                    int kb, int64_t index_offset)
+                                    int kb, int64_t index_offset, unsigned int* status)
 {
   const size_t gthread = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t gstride = (size_t)gridDim.x * blockDim.x;
+  if (gthread == 0) *status = 0;
   if (out != nullptr && out != in)
     for (size_t i = gthread; i < volume * kb; i += gstride) out[i] = in[i];
   if (idx != nullptr)
@@ -265,18 +266,17 @@ int b2s_local_sort(int dtype, const void* keys_in, void* keys_out, int64_t* idx_
   cudaError_t e;
 
   if (segment <= SEG_CAP) {
-    e = cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), stream);
-    if (e != cudaSuccess) return B2S_ERR_CUDA;
+    // on-chip kernels: no waits, hence no control block to clear in front of them
     if (segment == 1) {
       size_t grid = (volume + 4095) / 4096;
       if (grid > 148 * 8) grid = 148 * 8;
       prof::Scope ps(prof::K_UNIT, stream);
       unit_segment_kernel<<<(unsigned int)grid, 256, 0, stream>>>(static_cast<const unsigned char*>(keys_in),
                                                                  static_cast<unsigned char*>(keys_out), idx_out,
-                                                                 volume, di.kb, index_offset);
+                                                                 volume, di.kb, index_offset, &ctrl->status);
       return cudaGetLastError() == cudaSuccess ? B2S_OK : B2S_ERR_CUDA;
     }
-    e = seg_any(di.kb, di.xf, keys_in, keys_out, idx_out, (unsigned int)segment, nseg, index_offset, ctrl, stream);
+    e = seg_any(di.kb, di.xf, keys_in, keys_out, idx_out, (unsigned int)segment, nseg, index_offset, &ctrl->status, stream);
     return e == cudaSuccess ? B2S_OK : B2S_ERR_CUDA;
   }
 

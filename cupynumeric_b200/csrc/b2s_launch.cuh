@@ -278,14 +278,15 @@ cudaError_t launch_radix_1d(int xf, const void* in, void* out, int64_t* idx_out,
                             const uint32_t* idx_in = nullptr, const unsigned int* hist_parts = nullptr,
                             int hist_nparts = 0);
 
-// Segments of seg_len <= SEG_CAP elements, sorted on chip. `ctrl` must be a zeroed control block.
+// Segments of seg_len <= SEG_CAP elements, sorted on chip. `status` (the workspace's
+// status word) is set to 0 by the kernels, which have nothing to report.
 template <int KB>
 cudaError_t launch_segsort(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                           unsigned long long nseg, int64_t index_offset, Ctrl* ctrl, cudaStream_t stream);
+                           unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream);
 
 template <int KB, bool PAIRS, int THREADS, int ITEMS>
 inline cudaError_t segsort_cfg(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                               unsigned long long nseg, int64_t index_offset, Ctrl* ctrl, cudaStream_t stream)
+                               unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
   using K   = typename KeyOf<KB>::type;
   using S   = SegSmem<KB, PAIRS, THREADS, ITEMS>;
@@ -303,7 +304,7 @@ inline cudaError_t segsort_cfg(int xf, const void* in, void* out, int64_t* idx_o
   {
     prof::Scope ps(prof::K_SEGSORT, stream);
     kern<<<(unsigned int)grid, THREADS, S::BYTES, stream>>>(static_cast<const K*>(in), static_cast<K*>(out),
-                                                             idx_out, seg_len, nseg, xf, index_offset, ctrl);
+                                                             idx_out, seg_len, nseg, xf, index_offset, status);
   }
   return cudaGetLastError();
 }
@@ -311,7 +312,7 @@ inline cudaError_t segsort_cfg(int xf, const void* in, void* out, int64_t* idx_o
 // The merge-sort form of the on-chip row sort (4- and 8-byte keys, rows of more than 256 elements).
 template <int KB, bool PAIRS, int THREADS, int FORM>
 inline cudaError_t segmerge_cfg(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                                unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+                                unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
   using K   = typename KeyOf<KB>::type;
   using S   = SegMergeSmem<KB, PAIRS, THREADS>;
@@ -329,7 +330,7 @@ inline cudaError_t segmerge_cfg(int xf, const void* in, void* out, int64_t* idx_
   {
     prof::Scope ps(prof::K_SEGSORT, stream);
     kern<<<(unsigned int)grid, THREADS, S::BYTES, stream>>>(static_cast<const K*>(in), static_cast<K*>(out), idx_out, seg_len,
-                                                             nseg, xf, index_offset);
+                                                             nseg, xf, index_offset, status);
   }
   return cudaGetLastError();
 }
@@ -337,7 +338,7 @@ inline cudaError_t segmerge_cfg(int xf, const void* in, void* out, int64_t* idx_
 // Rows of up to SW_MAX elements: one warp per 32 / group rows.
 template <int KB, bool PAIRS, int VT, int GL>
 inline cudaError_t segwarp_cfg(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                               unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+                               unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
   using K = typename KeyOf<KB>::type;
   constexpr unsigned long long ROWS = (unsigned long long)SW_WARPS * (32 >> GL);
@@ -346,45 +347,45 @@ inline cudaError_t segwarp_cfg(int xf, const void* in, void* out, int64_t* idx_o
   {
     prof::Scope ps(prof::K_SEGSORT, stream);
     segwarp_kernel<KB, PAIRS, VT, GL><<<(unsigned int)grid, SW_WARPS * 32, 0, stream>>>(
-      static_cast<const K*>(in), static_cast<K*>(out), idx_out, seg_len, nseg, xf, index_offset);
+      static_cast<const K*>(in), static_cast<K*>(out), idx_out, seg_len, nseg, xf, index_offset, status);
   }
   return cudaGetLastError();
 }
 
 template <int KB, bool PAIRS>
 inline cudaError_t segwarp_any(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                               unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+                               unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
-  if (seg_len <= 2) return segwarp_cfg<KB, PAIRS, 2, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 4) return segwarp_cfg<KB, PAIRS, 4, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 8) return segwarp_cfg<KB, PAIRS, 8, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 16) return segwarp_cfg<KB, PAIRS, 16, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 32) return segwarp_cfg<KB, PAIRS, 16, 1>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 64) return segwarp_cfg<KB, PAIRS, 16, 2>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 128) return segwarp_cfg<KB, PAIRS, 16, 3>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 256) return segwarp_cfg<KB, PAIRS, 16, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  return segwarp_cfg<KB, PAIRS, 16, 5>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 2) return segwarp_cfg<KB, PAIRS, 2, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 4) return segwarp_cfg<KB, PAIRS, 4, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 8) return segwarp_cfg<KB, PAIRS, 8, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 16) return segwarp_cfg<KB, PAIRS, 16, 0>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 32) return segwarp_cfg<KB, PAIRS, 16, 1>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 64) return segwarp_cfg<KB, PAIRS, 16, 2>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 128) return segwarp_cfg<KB, PAIRS, 16, 3>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 256) return segwarp_cfg<KB, PAIRS, 16, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  return segwarp_cfg<KB, PAIRS, 16, 5>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
 }
 
 template <int KB, bool PAIRS, int FORM>
 inline cudaError_t segmerge_form(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                                 unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+                                 unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
   constexpr int V = SM_VT;
-  if (seg_len <= 64 * V) return segmerge_cfg<KB, PAIRS, 64, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 128 * V) return segmerge_cfg<KB, PAIRS, 128, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  if (seg_len <= 256 * V) return segmerge_cfg<KB, PAIRS, 256, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  return segmerge_cfg<KB, PAIRS, 512, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (seg_len <= 64 * V) return segmerge_cfg<KB, PAIRS, 64, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 128 * V) return segmerge_cfg<KB, PAIRS, 128, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 256 * V) return segmerge_cfg<KB, PAIRS, 256, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  return segmerge_cfg<KB, PAIRS, 512, FORM>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
 }
 
 template <int KB, bool PAIRS>
 inline cudaError_t segmerge_any(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                                unsigned long long nseg, int64_t index_offset, cudaStream_t stream)
+                                unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
-  if (xf == XF_FLOAT) return segmerge_form<KB, PAIRS, SM_FLOAT>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+  if (xf == XF_FLOAT) return segmerge_form<KB, PAIRS, SM_FLOAT>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
   if constexpr (KB == 8 && PAIRS)
-    if (xf == XF_CFLOAT) return segmerge_form<KB, PAIRS, SM_COMPLEX>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-  return segmerge_form<KB, PAIRS, SM_INT>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+    if (xf == XF_CFLOAT) return segmerge_form<KB, PAIRS, SM_COMPLEX>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  return segmerge_form<KB, PAIRS, SM_INT>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
 }
 
 inline bool seg_merge_enabled()
@@ -395,7 +396,7 @@ inline bool seg_merge_enabled()
 
 template <int KB, bool PAIRS>
 inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
-                                 unsigned long long nseg, int64_t index_offset, Ctrl* ctrl, cudaStream_t stream)
+                                 unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
   // Short rows go to the warp kernel (2^24 float32 keys with positions, against the one-CTA-per-row radix
   // kernel they took before: rows of 2 19.2 ms -> 0.09 ms, of 32 1.31 -> 0.16, of 100 0.47 -> 0.22, of 200
@@ -405,25 +406,25 @@ inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx
   // rows are sorted with positions and the keys fetched through them.  So are keys below 4 bytes, whose
   // words have room for the position anyway.
   if (KB == 1 && seg_len > 64 && seg_len <= 128)
-    return segsort_cfg<KB, PAIRS, 32, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
+    return segsort_cfg<KB, PAIRS, 32, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
   if (seg_len <= SW_MAX) {
     if constexpr (PAIRS || KB < 4) {
-      return segwarp_any<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+      return segwarp_any<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
     } else {
-      if (KB == 8 && xf == XF_CFLOAT) return segwarp_any<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
-      return segwarp_any<KB, false>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+      if (KB == 8 && xf == XF_CFLOAT) return segwarp_any<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+      return segwarp_any<KB, false>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
     }
   }
   if constexpr (KB == 4 || KB == 8) {
     if (seg_merge_enabled()) {
       if constexpr (!PAIRS && KB == 8)
-        if (xf == XF_CFLOAT) return segmerge_any<KB, true>(xf, in, out, nullptr, seg_len, nseg, index_offset, stream);
-      return segmerge_any<KB, PAIRS>(xf, in, out, idx_out, seg_len, nseg, index_offset, stream);
+        if (xf == XF_CFLOAT) return segmerge_any<KB, true>(xf, in, out, nullptr, seg_len, nseg, index_offset, status, stream);
+      return segmerge_any<KB, PAIRS>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
     }
   }
-  if (seg_len <= 1024) return segsort_cfg<KB, PAIRS, 128, 8>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
-  if (seg_len <= 4096) return segsort_cfg<KB, PAIRS, 256, 16>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
-  return segsort_cfg<KB, PAIRS, 512, 16>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);
+  if (seg_len <= 1024) return segsort_cfg<KB, PAIRS, 128, 8>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if (seg_len <= 4096) return segsort_cfg<KB, PAIRS, 256, 16>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  return segsort_cfg<KB, PAIRS, 512, 16>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
 }
 
 #define B2S_INSTANTIATE_KEY_WIDTH(KB, HAS_FLOAT, HAS_CFLOAT)                                                          \
@@ -455,13 +456,13 @@ inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx
   }                                                                                                       \
   template <>                                                                                             \
   cudaError_t launch_segsort<KB>(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len, \
-                                 unsigned long long nseg, int64_t index_offset, Ctrl* ctrl,               \
+                                 unsigned long long nseg, int64_t index_offset, unsigned int* status,               \
                                  cudaStream_t stream)                                                     \
   {                                                                                                       \
     if ((!HAS_FLOAT && xf == XF_FLOAT) || (!HAS_CFLOAT && xf == XF_CFLOAT)) return cudaErrorInvalidValue; \
     if (idx_out != nullptr)                                                                               \
-      return segsort_pairs<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);    \
-    return segsort_pairs<KB, false>(xf, in, out, idx_out, seg_len, nseg, index_offset, ctrl, stream);     \
+      return segsort_pairs<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);    \
+    return segsort_pairs<KB, false>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);     \
   }
 
 }  // namespace b2s

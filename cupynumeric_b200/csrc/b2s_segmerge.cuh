@@ -185,7 +185,8 @@ enum : int { SM_INT = 0, SM_FLOAT = 1, SM_COMPLEX = 2 };
 // One CTA sorts one row at a time (grid-stride over rows); seg_len <= THREADS * 16.
 template <int KB, bool PAIRS, int THREADS, int FORM>
 __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : THREADS == 256 ? 3 : THREADS == 128 ? 5 : 10)
-segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out /* may be `in`: no __restrict__ */, int64_t* idx_out, unsigned int seg_len, unsigned long long nseg, int xf, int64_t index_offset)
+segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out /* may be `in`: no __restrict__ */, int64_t* idx_out, unsigned int seg_len, unsigned long long nseg, int xf, int64_t index_offset,
+                unsigned int* __restrict__ status)
 {
   using K = typename KeyOf<KB>::type;
   using S = SegMergeSmem<KB, PAIRS, THREADS>;
@@ -214,6 +215,7 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
     else return (K)(o ^ flip);
   };
 
+  if (blockIdx.x == 0 && tid == 0) *status = 0;  // nothing here waits, so nothing can time out
   for (unsigned long long seg = blockIdx.x; seg < nseg; seg += gridDim.x) {
     const K* src = in + seg * seg_len;
     // ---- load: consecutive threads read consecutive elements ----

@@ -20,8 +20,7 @@ struct SegSmem {
   static constexpr size_t OFF_WHIST   = OFF_PAY + PAY_BYTES;
   static constexpr size_t OFF_EXCL    = OFF_WHIST + (size_t)WARPS * RADIX * 4;
   static constexpr size_t OFF_RED     = OFF_EXCL + RADIX * 4;        // 2 x WARPS x 8 bytes
-  static constexpr size_t OFF_BAR     = OFF_RED + (size_t)WARPS * 16;
-  static constexpr size_t BYTES       = OFF_BAR + 16;
+  static constexpr size_t BYTES       = OFF_RED + (size_t)WARPS * 16;
 };
 
 // One CTA sorts one segment at a time (grid-stride over segments). seg_len <= THREADS*ITEMS.
@@ -32,7 +31,7 @@ template <int KB, bool PAIRS, int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS)
 segsort_kernel(const typename KeyOf<KB>::type* __restrict__ in, typename KeyOf<KB>::type* __restrict__ out,
                int64_t* __restrict__ idx_out, unsigned int seg_len, unsigned long long nseg, int xf,
-               int64_t index_offset, Ctrl* ctrl)
+               int64_t index_offset, unsigned int* __restrict__ status)
 {
   using K = typename KeyOf<KB>::type;
   using S = SegSmem<KB, PAIRS, THREADS, ITEMS>;
@@ -45,7 +44,6 @@ segsort_kernel(const typename KeyOf<KB>::type* __restrict__ in, typename KeyOf<K
   unsigned int* warp_hist = reinterpret_cast<unsigned int*>(smem + S::OFF_WHIST);
   unsigned int* dig_excl  = reinterpret_cast<unsigned int*>(smem + S::OFF_EXCL);
   unsigned long long* red = reinterpret_cast<unsigned long long*>(smem + S::OFF_RED);
-  uint64_t* bar           = reinterpret_cast<uint64_t*>(smem + S::OFF_BAR);
 
   const int tid  = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -54,39 +52,18 @@ segsort_kernel(const typename KeyOf<KB>::type* __restrict__ in, typename KeyOf<K
   unsigned int* my_hist = warp_hist + warp * RADIX;
   const K pad           = pad_raw<KB>(xf);
 
-  if (tid == 0) {
-    mbar_init(bar, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  uint32_t phase = 0;
-
+  if (blockIdx.x == 0 && tid == 0) *status = 0;  // nothing here waits, so nothing can time out
   const size_t seg_bytes = (size_t)seg_len * KB;
   for (unsigned long long seg = blockIdx.x; seg < nseg; seg += gridDim.x) {
-    // one thread reads the abort flag; its answer reaches the others through the barrier below,
-    // so the whole CTA leaves together
-    int stop = 0;
-    if (tid == 0) stop = (int)ld_relaxed(&ctrl->abort);
     const K* src = in + seg * seg_len;
-    const bool use_bulk = ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) && (seg_bytes % 16 == 0);
-    if (use_bulk) {
-      for (unsigned int e = seg_len + tid; e < TILE; e += THREADS) skeys[e] = pad;
-      int arrived = 1;
-      if (tid == 0 && !stop) {
-        fence_proxy_async();  // earlier generic accesses to the buffer are ordered before the copy
-        mbar_expect_tx(bar, (uint32_t)seg_bytes);
-        bulk_load(skeys, src, (uint32_t)seg_bytes, bar);
-        arrived = mbar_wait_bounded(bar, phase);  // one thread waits; the others park at the barrier
-      }
-      phase ^= 1u;
-      if (!__syncthreads_and(arrived && !stop)) {
-        if (tid == 0 && !stop) raise_timeout(ctrl);
-        return;
-      }
+    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+      const unsigned int nvec = (unsigned int)(seg_bytes / 16);
+      for (unsigned int v = tid; v < nvec; v += THREADS) reinterpret_cast<uint4*>(skeys)[v] = reinterpret_cast<const uint4*>(src)[v];
+      for (unsigned int e = nvec * (16 / KB) + tid; e < TILE; e += THREADS) skeys[e] = e < seg_len ? src[e] : pad;
     } else {
       for (unsigned int e = tid; e < TILE; e += THREADS) skeys[e] = e < seg_len ? src[e] : pad;
-      if (__syncthreads_or(stop)) return;
     }
+    __syncthreads();
 
     K key[ITEMS];
     unsigned int pay[PAIRS ? ITEMS : 1];

@@ -37,7 +37,7 @@ template <int KB, bool PAIRS> struct SegWarpWord {
 template <int KB, bool PAIRS, int VT, int GL>
 __global__ void __launch_bounds__(SW_WARPS * 32, KB == 8 ? (PAIRS ? 4 : 6) : PAIRS ? 7 : 8)
 segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out,
-               int64_t* idx_out, unsigned int seg_len, unsigned long long nseg, int xf, int64_t index_offset)
+               int64_t* idx_out, unsigned int seg_len, unsigned long long nseg, int xf, int64_t index_offset, unsigned int* status)
 {
   using K  = typename KeyOf<KB>::type;
   using WD = SegWarpWord<KB, PAIRS>;
@@ -58,6 +58,7 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
   const int row0 = (lane >> GL) * RT;          // first position of my row
   const bool gather = PAIRS && (KB >= 4 || xf == XF_FLOAT);  // keys come back through the positions
 
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;  // nothing here waits, so nothing can time out
   const unsigned long long nblk = (nseg + ROWS - 1) / ROWS;
   for (unsigned long long blk = (unsigned long long)blockIdx.x * SW_WARPS + warp; blk < nblk;
        blk += (unsigned long long)gridDim.x * SW_WARPS) {

@@ -17,6 +17,7 @@ from . import _lib
 class Runtime:
     def __init__(self) -> None:
         self._ws: dict[int, torch.Tensor] = {}
+        self._ws_status: dict[int, torch.Tensor] = {}
         self._sticky: dict[int, torch.Tensor] = {}
         self._comm = None
 
@@ -54,10 +55,12 @@ class Runtime:
             cur = torch.empty(max(int(nbytes), 1 << 16), dtype=torch.uint8, device=self.device)
             assert cur.data_ptr() % 256 == 0
             self._ws[dev] = cur
+            self._ws_status[dev] = cur[:4].view(torch.int32)   # the status word at its head
         return cur
 
     def release_workspace(self) -> None:
         self._ws.clear()
+        self._ws_status.clear()
 
     # --- device-side status of the sorts enqueued so far ------------------------------------
     def note_sort(self, ws: torch.Tensor) -> None:
@@ -68,7 +71,8 @@ class Runtime:
         acc = self._sticky.get(dev)
         if acc is None:
             acc = self._sticky[dev] = torch.zeros(1, dtype=torch.int32, device=self.device)
-        torch.maximum(acc, ws[:4].view(torch.int32), out=acc)
+        own = self._ws.get(dev) is ws
+        torch.maximum(acc, self._ws_status[dev] if own else ws[:4].view(torch.int32), out=acc)
 
     def raise_pending(self) -> None:
         """Called where a result reaches the host: raises if any sort since the last call reported
