@@ -165,6 +165,10 @@ __device__ __forceinline__ void st_relaxed(unsigned int* p, unsigned int v)
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Dependent launches (launch_chained): wait until the kernels before this one in the stream are done and
+// their writes visible.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count)
 {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

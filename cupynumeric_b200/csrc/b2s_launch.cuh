@@ -86,19 +86,45 @@ inline Radix1dLayout radix_1d_layout(size_t n, bool pairs)
   return l;
 }
 
-template <int KB, int XF, bool PAIRS, int SIZE = SWEEP_MEDIUM>
+// Launches a kernel that calls chain_wait() before it reads anything its predecessor in the stream wrote:
+// its launch and first instructions overlap the predecessor's end.  A sort of 10^5 keys is a chain of six
+// launches: float32 argsort 67 -> 53 us, float64 sort of 2^20 163 -> 142.  Letting the CTAs in earlier, as soon as
+// the predecessor's have all started, crowds them on the SMs that have room then: float64 sort of 2^20 194 us.
+// Beyond CHAIN_MAX keys the launches no longer matter, and a pass that takes its ticket only after the
+// wait loses more than it hides (Zipf int64 sort of 2^28 7.17 -> 7.29 ms; at 2^22 keys int64 argsort still
+// gains, 343 -> 320 us): those sorts, and segments, launch their passes the plain way.
+constexpr size_t CHAIN_MAX = (size_t)1 << 23;
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kern)(P...), unsigned int grid, unsigned int block, size_t smem, cudaStream_t stream, A... args)
+{
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim          = dim3(grid);
+  cfg.blockDim         = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream           = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs    = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+template <int KB, int XF, bool PAIRS, int SIZE = SWEEP_MEDIUM, bool CHAINED = false>
 inline cudaError_t launch_sweeps(Ctrl* ctrl, unsigned int* lookback, unsigned int tiles, SegGeom geo,
                                  int64_t index_offset, cudaStream_t stream)
 {
   using C   = SweepCfg<KB, PAIRS, SIZE>;
   using S   = SweepSmem<KB, PAIRS, C::THREADS, C::ITEMS, C::CHAINS>;
-  auto kern = onesweep_kernel<KB, XF, PAIRS, C::THREADS, C::ITEMS, C::CHAINS, C::MINCTAS, C::WINDOW>;
+  auto kern = onesweep_kernel<KB, XF, PAIRS, C::THREADS, C::ITEMS, C::CHAINS, C::MINCTAS, C::WINDOW, CHAINED>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::BYTES);
   if (e != cudaSuccess) return e;
   for (int pass = 0; pass < KB; ++pass) {
     prof::Scope ps(prof::K_SWEEP, stream);
-    kern<<<tiles, C::THREADS, S::BYTES, stream>>>(ctrl, lookback + (size_t)pass * tiles * RADIX, pass, geo,
-                                                  index_offset);
+    unsigned int* table = lookback + (size_t)pass * tiles * RADIX;
+    if (CHAINED) e = launch_chained(kern, tiles, C::THREADS, S::BYTES, stream, ctrl, table, pass, geo, index_offset);
+    else kern<<<tiles, C::THREADS, S::BYTES, stream>>>(ctrl, table, pass, geo, index_offset);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
@@ -162,20 +188,23 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
     hist_kernel<KB, XF><<<hgrid, HIST_THREADS, 0, stream>>>(static_cast<const K*>(in), n, ctrl, ra);
   }
   const SegGeom geo{n, lay.tiles, 1u, KB, nullptr};
-  auto sweeps = [&](auto size) {
-    constexpr int SIZE = decltype(size)::value;
-    return pairs ? launch_sweeps<KB, XF, true, SIZE>(ctrl, lb, lay.tiles, geo, index_offset, stream)
-                 : launch_sweeps<KB, XF, false, SIZE>(ctrl, lb, lay.tiles, geo, index_offset, stream);
+  auto sweeps = [&](auto size, auto chained) {
+    constexpr int SIZE     = decltype(size)::value;
+    constexpr bool CHAINED = decltype(chained)::value;
+    return pairs ? launch_sweeps<KB, XF, true, SIZE, CHAINED>(ctrl, lb, lay.tiles, geo, index_offset, stream)
+                 : launch_sweeps<KB, XF, false, SIZE, CHAINED>(ctrl, lb, lay.tiles, geo, index_offset, stream);
   };
-  e = n <= SMALL_MAX    ? sweeps(std::integral_constant<int, SWEEP_SMALL>{})
-      : n <= MEDIUM_MAX ? sweeps(std::integral_constant<int, SWEEP_MEDIUM>{})
-                        : sweeps(std::integral_constant<int, SWEEP_LARGE>{});
+  e = n <= SMALL_MAX    ? sweeps(std::integral_constant<int, SWEEP_SMALL>{}, std::true_type{})
+      : n <= MEDIUM_MAX ? sweeps(std::integral_constant<int, SWEEP_MEDIUM>{}, std::true_type{})
+      : n <= CHAIN_MAX  ? sweeps(std::integral_constant<int, SWEEP_LARGE>{}, std::true_type{})
+                        : sweeps(std::integral_constant<int, SWEEP_LARGE>{}, std::false_type{});
   if (e != cudaSuccess) return e;
   unsigned int fgrid = (n + 256 * 16 - 1) / (256 * 16);
   if (fgrid > (unsigned int)sms * 8) fgrid = sms * 8;
   {
     prof::Scope ps(prof::K_FIXUP, stream);
-    fixup_kernel<<<fgrid, 256, 0, stream>>>(ctrl, n, index_offset);
+    e = launch_chained(fixup_kernel, fgrid, 256, 0, stream, ctrl, n, index_offset);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }

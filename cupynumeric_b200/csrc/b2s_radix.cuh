@@ -408,6 +408,7 @@ __device__ __forceinline__ void fixup_body(const FixDesc& f, unsigned int n, int
 // radix pass it cost the keys-only passes 5 % (measured), far more than the launch.
 static __global__ void __launch_bounds__(256) fixup_kernel(const Ctrl* ctrl, unsigned int n, int64_t index_offset)
 {
+  chain_wait();
   fixup_body(ctrl->fix, n, index_offset, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 }
 
@@ -519,7 +520,7 @@ struct SegGeom {
   const unsigned int* seg_bases;  // [nseg][npass][RADIX] exclusive digit bases, or null
 };
 
-template <int KB, int XF, bool PAIRS, int THREADS, int ITEMS, int CHAINS, int MIN_CTAS, int WINDOW>
+template <int KB, int XF, bool PAIRS, int THREADS, int ITEMS, int CHAINS, int MIN_CTAS, int WINDOW, bool CHAINED>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS)
 onesweep_kernel(Ctrl* ctrl, unsigned int* __restrict__ lookback, int pass, SegGeom geo, int64_t index_offset)
 {
@@ -530,9 +531,6 @@ onesweep_kernel(Ctrl* ctrl, unsigned int* __restrict__ lookback, int pass, SegGe
   constexpr int IPC   = ITEMS / CHAINS;  // items per chain
   static_assert(THREADS >= RADIX, "one thread per digit is needed for the look-back");
   static_assert(ITEMS % CHAINS == 0, "chains split the items evenly");
-
-  const PassDesc pd = ctrl->pass[pass];
-  if (!pd.active) return;
 
   extern __shared__ __align__(128) unsigned char smem[];
   K* stage_keys          = reinterpret_cast<K*>(smem);
@@ -548,15 +546,31 @@ onesweep_kernel(Ctrl* ctrl, unsigned int* __restrict__ lookback, int pass, SegGe
   const int shift   = pass * RADIX_BITS;
   const DigitSel ds = make_digit_sel<KB, XF>(pass);
 
+  auto clear_counters = [&] {
+    for (int i = tid; i < (ROWS + (B2S_RANK_ATOMIC ? S::WARPS : 0)) * RADIX; i += THREADS) hist[i] = 0;
+  };
+  if (CHAINED) {
+    // what needs nothing from the kernel before runs while that one drains
+    clear_counters();
+    if (tid == 0) {
+      mbar_init(bar, 1);
+      fence_mbar_init();
+    }
+    chain_wait();
+  }
+  const PassDesc pd = ctrl->pass[pass];
+  if (!pd.active) return;
   if (tid == 0) {
     // one thread reads the abort flag for the whole CTA, so that all of its threads leave together
     const unsigned int ticket = atomicAdd(&ctrl->tile_counter[pass], 1u);
     misc[1] = ld_relaxed(&ctrl->abort);
     misc[0] = ticket;
-    mbar_init(bar, 1);
-    fence_mbar_init();
+    if (!CHAINED) {
+      mbar_init(bar, 1);
+      fence_mbar_init();
+    }
   }
-  for (int i = tid; i < (ROWS + (B2S_RANK_ATOMIC ? S::WARPS : 0)) * RADIX; i += THREADS) hist[i] = 0;
+  if (!CHAINED) clear_counters();  // (while the ticket is on its way)
   __syncthreads();
   if (misc[1]) return;
   const unsigned int tile = misc[0];
