@@ -146,8 +146,9 @@ template <int KB, int NB> struct RowBuckets {
     const K a = KB == 8 ? (K)((unsigned long long)lo << 32) : (K)lo;
     const K b = KB == 8 ? (K)(((unsigned long long)hi << 32) | 0xFFFFFFFFull) : (K)hi;
     fmin      = value(sm_from_ordered<KB>(a, XF_FLOAT));
-    fscale    = (F)NB / (value(sm_from_ordered<KB>(b, XF_FLOAT)) - fmin);
-    ok        = lo <= hi && fscale > (F)0 && fscale < (F)(KB == 8 ? 1e300 : 1e37f);
+    // a rough quotient will do: any positive scale keeps the order, and buckets are clamped
+    fscale    = (F)__fdividef((float)NB, (float)(value(sm_from_ordered<KB>(b, XF_FLOAT)) - fmin));
+    ok        = lo <= hi && fscale > (F)0 && fscale < (F)1e37f;
     exact     = false;
   }
   __device__ __forceinline__ unsigned int bucket_float(K o) const
@@ -169,13 +170,13 @@ template <int KB, int NB> struct RowBuckets {
     imin  = lo;
     exact = range < NB;
     shift = KB == 8 && (range >> 32) != 0 ? 32 - __clz((int)(range >> 32)) : 0;
-    mult  = exact ? 0u : (unsigned int)(((unsigned long long)NB << 32) / ((range >> shift) + 1));
+    mult  = exact ? 0u : __float2uint_rz(__fdividef((float)NB * 4294967296.0f, (float)(unsigned int)(range >> shift)));
     ok    = true;
   }
   __device__ __forceinline__ unsigned int bucket_image(K o) const
   {
     const unsigned int x = (unsigned int)((unsigned long long)(K)(o - imin) >> shift);
-    return exact ? x : __umulhi(x, mult);
+    return exact ? x : min(__umulhi(x, mult), (unsigned int)NB - 1);
   }
 };
 

@@ -48,6 +48,11 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
   constexpr W WMAX   = (W)~(W)0;
   __shared__ W sw_all[SW_WARPS * SPAN];
   __shared__ unsigned short sp_all[SIDE ? SW_WARPS * SPAN : 1];
+  // rows long enough for it are sorted by buckets first (b2s_segmerge.cuh): two 16-bit counters per element
+  constexpr bool BUCKETS = VT == 16 && GL >= 3;
+  constexpr int NB       = 2 * RT;
+  constexpr int CNT      = BUCKETS ? 32 * VT + 32 * VT / 8 : 4;  // words per warp, four spare ones after every 32
+  __shared__ __align__(16) unsigned int cnt_all[SW_WARPS * CNT];
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g    = lane & (G - 1);          // my place in the row's group
@@ -65,31 +70,25 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
     const unsigned long long base = blk * ROWS;
     const int rows = (int)(nseg - base < (unsigned long long)ROWS ? nseg - base : ROWS);
     const K* src   = in + base * seg_len;
-    // ---- load: consecutive lanes read consecutive elements ----
+    // ---- load: consecutive lanes read consecutive elements; element j of a lane is in row j * 32 / RT ----
     int special = 0;
+    K img[VT];
 #pragma unroll
     for (int j = 0; j < VT; ++j) {
       const int i = j * 32 + lane, r = i / RT, c = i % RT;
-      W w = WMAX;
-      if (r < rows && (unsigned int)c < seg_len) {
-        const K raw = src[r * seg_len + c];
-        if (!PAIRS) special |= sm_is_special<KB>(raw, xf) ? 1 : 0;
-        const K o = to_ordered_rt<KB>(raw, xf);
-        w         = PACK ? (W)(((W)o << (PACK ? WD::SHIFT : 0)) | (W)(unsigned int)c) : (W)o;
-      }
-      sw[at(i)] = w;
+      img[j]      = r < rows && (unsigned int)c < seg_len ? src[r * seg_len + c] : (K)0;
     }
-    if (!PAIRS) special = __any_sync(0xFFFFFFFFu, special);
-    __syncwarp();
-    W key[VT];
-    unsigned int pay[SIDE ? VT : 1];
 #pragma unroll
     for (int j = 0; j < VT; ++j) {
-      key[j] = sw[mine + j];
-      if (SIDE) pay[j] = g * VT + j;
+      const K raw = img[j];
+      img[j]      = to_ordered_rt<KB>(raw, xf);
+      if (!PAIRS && xf == XF_FLOAT) special |= sm_is_special<KB>(raw, xf) ? 1 : 0;  // (0 is not)
     }
-    // ---- my elements in registers ----
-    odd_even_merge_sort<VT, 1>([&](int a, int b) {
+    if (!PAIRS) special = __any_sync(0xFFFFFFFFu, special);
+    auto word_of = [&](K o, int c) { return PACK ? (W)(((W)o << (PACK ? WD::SHIFT : 0)) | (W)(unsigned int)c) : (W)o; };
+    W key[VT];
+    unsigned int pay[SIDE ? VT : 1];
+    auto cmp_swap = [&](int a, int b) {
       const W x = key[a], y = key[b];
       if (SIDE) {
         const unsigned int p = pay[SIDE ? a : 0], q = pay[SIDE ? b : 0];
@@ -103,10 +102,166 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
         key[a] = sw_ ? y : x;
         key[b] = sw_ ? x : y;
       }
-    });
+    };
+    auto read_words = [&](int first) {
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        key[j] = sw[at(first + j)];
+        if (SIDE) pay[SIDE ? j : 0] = sp[at(first + j)];
+      }
+    };
+    auto write_words = [&](int first) {
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        sw[at(first + j)] = key[j];
+        if (SIDE) sp[at(first + j)] = (unsigned short)pay[SIDE ? j : 0];
+      }
+    };
+    bool sorted = false;
+    if constexpr (BUCKETS) {
+      constexpr int PER = RT / 32;  // a lane's elements of one row
+      unsigned char* cnt = reinterpret_cast<unsigned char*>(cnt_all + warp * CNT);
+      for (int i = lane; i < CNT / 4; i += 32) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0u, 0u, 0u, 0u);
+      __syncwarp();
+      unsigned int br[VT];  // where the bucket's counter is | rank in the bucket << 16
+      int over = 0;
+#pragma unroll
+      for (int q = 0; q < ROWS; ++q) {
+        if (q < rows) {
+          auto mine_in = [&](int j) { return (unsigned int)((j * 32 + lane) % RT) < seg_len; };
+          RowBuckets<KB, NB> rb;
+          bool by_value = false;
+          if constexpr (KB >= 4) by_value = xf == XF_FLOAT;
+          if (by_value) {
+            unsigned int lo = 0xFFFFFFFFu, hi = 0;
+#pragma unroll
+            for (int j = q * PER; j < (q + 1) * PER; ++j) {
+              const unsigned int u = RowBuckets<KB, NB>::upper(img[j]);
+              if (mine_in(j) && u - RowBuckets<KB, NB>::FIN_LO < RowBuckets<KB, NB>::FIN_N) {
+                lo = min(lo, u);
+                hi = max(hi, u);
+              }
+            }
+            lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+            hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+            if constexpr (KB >= 4) rb.from_floats(lo, hi);
+          } else {
+            K lo = (K)~(K)0, hi = 0;
+#pragma unroll
+            for (int j = q * PER; j < (q + 1) * PER; ++j)
+              if (mine_in(j)) {
+                lo = img[j] < lo ? img[j] : lo;
+                hi = img[j] > hi ? img[j] : hi;
+              }
+            if constexpr (KB < 8) {
+              lo = (K)__reduce_min_sync(0xFFFFFFFFu, (unsigned int)lo);
+              hi = (K)__reduce_max_sync(0xFFFFFFFFu, (unsigned int)hi);
+            } else {
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) {
+                const K l = __shfl_xor_sync(0xFFFFFFFFu, lo, o), h = __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+                lo        = l < lo ? l : lo;
+                hi        = h > hi ? h : hi;
+              }
+            }
+            rb.from_images(lo, hi);
+          }
+          const bool counted = !PAIRS && rb.exact;  // a bucket holds equal keys, which need no order
+          if (!rb.ok) over = 1;
+          else {
+#pragma unroll
+            for (int j = q * PER; j < (q + 1) * PER; ++j)
+              if (mine_in(j)) {
+                unsigned int b = 0;
+                if constexpr (KB >= 4) b = by_value ? rb.bucket_float(img[j]) : rb.bucket_image(img[j]);
+                else b = rb.bucket_image(img[j]);
+                b += q * NB;
+                const unsigned int place = b * 2 + (b >> 6) * 16;  // of the bucket's 16 bits
+                const unsigned int h     = (b & 1u) * 16u;
+                const unsigned int r     = (atomicAdd(reinterpret_cast<unsigned int*>(cnt + (place & ~3u)), 1u << h) >> h) & 0xFFFFu;
+                over |= !counted && r >= (unsigned int)SM_BUCKET ? 1 : 0;
+                br[j] = place | (r << 16);
+              }
+          }
+        }
+      }
+      sorted = !__any_sync(0xFFFFFFFFu, over);
+      __syncwarp();
+      if (sorted) {
+        // counts -> places: my 32 buckets, then the lanes of my row before me
+        uint4* mine4     = reinterpret_cast<uint4*>(cnt) + 4 * lane + (lane >> 1);
+        unsigned int sum = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint4 c = mine4[j];
+          sum += c.x + c.y + c.z + c.w;  // two counts per word, added side by side
+        }
+        sum = (sum & 0xFFFFu) + (sum >> 16);
+        unsigned int incl = sum;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+          const unsigned int t = __shfl_up_sync(0xFFFFFFFFu, incl, o, G);
+          if (g >= o) incl += t;
+        }
+        unsigned int run = incl - sum;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4 c = mine4[j];
+          auto place = [&](unsigned int& two) {
+            const unsigned int first_n = two & 0xFFFFu, both = first_n + (two >> 16);
+            two = run | ((run + first_n) << 16);
+            run += both;
+          };
+          place(c.x);
+          place(c.y);
+          place(c.z);
+          place(c.w);
+          mine4[j] = c;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < VT; ++j) {
+          const int i = j * 32 + lane, r = i / RT, c = i % RT;
+          if (r < rows && (unsigned int)c < seg_len) {
+            const int p = r * RT + *reinterpret_cast<const unsigned short*>(cnt + (br[j] & 0xFFFFu)) + (int)(br[j] >> 16);
+            sw[at(p)]   = word_of(img[j], c);
+            if (SIDE) sp[at(p)] = (unsigned short)c;
+          } else {
+            sw[at(i)] = WMAX;
+            if (SIDE) sp[at(i)] = (unsigned short)c;
+          }
+        }
+        __syncwarp();
+        read_words(lane * VT);
+        odd_even_merge_sort<VT, 1>(cmp_swap);
+        write_words(lane * VT);
+        __syncwarp();
+        if (g < G - 1) {
+          read_words(lane * VT + VT / 2);
+          odd_even_merge_sort<VT, VT / 2>(cmp_swap);
+          write_words(lane * VT + VT / 2);
+        }
+        __syncwarp();
+        read_words(lane * VT);
+      }
+    }
+    if (!sorted) {
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        const int i = j * 32 + lane, r = i / RT, c = i % RT;
+        sw[at(i)]   = r < rows && (unsigned int)c < seg_len ? word_of(img[j], c) : WMAX;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        key[j] = sw[mine + j];
+        if (SIDE) pay[SIDE ? j : 0] = g * VT + j;
+      }
+      odd_even_merge_sort<VT, 1>(cmp_swap);
+    }
     // ---- merge rounds: runs of `run` elements, pairwise; my VT outputs start at g * VT of the row ----
 #pragma unroll 1
-    for (int run = VT; run < RT; run <<= 1) {
+    for (int run = sorted ? RT : VT; run < RT; run <<= 1) {
       __syncwarp();
 #pragma unroll
       for (int j = 0; j < VT; ++j) {

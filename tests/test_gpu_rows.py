@@ -79,6 +79,23 @@ def test_rows_of_one_block(cuda_device, dtype, how):
         assert_bit_equal(out, want, f"keys beside the indices {dtype} {how} 5x{seg}")
 
 
+@pytest.mark.parametrize("dtype", [np.uint8, np.int16, np.float16, np.int32, np.float32, np.int64, np.float64])
+@pytest.mark.parametrize("how", ["full", "bell", "outlier", "few", "cluster"])
+def test_rows_of_one_warp(cuda_device, dtype, how):
+    rng = np.random.default_rng(11)
+    for seg in (65, 100, 128, 129, 256, 300, 512):
+        a = _long_rows(rng, dtype, 9, seg, how)
+        if a.dtype.kind == "f":
+            a[seg:2 * seg] = np.nan if how == "few" else 2.5   # a row of one value
+        idx = np_task_sort(a, seg, True, 0, False)
+        want = a[np.arange(9).repeat(seg) * seg + idx]
+        out, _ = cabi_local_sort(a, seg, False, ndim_is_1=False)
+        assert_bit_equal(out, want, f"sort {dtype} {how} 9x{seg}")
+        out, got = cabi_local_sort(a, seg, True, ndim_is_1=False, want_keys_too=True, inplace=True)
+        assert np.array_equal(got, idx), f"argsort {dtype} {how} 9x{seg}"
+        assert_bit_equal(out, want, f"keys beside the indices {dtype} {how} 9x{seg}")
+
+
 def test_complex_rows_of_one_block(cuda_device):
     rng = np.random.default_rng(10)
     for seg in (600, 2000, 4097):
