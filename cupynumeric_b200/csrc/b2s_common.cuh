@@ -301,6 +301,9 @@ template <int KB, int XF>
 __device__ __forceinline__ unsigned int digit_fast(typename KeyOf<KB>::type raw, const DigitSel& s, int shift)
 {
   if (XF == XF_FLOAT) {
+    // one byte permutation in place of a shift and a mask (float32 argsort of 2^28 5.86 -> 5.81 ms, sort of 2^27
+    // 2.51 -> 2.48); the same on the chosen half of an 8-byte image slowed float64 by 4 %
+    if (KB == 4) return __byte_perm((unsigned int)to_ordered<KB, XF>(raw), 0u, s.prmt);
     return (unsigned int)(to_ordered<KB, XF>(raw) >> shift) & (RADIX - 1);
   } else if (XF == XF_CFLOAT) {
     // passes 0-3 look at the imaginary part (high word in memory), passes 4-7 at the real part
