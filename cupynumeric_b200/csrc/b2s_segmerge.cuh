@@ -4,16 +4,17 @@
 // * Buckets.  A linear function of the key that never inverts the order maps the row's keys to twice as
 //   many buckets as there are keys; counting and a scan give every bucket its place, and what is left is
 //   the order inside the buckets.  If none holds more than nine keys, two sorting networks over 16
-//   neighbours (the second one halfway between the first one's blocks) finish the row.  About 90 thread
-//   instructions per key, whatever the key's width.
+//   neighbours (the second one halfway between the first one's blocks) finish the row.  About 160 thread
+//   instructions per 8-byte key.
 // * Merging, for rows whose keys crowd: every thread sorts 16 consecutive elements in registers, then
 //   log2(threads) rounds of pairwise merge-path merges run in one shared-memory buffer; about 480
 //   instructions per 8-byte key.  A row finds out after its counting step, a sixth of the work of merging.
 //
 // Both are bound by instruction issue and the shared-memory pipe, not by HBM.  2^24 elements with NaNs and
-// duplicates, merging only -> buckets: float64 rows of 4096 0.390 -> 0.211 ms, of 1000 0.321 -> 0.208;
-// float32 with positions, rows of 2000 0.345 -> 0.175 ms.  The registers the compiler may use (64 for 512
+// duplicates, merging only -> buckets: float64 rows of 4096 0.390 -> 0.171 ms, of 1000 0.321 -> 0.146;
+// float32 with positions, rows of 2000 0.345 -> 0.135 ms.  The registers the compiler may use (64 for 512
 // threads, 80 for 256, 100 below) are the measured best per block size.
+//
 // Stands, like the on-chip radix kernel beside it, for cub::DeviceSegmentedRadixSort and the
 // short-segment thrust sort (src/cupynumeric/sort/cub_sort.cuh:73-107,145-184,
 // src/cupynumeric/sort/thrust_sort.cuh:61-123).
@@ -443,8 +444,9 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
       W ka = ia < run ? sw[smpad(a0 + ia)] : WMAX, kb = ib < run ? sw[smpad(b0 + ib)] : WMAX;
 #pragma unroll
       for (int j = 0; j < SM_VT; ++j) {
-        // an exhausted run never wins; on equal images the lower run goes first
-        const bool take_a = ib >= run || (ia < run && ka <= kb);
+        // on equal words the lower run goes first; an exhausted run shows the largest word, which only its like
+        // ties with (beside positions of their own that would matter, so it must not win there)
+        const bool take_a = SIDE ? ib >= run || (ia < run && ka <= kb) : ka <= kb;
         key[j]            = take_a ? ka : kb;
         if (SIDE) pay[j] = sp[smpad(take_a ? a0 + ia : b0 + ib)];
         ia += take_a ? 1 : 0;
