@@ -428,9 +428,9 @@ inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx
                                  unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
 {
   // Short rows go to the warp kernel (2^24 float32 keys with positions, against the one-CTA-per-row radix
-  // kernel they took before: rows of 2 19.2 ms -> 0.09 ms, of 32 1.31 -> 0.16, of 100 0.47 -> 0.22, of 200
-  // 1.42 -> 0.25, of 512 0.34 -> 0.23).  One-byte rows of 65 to 128 stay with the radix kernel, which needs
-  // a single pass for them (0.140 ms against 0.146).
+  // and merge kernels they took before: rows of 2 19.2 ms -> 0.07 ms, of 32 1.31 -> 0.10, of 100 0.47 -> 0.17, of
+  // 200 1.42 -> 0.15, of 512 0.34 -> 0.12).  One-byte rows of 65 to 128 stay with the radix kernel, which
+  // needs a single pass for them (0.140 ms against 0.146 when this kernel still merged them).
   // Keys of a sort are mapped back from their images, which the complex64 image does not allow: those
   // rows are sorted with positions and the keys fetched through them.  So are keys below 4 bytes, whose
   // words have room for the position anyway.

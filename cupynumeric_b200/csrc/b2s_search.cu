@@ -18,7 +18,8 @@ constexpr int SS_SAMPLES = 4096;
 // searches there; only the levels below go to memory.  A warp's 32 probes at different places of
 // memory cost the L1 a lookup each, 32 cycles per level, while shared memory answers 32 random
 // probes in about 3.5: that, and not the bytes, is what bounds a search without the samples, even though
-// its upper levels sit in the L1.  More samples would cost each CTA more to fetch than they save.
+// its upper levels sit in the L1 (10^6 values in 2^24 doubles: 114 us, 94 with the samples).  More samples
+// would cost each CTA more to fetch than they save.
 // STORE: the tile is the whole array, positions are stored; else they are combined with what is there.
 template <int KB, bool STORE>
 __global__ void __launch_bounds__(SS_THREADS)

