@@ -434,8 +434,9 @@ inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx
   // Keys of a sort are mapped back from their images, which the complex64 image does not allow: those
   // rows are sorted with positions and the keys fetched through them.  So are keys below 4 bytes, whose
   // words have room for the position anyway.
-  if (KB == 1 && seg_len > 64 && seg_len <= 128)
-    return segsort_cfg<KB, PAIRS, 32, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
+  if constexpr (KB == 1)
+    if (seg_len > 64 && seg_len <= 128)
+      return segsort_cfg<KB, PAIRS, 32, 4>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
   if (seg_len <= SW_MAX) {
     if constexpr (PAIRS || KB < 4) {
       return segwarp_any<KB, true>(xf, in, out, idx_out, seg_len, nseg, index_offset, status, stream);
