@@ -18,6 +18,8 @@ struct UniqueCtrl {
   unsigned long long total;  // heads in the whole array, written by the last tile
   unsigned int ticket;       // next tile
   unsigned int status;       // 0 or DEV_ERR_TIMEOUT
+  unsigned int spin_limit;   // 0: SPIN_LIMIT; else the poll limit of the look-back wait (self-test)
+  unsigned int pad_;
 };
 constexpr unsigned long long UQ_AGG = 1ull << 62, UQ_INCL = 2ull << 62, UQ_VALUE = UQ_AGG - 1;
 
@@ -92,7 +94,7 @@ unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int x
     if (tile != 0) {
       if (lane == 0) st_relaxed64(state + tile, UQ_AGG | mine);
       long long t        = (long long)tile - 1 - lane;
-      unsigned int spins = 0;
+      unsigned int spins = 0, spin_cap = SPIN_LIMIT;
       while (true) {
         const unsigned long long v  = t >= 0 ? ld_relaxed64(state + t) : UQ_INCL;
         const unsigned int missing  = __ballot_sync(0xFFFFFFFFu, v == 0);
@@ -108,10 +110,16 @@ unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int x
         t -= used;
         if (stop < gap) break;
         if (used == 0) {
-          if (++spins > SPIN_LIMIT || ((spins & 1023u) == 0 && ld_relaxed(&ctrl->status) != 0)) {
-            if (lane == 0) atomicMax(&ctrl->status, DEV_ERR_TIMEOUT);
-            break;
+          // one lane decides for the warp: the status may change between two lanes' loads of it, and lanes
+          // that left would be missing from the votes of those that stayed
+          ++spins;
+          int give_up = 0;
+          if (lane == 0) {
+            if (spins == 1 && ctrl->spin_limit != 0) spin_cap = ctrl->spin_limit;
+            give_up = spins > spin_cap || ((spins & 1023u) == 0 && ld_relaxed(&ctrl->status) != 0);
+            if (give_up) atomicMax(&ctrl->status, DEV_ERR_TIMEOUT);
           }
+          if (__shfl_sync(0xFFFFFFFFu, give_up, 0)) break;
           if (spins > 4) __nanosleep(64);
         }
       }
@@ -129,19 +137,39 @@ unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int x
     if ((bal[j] >> lane) & 1u) dst[heads[j * UQ_WARPS + w] + __popc(bal[j] & ((1u << lane) - 1))] = key[j];
 }
 
+// skip > 0 (self-test): the first `skip` tiles are left to nobody, and waits give up after spin_limit polls.
 template <int KB>
-static cudaError_t unique_launch(const void* a, long long n, int xf, void* out, unsigned char* ws, cudaStream_t stream)
+static cudaError_t unique_launch(const void* a, long long n, int xf, void* out, unsigned char* ws, cudaStream_t stream,
+                                 unsigned int skip = 0, unsigned int spin_limit = 0)
 {
   using K = typename KeyOf<KB>::type;
   const long long ntiles = (n + UQ_TILE - 1) / UQ_TILE;
   UniqueCtrl* ctrl          = reinterpret_cast<UniqueCtrl*>(ws);
   unsigned long long* state = reinterpret_cast<unsigned long long*>(ws + 256);
-  const cudaError_t e       = cudaMemsetAsync(ws, 0, 256 + (size_t)ntiles * 8, stream);
+  cudaError_t e             = cudaMemsetAsync(ws, 0, 256 + (size_t)ntiles * 8, stream);
   if (e != cudaSuccess) return e;
+  if (skip != 0) {
+    UniqueCtrl start{};
+    start.ticket     = skip;
+    start.spin_limit = spin_limit;
+    e                = cudaMemcpyAsync(ctrl, &start, sizeof(start), cudaMemcpyHostToDevice, stream);
+    if (e != cudaSuccess) return e;
+  }
   prof::Scope ps(prof::K_DIST, stream);
-  unique_kernel<KB><<<(unsigned int)ntiles, UQ_THREADS, 0, stream>>>(static_cast<const K*>(a), n, xf, ctrl, state,
+  unique_kernel<KB><<<(unsigned int)(ntiles - skip), UQ_THREADS, 0, stream>>>(static_cast<const K*>(a), n, xf, ctrl, state,
                                                                     static_cast<K*>(out));
   return cudaGetLastError();
+}
+
+// Waits for the launch above and reads its result: a b2s_status_t, and the number of heads.
+static int unique_result(const unsigned char* ws, size_t* out_len, cudaStream_t stream)
+{
+  UniqueCtrl done{};
+  if (cudaMemcpyAsync(&done, ws, sizeof(done), cudaMemcpyDeviceToHost, stream) != cudaSuccess) return B2S_ERR_CUDA;
+  if (cudaStreamSynchronize(stream) != cudaSuccess) return B2S_ERR_CUDA;
+  if (done.status != 0) return (int)done.status;
+  *out_len = (size_t)done.total;
+  return B2S_OK;
 }
 
 }  // namespace b2s
@@ -194,11 +222,22 @@ int b2s_unique_sorted(int dtype, const void* sorted, size_t n, void* out, size_t
     default: e = unique_launch<8>(sorted, (long long)n, xf, out, w, stream); break;
   }
   if (e != cudaSuccess) return B2S_ERR_CUDA;
-  UniqueCtrl done{};
-  if (cudaMemcpyAsync(&done, w, sizeof(done), cudaMemcpyDeviceToHost, stream) != cudaSuccess) return B2S_ERR_CUDA;
-  if (cudaStreamSynchronize(stream) != cudaSuccess) return B2S_ERR_CUDA;
-  if (done.status != 0) return (int)done.status;
-  *out_len = (size_t)done.total;
-  return B2S_OK;
+  return unique_result(w, out_len, stream);
+}
+
+int b2s_selftest_unique_timeout(void* ws, size_t ws_bytes, void* cuda_stream)
+{
+  // 40 tiles of equal keys: more than one look-back window
+  constexpr size_t N = (size_t)UQ_TILE * 40;
+  size_t need        = 0;
+  b2s_unique_workspace_bytes(N, &need);
+  if (ws == nullptr || ws_bytes < need + 2 * N * 4 || (reinterpret_cast<uintptr_t>(ws) & 255u)) return B2S_ERR_WORKSPACE;
+  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  unsigned char* w    = static_cast<unsigned char*>(ws);
+  unsigned char* keys = w + need;
+  if (cudaMemsetAsync(keys, 0, N * 4, stream) != cudaSuccess) return B2S_ERR_CUDA;
+  if (unique_launch<4>(keys, (long long)N, XF_UNSIGNED, keys + N * 4, w, stream, 1, 4096) != cudaSuccess) return B2S_ERR_CUDA;
+  size_t heads = 0;
+  return unique_result(w, &heads, stream);
 }
 }

@@ -308,6 +308,13 @@ int b2s_unique_workspace_bytes(size_t n, size_t* bytes);
 int b2s_unique_sorted(int dtype, const void* sorted, size_t n, void* out, size_t* out_len, void* ws,
                       size_t ws_bytes, void* cuda_stream);
 
+/* Self-test of the wait in b2s_unique_sorted (a tile waits for the counts of the tiles before it): runs the
+ * same kernel over keys of the library's own with the first tile left out and a poll limit of a few
+ * thousand, so that the wait runs out within milliseconds.  Answers what b2s_unique_sorted would:
+ * B2S_ERR_TIMEOUT.  The workspace, the stream and the context stay usable.  `ws`: at least 2 MiB, 256-byte
+ * aligned. */
+int b2s_selftest_unique_timeout(void* ws, size_t ws_bytes, void* cuda_stream);
+
 /* ---- PARTITION by selection, LEXSORT over several keys --------------------------------------- */
 
 /* Partitions a 1-D tile around its element of rank `kth` (0-based, in the sort's total order)

@@ -52,3 +52,16 @@ def test_unique_reports_the_count_of_every_head(cuda_device):
     _lib.check(lib.b2s_unique_sorted(_lib.DTYPE_CODE[np.dtype(np.int64)], a.data_ptr(), n, out.data_ptr(), ctypes.byref(count),
                                      ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), "unique")
     assert count.value == n and torch.equal(out, a)
+
+
+def test_unique_reports_a_wait_that_runs_out(cuda_device):
+    """The library's own self-test: the first tile is processed by nobody, so the chain over the tiles gives
+    up after a few thousand polls.  The workspace serves a correct call afterwards."""
+    lib, stream = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    ws = torch.empty(2 << 20, dtype=torch.uint8, device="cuda")
+    assert lib.b2s_selftest_unique_timeout(ws.data_ptr(), ws.numel(), stream) == 5   # B2S_ERR_TIMEOUT
+    a = torch.arange(4096 * 40, dtype=torch.int32, device="cuda") // 3
+    out, count = torch.empty_like(a), ctypes.c_size_t()
+    _lib.check(lib.b2s_unique_sorted(_lib.DTYPE_CODE[np.dtype(np.int32)], a.data_ptr(), a.numel(), out.data_ptr(),
+                                     ctypes.byref(count), ws.data_ptr(), ws.numel(), stream), "unique")
+    assert torch.equal(out[:count.value], torch.unique(a))
