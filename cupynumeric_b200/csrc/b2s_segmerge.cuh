@@ -13,7 +13,12 @@
 // Both are bound by instruction issue and the shared-memory pipe, not by HBM.  2^24 elements with NaNs and
 // duplicates, merging only -> buckets: float64 rows of 4096 0.390 -> 0.171 ms, of 1000 0.321 -> 0.146;
 // float32 with positions, rows of 2000 0.345 -> 0.135 ms.  The registers the compiler may use (64 for 512
-// threads, 80 for 256, 100 below) are the measured best per block size.
+// threads, 80 for 256, 100 below) are the measured best per block size for the sort of keys and for 4-byte keys;
+// 8-byte keys with positions need 124 KB of shared memory for 512 threads, so that one block is all an SM
+// takes, and get the registers of two (2^22 int64 in rows of 8192, three values, argsort 6 to 18 % faster).
+//
+// A row is merged where its keys crowd: heavy duplicates in an argsort, an outlier that takes most buckets for
+// itself, doubles whose spread is below 1e-33 or above float32's range (the scale is computed in float32).
 //
 // Stands, like the on-chip radix kernel beside it, for cub::DeviceSegmentedRadixSort and the
 // short-segment thrust sort (src/cupynumeric/sort/cub_sort.cuh:73-107,145-184,
@@ -132,6 +137,7 @@ template <int KB, int NB> struct RowBuckets {
   F fmin, fscale;
   K imin;
   unsigned int mult;
+  unsigned int range;  // exact: the last bucket in use
   int shift;
   bool ok, exact;  // exact: a bucket holds equal keys only
 
@@ -167,11 +173,12 @@ template <int KB, int NB> struct RowBuckets {
   // from the smallest and largest images
   __device__ __forceinline__ void from_images(K lo, K hi)
   {
-    const unsigned long long range = (unsigned long long)hi - (unsigned long long)lo;
+    const unsigned long long span = (unsigned long long)hi - (unsigned long long)lo;
     imin  = lo;
-    exact = range < NB;
-    shift = KB == 8 && (range >> 32) != 0 ? 32 - __clz((int)(range >> 32)) : 0;
-    mult  = exact ? 0u : __float2uint_rz(__fdividef((float)NB * 4294967296.0f, (float)(unsigned int)(range >> shift)));
+    range = (unsigned int)span;
+    exact = span < NB;
+    shift = KB == 8 && (span >> 32) != 0 ? 32 - __clz((int)(span >> 32)) : 0;
+    mult  = exact ? 0u : __float2uint_rz(__fdividef((float)NB * 4294967296.0f, (float)(unsigned int)(span >> shift)));
     ok    = true;
   }
   __device__ __forceinline__ unsigned int bucket_image(K o) const
@@ -186,7 +193,7 @@ enum : int { SM_INT = 0, SM_FLOAT = 1, SM_COMPLEX = 2 };
 
 // One CTA sorts one row at a time (grid-stride over rows); seg_len <= THREADS * 16.
 template <int KB, bool PAIRS, int THREADS, int FORM>
-__global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : THREADS == 256 ? 3 : THREADS == 128 ? 5 : 10)
+__global__ void __launch_bounds__(THREADS, THREADS == 512 ? (PAIRS && KB == 8 ? 1 : 2) : THREADS == 256 ? 3 : THREADS == 128 ? 5 : 10)
 segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out /* may be `in`: no __restrict__ */, int64_t* idx_out, unsigned int seg_len, unsigned long long nseg, int xf, int64_t index_offset,
                 unsigned int* __restrict__ status)
 {
@@ -333,8 +340,10 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
       // done once it is counted
       const bool counted = !PAIRS && rb.exact;
       unsigned int br[SM_VT];  // where the bucket's counter is | rank in the bucket << 16
-      int over = rb.ok ? 0 : 1;
-      if (rb.ok) {
+      // fewer values than a ninth of the row: some bucket is too full, whatever the row holds
+      const bool full = PAIRS && rb.exact && (rb.range + 1) * SM_BUCKET < seg_len;
+      int over = rb.ok && !full ? 0 : 1;
+      if (!over) {
 #pragma unroll
         for (int j = 0; j < SM_VT; ++j) {
           if ((unsigned int)(j * THREADS + tid) < seg_len) {
@@ -425,10 +434,17 @@ segmerge_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* ou
       }
       __syncthreads();
       read_words(first);
-      odd_even_merge_sort<SM_VT, 1>(cmp_swap);
-      __syncthreads();  // everybody holds its elements: the buffer may be rewritten
-      write_words(first);
-      __syncthreads();
+      // rows of one value (which the buckets of floats and complex keys do not tell from crowded ones) and rows
+      // that come in order have nothing to sort
+      int back = tid < THREADS - 1 && sw[smpad(first + SM_VT)] < key[SM_VT - 1] ? 1 : 0;
+#pragma unroll
+      for (int j = 0; j + 1 < SM_VT; ++j) back |= key[j + 1] < key[j] ? 1 : 0;
+      sorted = !__syncthreads_or(back);  // (and everybody holds its elements: the buffer may be rewritten)
+      if (!sorted) {
+        odd_even_merge_sort<SM_VT, 1>(cmp_swap);
+        write_words(first);
+        __syncthreads();
+      }
     }
     // ---- merge rounds: runs of `run` elements, pairwise; my 16 outputs start at `first` ----
     for (int run = sorted ? TILE : SM_VT; run < TILE; run <<= 1) {

@@ -103,3 +103,37 @@ def test_complex_rows_of_one_block(cuda_device):
         idx = complex_lex_argsort(a, seg)
         out, _ = cabi_local_sort(a, seg, False, ndim_is_1=False)
         assert_bit_equal(out, a[np.arange(5).repeat(seg) * seg + idx], f"sort 5x{seg}")
+
+
+def _crowded_rows(dtype, seg, how, rng):
+    """Rows for which counting by buckets is of no use: one value, three values, already in order (an outlier
+    at the end takes most buckets), blocks of sixteen in order, and rows of all four kinds side by side."""
+    kinds = ["one", "three", "in order", "blocks"] if how == "mixed" else [how] * 7
+    rows = []
+    for k in (kinds * 2)[:7]:
+        if k == "one":
+            x = np.full(seg, 5.0)
+        elif k == "three":
+            x = rng.integers(0, 3, seg).astype(float)
+        else:
+            x = np.sort(rng.integers(0, 60, seg)).astype(float)
+            if k == "blocks":
+                for i in range(0, seg, 16):
+                    rng.shuffle(x[i:i + 16])
+            x[-1] = 1e9 if np.dtype(dtype).itemsize > 2 else 100.0
+        rows.append(x)
+    a = np.concatenate(rows)
+    return (a + 1j * np.tile(a[:seg], 7)).astype(dtype) if np.dtype(dtype).kind == "c" else a.astype(dtype)
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.float16, np.int32, np.float32, np.int64, np.float64, np.complex64])
+@pytest.mark.parametrize("how", ["one", "three", "in order", "blocks", "mixed"])
+def test_rows_whose_keys_crowd(cuda_device, dtype, how):
+    rng = np.random.default_rng(12)
+    for seg in (65, 128, 129, 200, 257, 512, 513, 1024, 2000, 4096, 4097, 8192):
+        a = _crowded_rows(dtype, seg, how, rng)
+        idx = complex_lex_argsort(a, seg) if a.dtype.kind == "c" else np_task_sort(a, seg, True, 0, False)
+        out, _ = cabi_local_sort(a, seg, False, ndim_is_1=False)
+        assert_bit_equal(out, a[np.arange(7).repeat(seg) * seg + idx], f"sort {dtype} {how} 7x{seg}")
+        _, got = cabi_local_sort(a, seg, True, ndim_is_1=False)
+        assert np.array_equal(got, idx), f"argsort {dtype} {how} 7x{seg}"
