@@ -17,7 +17,7 @@
 // -> 0.153, of 512 (merged by a block before) 0.339 -> 0.230 -> 0.116; float64 rows of 200 3.05 -> 0.310 -> 0.215.
 // Rows whose keys crowd (heavy duplicates, an outlier) are merged; where counting cannot succeed it is left out, and
 // where the threads' blocks come in order so are the merge rounds: 2^22 int64 keys of one value in rows of 100,
-// argsort 87 -> 37 us (the radix kernel, which skips constant digits: 22), of three values 87 -> 79.
+// argsort 89 -> 44 us (the radix kernel, which skips constant digits: 24), of three values 88 -> 78 (47).
 // 16 elements per thread: the network costs 4 comparators per element, a merge round about 20 instructions,
 // and 16 words are what the registers of 28 warps per SM hold.  Up to 64 elements two merge rounds cost no
 // more than counting, scanning and placing.
@@ -58,6 +58,10 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
   // rows long enough for it are sorted by buckets first (b2s_segmerge.cuh): two 16-bit counters per element
   constexpr bool BUCKETS = VT == 16 && GL >= 3;
   constexpr int NB       = 2 * RT;
+  // 4-byte keys with positions are the form with the fewest registers to spare: leaving the counting out costs their
+  // evenly spread rows 5 %, looking for rows in order 4 % above 128 elements (nothing up to there)
+  constexpr bool FOUR_PAIRS = PAIRS && KB == 4;
+  constexpr bool CHECKS     = BUCKETS && !(FOUR_PAIRS && GL > 3);
   constexpr int CNT      = BUCKETS ? 32 * VT + 32 * VT / 8 : 4;  // words per warp, four spare ones after every 32
   __shared__ __align__(16) unsigned int cnt_all[SW_WARPS * CNT];
 
@@ -176,7 +180,7 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
           const bool counted = !PAIRS && rb.exact;  // a bucket holds equal keys, which need no order
           // fewer values than a ninth of the row: some bucket is too full, whatever the row holds (and a single
           // value would keep the counters waiting for each other)
-          const bool full = rb.exact && (PAIRS ? (rb.range + 1) * SM_BUCKET < seg_len : rb.range == 0);
+          const bool full = !FOUR_PAIRS && rb.exact && (PAIRS ? (rb.range + 1) * SM_BUCKET < seg_len : rb.range == 0);
           if (!rb.ok || full) over = 1;
           else {
 #pragma unroll
@@ -268,11 +272,12 @@ segwarp_kernel(const typename KeyOf<KB>::type* in, typename KeyOf<KB>::type* out
         if (SIDE) pay[SIDE ? j : 0] = g * VT + j;
       }
       odd_even_merge_sort<VT, 1>(cmp_swap);
-      if constexpr (BUCKETS) {
+      if constexpr (CHECKS) {
         // rows of one value (which the buckets of floats and complex keys do not tell from crowded ones) and rows
         // whose blocks come in order need no merging
-        const W next = __shfl_down_sync(0xFFFFFFFFu, key[0], 1);
-        sorted       = !__any_sync(0xFFFFFFFFu, g < G - 1 && next < key[VT - 1]);
+        sw[mine] = key[0];
+        __syncwarp();
+        sorted = !__any_sync(0xFFFFFFFFu, g < G - 1 && sw[mine + VT + 1] < key[VT - 1]);
       }
     }
     // ---- merge rounds: runs of `run` elements, pairwise; my VT outputs start at g * VT of the row ----
