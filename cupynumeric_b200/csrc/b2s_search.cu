@@ -9,47 +9,57 @@
 #include "b2s_common.cuh"
 #include "b2s_prof.h"
 
+#include <type_traits>
+
 namespace b2s {
 
-constexpr int SS_THREADS = 512;
-constexpr int SS_SAMPLES = 4096;
+constexpr int SS_SAMPLES  = 4096;
+constexpr size_t SS_MANY  = (size_t)1 << 19;  // values from which on a search goes through samples
+constexpr size_t SS_BYTES = (size_t)1 << 28;  // longest tile for which it does
 
-// Every CTA first puts SS_SAMPLES evenly spaced keys of the tile (their images) into shared memory and
+// SAMPLES > 0: every CTA first puts SS_SAMPLES evenly spaced keys of the tile (their images) into shared memory and
 // searches there; only the levels below go to memory.  A warp's 32 probes at different places of
 // memory cost the L1 a lookup each, 32 cycles per level, while shared memory answers 32 random
 // probes in about 3.5: that, and not the bytes, is what bounds a search without the samples, even though
 // its upper levels sit in the L1 (10^6 values in 2^24 doubles: 114 us, 94 with the samples).  More samples
 // would cost each CTA more to fetch than they save.
+// SAMPLES == 0: every value is searched for in memory from the start.
 // STORE: the tile is the whole array, positions are stored; else they are combined with what is there.
-template <int KB, bool STORE>
-__global__ void __launch_bounds__(SS_THREADS)
+template <int KB, bool STORE, int SAMPLES, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 searchsorted_kernel(const typename KeyOf<KB>::type* __restrict__ sorted, long long n, long long global_offset,
                     const typename KeyOf<KB>::type* __restrict__ values, long long num_values, int left, int xf,
                     long long* __restrict__ positions)
 {
   using K = typename KeyOf<KB>::type;
-  __shared__ K sample[SS_SAMPLES];
-  const long long step = (n + SS_SAMPLES - 1) / SS_SAMPLES;
-  const int m          = n > 0 ? (int)((n + step - 1) / step) : 0;
-  for (int k = threadIdx.x; k < m; k += SS_THREADS) sample[k] = to_ordered_rt<KB>(sorted[k * step], xf);
-  __syncthreads();
-  for (long long i = (long long)blockIdx.x * SS_THREADS + threadIdx.x; i < num_values; i += (long long)gridDim.x * SS_THREADS) {
+  __shared__ K sample[SAMPLES > 0 ? SAMPLES : 1];
+  const long long step = SAMPLES > 0 ? (n + SAMPLES - 1) / (SAMPLES > 0 ? SAMPLES : 1) : 0;
+  const int m          = SAMPLES > 0 && n > 0 ? (int)((n + step - 1) / step) : 0;
+  if (SAMPLES > 0) {
+    for (int k = threadIdx.x; k < m; k += THREADS) sample[k] = to_ordered_rt<KB>(sorted[k * step], xf);
+    __syncthreads();
+  }
+  for (long long i = (long long)blockIdx.x * THREADS + threadIdx.x; i < num_values; i += (long long)gridDim.x * THREADS) {
     const K v = to_ordered_rt<KB>(values[i], xf);
-    int below = 0, top = m;  // samples in front of the position
-    while (below < top) {
-      const int mid       = (below + top) >> 1;
-      const K k           = sample[mid];
-      const bool go_right = left ? (k < v) : (k <= v);
-      if (go_right) below = mid + 1; else top = mid;
+    long long lo = 0, hi = n;
+    if (SAMPLES > 0) {
+      int below = 0, top = m;  // samples in front of the position
+      while (below < top) {
+        const int mid       = (below + top) >> 1;
+        const K k           = sample[mid];
+        const bool go_right = left ? (k < v) : (k <= v);
+        if (go_right) below = mid + 1; else top = mid;
+      }
+      // the position lies behind sample below - 1 and not behind sample `below`
+      lo = below == 0 ? 0 : (below - 1) * step + 1;
+      hi = below == 0 ? 0 : (below * step < n ? below * step : n);
     }
-    // the position lies behind sample below - 1 and not behind sample `below`
-    long long lo = below == 0 ? 0 : (below - 1) * step + 1;
-    long long hi = below == 0 ? 0 : (below * step < n ? below * step : n);
-    const K* base      = sorted + lo;
-    unsigned int len   = (unsigned int)(hi - lo);  // (step of a tile of up to 2^44 keys fits)
-    unsigned int first = 0;
+    using Len     = typename std::conditional<SAMPLES != 0, unsigned int, long long>::type;  // (a step of up to 2^44 keys)
+    const K* base = sorted + lo;
+    Len len       = (Len)(hi - lo);
+    Len first     = 0;
     while (first < len) {
-      const unsigned int mid = (first + len) >> 1;
+      const Len mid          = first + ((len - first) >> 1);
       const K k              = to_ordered_rt<KB>(base[mid], xf);
       const bool go_right    = left ? (k < v) : (k <= v);
       if (go_right) first = mid + 1; else len = mid;
@@ -73,14 +83,25 @@ static cudaError_t searchsorted_launch(const void* sorted, size_t n, int64_t glo
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  size_t grid = (num_values + SS_THREADS - 1) / SS_THREADS;
-  if (grid > (size_t)sms * 4) grid = (size_t)sms * 4;  // all resident: the samples are fetched once per CTA
-  auto kern = whole ? searchsorted_kernel<KB, true> : searchsorted_kernel<KB, false>;
   prof::Scope ps(prof::K_DIST, stream);
-  kern<<<(unsigned int)grid, SS_THREADS, 0, stream>>>(static_cast<const K*>(sorted), (long long)n, global_offset,
-                                                       static_cast<const K*>(values), (long long)num_values, left, xf,
-                                                       reinterpret_cast<long long*>(positions));
-  return cudaGetLastError();
+  auto launch = [&](auto kern, int threads, size_t grid) {
+    kern<<<(unsigned int)grid, threads, 0, stream>>>(static_cast<const K*>(sorted), (long long)n, global_offset,
+                                                     static_cast<const K*>(values), (long long)num_values, left, xf,
+                                                     reinterpret_cast<long long*>(positions));
+    return cudaGetLastError();
+  };
+  // The samples pay where a CTA has several rounds of values for the ones it fetched, and where the probes below
+  // them find the tile in the L2: 10^5 values in 2^24 doubles take 19 us with them and 13 without, 2 * 10^5 26 and 20,
+  // 3 * 10^5 35 and 31, 2^20 95 and 110; in 2^26 doubles (512 MiB) 2^22 values take 1071 us with them and 994 without.
+  if (num_values >= SS_MANY && n <= SS_BYTES / KB) {
+    size_t grid = (num_values + 511) / 512;
+    if (grid > (size_t)sms * 4) grid = (size_t)sms * 4;  // all resident: the samples are fetched once per CTA
+    return whole ? launch(searchsorted_kernel<KB, true, SS_SAMPLES, 512>, 512, grid)
+                 : launch(searchsorted_kernel<KB, false, SS_SAMPLES, 512>, 512, grid);
+  }
+  size_t grid = (num_values + 255) / 256;
+  if (grid > (1ull << 30)) grid = 1ull << 30;
+  return whole ? launch(searchsorted_kernel<KB, true, 0, 256>, 256, grid) : launch(searchsorted_kernel<KB, false, 0, 256>, 256, grid);
 }
 
 }  // namespace b2s

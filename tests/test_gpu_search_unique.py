@@ -65,3 +65,31 @@ def test_unique_reports_a_wait_that_runs_out(cuda_device):
     _lib.check(lib.b2s_unique_sorted(_lib.DTYPE_CODE[np.dtype(np.int32)], a.data_ptr(), a.numel(), out.data_ptr(),
                                      ctypes.byref(count), ws.data_ptr(), ws.numel(), stream), "unique")
     assert torch.equal(out[:count.value], torch.unique(a))
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32, np.int64])
+@pytest.mark.parametrize("n", [1, 4095, 4097, 12_289, 300_001])
+def test_searchsorted_of_many_values(cuda_device, n, dtype):
+    """From 2^19 values on the upper levels are searched in samples."""
+    rng = np.random.default_rng(n)
+    for m in ((1 << 19) - 1, 1 << 19, (1 << 19) + 301):
+        a = np.sort(rng.integers(0, 200, n).astype(dtype) if dtype == np.uint8 else rng.integers(0, 2 * n, n).astype(dtype))
+        v = np.concatenate([a[:500], a[-500:], rng.integers(0, 250, m).astype(dtype)])[:m]
+        d_a, d_v = to_device(a), to_device(v)
+        for side in ("left", "right"):
+            want = np.searchsorted(a, v, side=side)
+            assert np.array_equal(num.searchsorted(a, v, side=side).to_numpy(), want), (m, side)
+            left = int(side == "left")
+            pos = torch.full((m,), n if left else 0, dtype=torch.int64, device="cuda")
+            _lib.check(_lib.lib().b2s_searchsorted(_lib.DTYPE_CODE[a.dtype], d_a.data_ptr(), n, 0, d_v.data_ptr(), m, left,
+                                                   pos.data_ptr(), torch.cuda.current_stream().cuda_stream), "b2s_searchsorted")
+            assert np.array_equal(pos.cpu().numpy(), want), (m, side)
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.int16, torch.float32, torch.int64])
+def test_unique_of_long_arrays(cuda_device, dtype):
+    """From 2^22 keys on the tiles are twice as long."""
+    for n in ((1 << 22) - 1, 1 << 22, (1 << 22) + 1, (1 << 22) + 8192, (1 << 22) + 8193):
+        for top in (3, 100 if dtype == torch.uint8 else 30_000):
+            a = torch.randint(0, top, (n,), device="cuda").to(dtype)
+            assert torch.equal(num.unique(num.array(a)).torch(), torch.unique(a)), (n, top)
