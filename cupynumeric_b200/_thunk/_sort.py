@@ -64,24 +64,35 @@ def sort_flattened(output: DeferredArray, input: DeferredArray, argsort: bool, s
     output.base, output.global_lo, output.tiled_axis = result.base, result.global_lo, result.tiled_axis
 
 
-# Shorter sides than this leave most of a transposed tile empty: torch's strided copy takes those.
-TRANSPOSE_MIN = 32
+def _transposes(size: int, batch: int, rows: int, cols: int) -> bool:
+    """Whether the tiled transpose is the faster copy of ``batch`` matrices of elements of ``size`` bytes.
+
+    Its tiles are 64 x 64 elements, and what they cost hardly depends on how full they are.  Measured against
+    torch's strided copy at 2^22 elements: many small matrices break even where the tiles are 0.7, 0.6, 0.5 and
+    0.6 full for 1, 2, 4 and 8 bytes (100000 x 32 x 32, a quarter full: uint8 448 against 181 us; 5000 x 64 x 100:
+    float32 54 against 91).  One long matrix pays from half full on, since torch reads a sector per element there
+    (float32 2^20 x 33: 74 against 632 us), but for bytes in short rows."""
+    if size > 8 or min(rows, cols) < 32:
+        return False
+    fill = rows * cols / (-(-rows // 64) * -(-cols // 64) * 4096)
+    long = batch == 1 and not (size == 1 and cols < 64)
+    return fill >= (0.5 if long else {1: 0.7, 2: 0.6, 4: 0.5, 8: 0.6}[size])
 
 
 def _transpose(moved: DeferredArray, input: DeferredArray, sort_axis: int) -> bool:
     """Fills ``moved`` with the dense copy of ``input`` whose last two axes are swapped, tile by tile
     through shared memory.  False (nothing done) where that is not the copy that is wanted: other axes, a
-    strided or conjugated input, 16-byte elements, short sides, more tiles than a grid holds."""
+    strided or conjugated input, shapes that torch copies faster, more tiles than a grid holds."""
     t = input.base
     if sort_axis != input.ndim - 2 or not t.is_contiguous() or t.is_conj() or t.is_neg() or not t.is_cuda:
         return False
     rows, cols = t.shape[-2:]
     size = t.element_size()
-    if size > 8 or min(rows, cols) < TRANSPOSE_MIN or t.numel() >= 1 << 40:
+    batch = t.numel() // max(rows * cols, 1)
+    if not _transposes(size, batch, rows, cols) or t.numel() >= 1 << 40:
         return False
     swapped = input.swapaxes(sort_axis, input.ndim - 1)
     out = torch.empty(swapped.shape, dtype=t.dtype, device=t.device)
-    batch = t.numel() // (rows * cols)
     _lib.check(_lib.lib().b2s_transpose(size, t.data_ptr(), out.data_ptr(), batch, rows, cols, runtime.stream_handle()),
                "b2s_transpose")
     moved.base = out

@@ -31,3 +31,22 @@ def test_sort_columns_of_a_strided_view(cuda_device):
     view = t[::2, 5:85]
     got = num.sort(num.array(view), axis=0).torch()
     assert torch.equal(got, torch.sort(view, dim=0).values)
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.int16, torch.float32, torch.int64])
+def test_transposed_matrices(cuda_device, dtype):
+    from cupynumeric_b200 import _lib
+
+    for shape in ((1, 64, 64), (3, 65, 129), (5, 33, 40), (7, 1, 200), (2, 200, 1)):
+        a = torch.randint(0, 100, shape, device="cuda").to(dtype)
+        out = torch.empty(shape[0], shape[2], shape[1], dtype=dtype, device="cuda")
+        _lib.check(_lib.lib().b2s_transpose(a.element_size(), a.data_ptr(), out.data_ptr(), *shape,
+                                            torch.cuda.current_stream().cuda_stream), "b2s_transpose")
+        assert torch.equal(out, a.transpose(1, 2)), shape
+
+
+@pytest.mark.parametrize("shape,axis", [((5, 64, 128), 1), ((70, 200, 64), 1), ((2000, 32, 32), 1), ((40, 33, 65), 1), ((33, 70_001), 0)])
+def test_sort_along_other_axes_on_either_side_of_the_rule(cuda_device, shape, axis):
+    for dtype in (torch.uint8, torch.int16, torch.int32, torch.float64):
+        a = torch.randint(0, 100, shape, device="cuda").to(dtype)
+        assert torch.equal(num.sort(num.array(a), axis=axis).torch(), torch.sort(a, dim=axis).values), (shape, dtype)

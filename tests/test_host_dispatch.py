@@ -87,3 +87,14 @@ def test_one_dim_tiles_carry_their_global_offset(cpu_point_task):
     out = create_deferred_thunk((3,), np.int64)
     out.sort(rhs, argsort=True, axis=0, kind="stable")
     assert out.base.tolist() == [101, 102, 100] and cpu_point_task[-1][3] == 100
+
+
+def test_the_transposed_copy_is_taken_where_its_tiles_are_full():
+    from cupynumeric_b200._thunk._sort import _transposes
+
+    assert _transposes(4, 1, 100_003, 257) and _transposes(4, 1, 1 << 20, 33) and _transposes(1, 1, 33, 1 << 20)
+    assert _transposes(8, 5000, 64, 100) and _transposes(2, 10, 64, 128)
+    for size in (1, 2, 4, 8):   # mostly empty tiles
+        assert not _transposes(size, 100_000, 32, 32) and not _transposes(size, 1000, 33, 65)
+    assert not _transposes(1, 1, 1 << 20, 33) and not _transposes(4, 1, 1 << 20, 31) and not _transposes(16, 1, 4096, 4096)
+    assert not _transposes(4, 0, 0, 64)
