@@ -10,8 +10,13 @@ namespace b2s {
 
 constexpr int UQ_THREADS = 256;
 constexpr int UQ_WARPS   = UQ_THREADS / 32;
-constexpr int UQ_ITEMS   = 16;
+constexpr int UQ_ITEMS   = 16;  // keys per thread of short arrays
 constexpr int UQ_TILE    = UQ_THREADS * UQ_ITEMS;
+// From here on a thread takes twice as many.  The chain over the tiles advances by about 50 of them per microsecond
+// whatever they hold, which bounds long arrays: 2^27 uint8 keys 660 -> 560 us, int64 with few distinct ones 712 ->
+// 588.  (A look-back of 128 tiles per round trip instead of 32 made it worse: 907 us.)  10^5 keys take 28 us with
+// the small tiles and 35 with the large ones.
+constexpr long long UQ_LONG = 1ll << 22;
 
 // Head of the workspace; one state word per tile follows (0: nothing yet).
 struct UniqueCtrl {
@@ -37,31 +42,32 @@ __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned lon
 // One pass over the sorted keys: a CTA takes the next tile (ticket), counts its heads, chains the count
 // to its predecessors (decoupled look-back, 32 tiles per round trip, one lane each) and writes its heads
 // in order.  Bound by memory: every key is read once from HBM (its left neighbour comes from the L1),
-// every head written once; counting, scanning and writing in three launches read the keys twice (33.5 M
-// int64 ids, an eighth of them heads, with the sort in front: 1154 -> 1120 us).
-template <int KB>
+// every head written once; counting, scanning and writing in three launches read the keys twice (2^25 float32
+// keys, most of them heads: 214 -> 170 us, few heads 197 -> 147; uint8 163 -> 145; int64 225 -> 209 and 190 -> 170).
+template <int KB, int ITEMS>
 __global__ void __launch_bounds__(UQ_THREADS)
 unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int xf, UniqueCtrl* ctrl,
               unsigned long long* __restrict__ state, typename KeyOf<KB>::type* __restrict__ out)
 {
   using K = typename KeyOf<KB>::type;
-  __shared__ unsigned int heads[UQ_ITEMS * UQ_WARPS];  // per group of 32 keys, in key order; then their prefix
+  constexpr int TILE = UQ_THREADS * ITEMS;
+  __shared__ unsigned int heads[ITEMS * UQ_WARPS];  // per group of 32 keys, in key order; then their prefix
   __shared__ unsigned int tile_sh;
   __shared__ unsigned long long before_sh;
   if (threadIdx.x == 0) tile_sh = atomicAdd(&ctrl->ticket, 1u);
   __syncthreads();
   const unsigned int tile = tile_sh;
-  const long long base    = (long long)tile * UQ_TILE;
+  const long long base    = (long long)tile * TILE;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  K key[UQ_ITEMS];
-  unsigned int bal[UQ_ITEMS];
+  K key[ITEMS];
+  unsigned int bal[ITEMS];
 #pragma unroll
-  for (int j = 0; j < UQ_ITEMS; ++j) {
+  for (int j = 0; j < ITEMS; ++j) {
     const long long i = base + j * UQ_THREADS + threadIdx.x;
     key[j]            = i < n ? a[i] : (K)0;
   }
 #pragma unroll
-  for (int j = 0; j < UQ_ITEMS; ++j) {
+  for (int j = 0; j < ITEMS; ++j) {
     const long long i = base + j * UQ_THREADS + threadIdx.x;
     const bool head   = i < n && (i == 0 || to_ordered_rt<KB>(key[j], xf) != to_ordered_rt<KB>(a[i - 1], xf));
     bal[j]            = __ballot_sync(0xFFFFFFFFu, head);
@@ -69,8 +75,8 @@ unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int x
   }
   __syncthreads();
   if (w == 0) {
-    // 128 counts, four consecutive ones per lane
-    constexpr int PER = UQ_ITEMS * UQ_WARPS / 32;
+    // one count per group, PER consecutive ones per lane
+    constexpr int PER = ITEMS * UQ_WARPS / 32;
     unsigned int c[PER], sum = 0;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
@@ -127,23 +133,23 @@ unique_kernel(const typename KeyOf<KB>::type* __restrict__ a, long long n, int x
     if (lane == 0) {
       st_relaxed64(state + tile, UQ_INCL | (before + mine));
       before_sh = before;
-      if (base + UQ_TILE >= n) ctrl->total = before + mine;
+      if (base + TILE >= n) ctrl->total = before + mine;
     }
   }
   __syncthreads();
   K* dst = out + before_sh;
 #pragma unroll
-  for (int j = 0; j < UQ_ITEMS; ++j)
+  for (int j = 0; j < ITEMS; ++j)
     if ((bal[j] >> lane) & 1u) dst[heads[j * UQ_WARPS + w] + __popc(bal[j] & ((1u << lane) - 1))] = key[j];
 }
 
 // skip > 0 (self-test): the first `skip` tiles are left to nobody, and waits give up after spin_limit polls.
-template <int KB>
-static cudaError_t unique_launch(const void* a, long long n, int xf, void* out, unsigned char* ws, cudaStream_t stream,
-                                 unsigned int skip = 0, unsigned int spin_limit = 0)
+template <int KB, int ITEMS>
+static cudaError_t unique_launch_items(const void* a, long long n, int xf, void* out, unsigned char* ws, cudaStream_t stream,
+                                       unsigned int skip, unsigned int spin_limit)
 {
   using K = typename KeyOf<KB>::type;
-  const long long ntiles = (n + UQ_TILE - 1) / UQ_TILE;
+  const long long ntiles    = (n + UQ_THREADS * ITEMS - 1) / (UQ_THREADS * ITEMS);
   UniqueCtrl* ctrl          = reinterpret_cast<UniqueCtrl*>(ws);
   unsigned long long* state = reinterpret_cast<unsigned long long*>(ws + 256);
   cudaError_t e             = cudaMemsetAsync(ws, 0, 256 + (size_t)ntiles * 8, stream);
@@ -156,9 +162,16 @@ static cudaError_t unique_launch(const void* a, long long n, int xf, void* out, 
     if (e != cudaSuccess) return e;
   }
   prof::Scope ps(prof::K_DIST, stream);
-  unique_kernel<KB><<<(unsigned int)(ntiles - skip), UQ_THREADS, 0, stream>>>(static_cast<const K*>(a), n, xf, ctrl, state,
-                                                                    static_cast<K*>(out));
+  unique_kernel<KB, ITEMS><<<(unsigned int)(ntiles - skip), UQ_THREADS, 0, stream>>>(static_cast<const K*>(a), n, xf, ctrl, state,
+                                                                                     static_cast<K*>(out));
   return cudaGetLastError();
+}
+
+template <int KB>
+static cudaError_t unique_launch(const void* a, long long n, int xf, void* out, unsigned char* ws, cudaStream_t stream)
+{
+  return n < UQ_LONG ? unique_launch_items<KB, UQ_ITEMS>(a, n, xf, out, ws, stream, 0, 0)
+                     : unique_launch_items<KB, 2 * UQ_ITEMS>(a, n, xf, out, ws, stream, 0, 0);
 }
 
 // Waits for the launch above and reads its result: a b2s_status_t, and the number of heads.
@@ -227,17 +240,20 @@ int b2s_unique_sorted(int dtype, const void* sorted, size_t n, void* out, size_t
 
 int b2s_selftest_unique_timeout(void* ws, size_t ws_bytes, void* cuda_stream)
 {
-  // 40 tiles of equal keys: more than one look-back window
-  constexpr size_t N = (size_t)UQ_TILE * 40;
+  // 80 tiles of equal keys, then 40 larger ones: more than one look-back window
+  constexpr size_t N = (size_t)UQ_TILE * 80;
   size_t need        = 0;
   b2s_unique_workspace_bytes(N, &need);
-  if (ws == nullptr || ws_bytes < need + 2 * N * 4 || (reinterpret_cast<uintptr_t>(ws) & 255u)) return B2S_ERR_WORKSPACE;
+  if (ws == nullptr || ws_bytes < need + 2 * N || (reinterpret_cast<uintptr_t>(ws) & 255u)) return B2S_ERR_WORKSPACE;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   unsigned char* w    = static_cast<unsigned char*>(ws);
   unsigned char* keys = w + need;
-  if (cudaMemsetAsync(keys, 0, N * 4, stream) != cudaSuccess) return B2S_ERR_CUDA;
-  if (unique_launch<4>(keys, (long long)N, XF_UNSIGNED, keys + N * 4, w, stream, 1, 4096) != cudaSuccess) return B2S_ERR_CUDA;
-  size_t heads = 0;
+  size_t heads        = 0;
+  if (cudaMemsetAsync(keys, 0, N, stream) != cudaSuccess) return B2S_ERR_CUDA;
+  if (unique_launch_items<1, UQ_ITEMS>(keys, (long long)N, XF_UNSIGNED, keys + N, w, stream, 1, 4096) != cudaSuccess) return B2S_ERR_CUDA;
+  const int rc = unique_result(w, &heads, stream);
+  if (rc != B2S_ERR_TIMEOUT) return rc;
+  if (unique_launch_items<1, 2 * UQ_ITEMS>(keys, (long long)N, XF_UNSIGNED, keys + N, w, stream, 1, 4096) != cudaSuccess) return B2S_ERR_CUDA;
   return unique_result(w, &heads, stream);
 }
 }
