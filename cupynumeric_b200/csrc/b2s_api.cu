@@ -322,8 +322,8 @@ int b2s_local_sort(int dtype, const void* keys_in, void* keys_out, int64_t* idx_
 
 // Self-test of the bounded waits.  Sorts a small array of its own whose first tile is never
 // processed (the tile tickets of the first pass start at 1), with a poll limit of a few thousand:
-// every later tile waits for the first tile's look-back entry, gives up within milliseconds,
-// records DEV_ERR_TIMEOUT and raises the abort flag; the remaining passes see the flag and
+// the tiles behind it wait for its look-back entry, give up within milliseconds,
+// record DEV_ERR_TIMEOUT and raise the abort flag; the remaining passes see the flag and
 // return.  Nothing traps, faults or waits without a bound; the workspace and the context stay usable.
 namespace b2s {
 __global__ void selftest_fill_kernel(uint32_t* keys, unsigned int n)
@@ -332,37 +332,57 @@ __global__ void selftest_fill_kernel(uint32_t* keys, unsigned int n)
 }
 }  // namespace b2s
 
-int b2s_selftest_wait_timeout(void* ws, size_t ws_bytes, void* cuda_stream)
+int b2s_selftest_wait_timeout_in(int which, void* ws, size_t ws_bytes, void* cuda_stream)
 {
-  constexpr unsigned int N = 1u << 16;  // 32 small tiles
-  const auto lay           = radix_1d_layout<4>(N, false);
-  const size_t need        = lay.total + 2 * (size_t)N * 4;
-  if (ws == nullptr || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u) != 0) return B2S_ERR_WORKSPACE;
+  if (which < SELFTEST_SHORT || which > SELFTEST_LONG) return B2S_ERR_INVALID_ARG;
+  // three rows of seven tiles, or one array of 32 small or 11 large ones
+  constexpr unsigned int ROW = 1u << 15, ROWS = 3, ONE = 1u << 16;
+  const bool rows      = which == SELFTEST_ROWS;
+  const unsigned int N = rows ? ROW * ROWS : ONE;
+  const auto seg       = radix_seg_layout<4>(ROW, ROWS, false);
+  const auto one       = radix_1d_layout<4>(ONE, false);
+  const size_t total   = rows ? seg.total : one.total;
+  const size_t *keys   = rows ? seg.off_keys : one.off_keys;
+  if (ws == nullptr || ws_bytes < total + 2 * (size_t)N * 4 || (reinterpret_cast<uintptr_t>(ws) & 255u) != 0) return B2S_ERR_WORKSPACE;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   unsigned char* base = static_cast<unsigned char*>(ws);
   Ctrl* ctrl          = reinterpret_cast<Ctrl*>(base);
-  uint32_t* in        = reinterpret_cast<uint32_t*>(base + lay.total);
+  uint32_t* in        = reinterpret_cast<uint32_t*>(base + total);
   uint32_t* out       = in + N;
-  unsigned int* lb    = reinterpret_cast<unsigned int*>(base + lay.off_lookback);
-  if (cudaMemsetAsync(base, 0, lay.off_keys[0], stream) != cudaSuccess) return B2S_ERR_CUDA;
+  unsigned int* lb    = reinterpret_cast<unsigned int*>(base + LOOKBACK_OFFSET);
+  unsigned int* sh    = reinterpret_cast<unsigned int*>(base + seg.off_seghist);
+  if (cudaMemsetAsync(base, 0, keys[0], stream) != cudaSuccess) return B2S_ERR_CUDA;
   selftest_fill_kernel<<<64, 256, 0, stream>>>(in, N);
   RouteArgs ra{};
   ra.keys_in     = in;
   ra.keys_out    = out;
-  ra.tmp_keys[0] = base + lay.off_keys[0];
-  ra.tmp_keys[1] = base + lay.off_keys[1];
+  ra.tmp_keys[0] = base + keys[0];
+  ra.tmp_keys[1] = base + keys[1];
   ra.n           = N;
   ra.npass       = 4;
   ra.key_bytes   = 4;
-  hist_kernel<4, XF_UNSIGNED><<<16, HIST_THREADS, 0, stream>>>(in, N, ctrl, ra);
+  if (rows) {
+    const unsigned int chunks = (ROW + SEG_HIST_CHUNK - 1) / SEG_HIST_CHUNK;
+    seg_hist_kernel<4, XF_UNSIGNED><<<ROWS * chunks, 256, 0, stream>>>(in, ROW, chunks, sh);
+    seg_scan_kernel<<<ROWS * 4, RADIX, 0, stream>>>(sh);
+    scan_route_kernel<<<1, RADIX, 0, stream>>>(ctrl, ra);
+  } else {
+    hist_kernel<4, XF_UNSIGNED><<<16, HIST_THREADS, 0, stream>>>(in, N, ctrl, ra);
+  }
   // the sabotage: the first pass hands out tickets 1, 2, ... so that tile 0 is never taken, and a
   // short poll limit
-  const unsigned int one = 1, limit = 4096;
-  if (cudaMemcpyAsync(&ctrl->tile_counter[0], &one, 4, cudaMemcpyHostToDevice, stream) != cudaSuccess) return B2S_ERR_CUDA;
+  const unsigned int first = 1, limit = 4096;
+  if (cudaMemcpyAsync(&ctrl->tile_counter[0], &first, 4, cudaMemcpyHostToDevice, stream) != cudaSuccess) return B2S_ERR_CUDA;
   if (cudaMemcpyAsync(&ctrl->spin_limit, &limit, 4, cudaMemcpyHostToDevice, stream) != cudaSuccess) return B2S_ERR_CUDA;
-  const SegGeom geo{N, lay.tiles, 1u, 4, nullptr};
-  const cudaError_t e = launch_sweeps<4, XF_UNSIGNED, false, SWEEP_SMALL>(ctrl, lb, lay.tiles, geo, 0, stream);
-  return e == cudaSuccess ? B2S_OK : B2S_ERR_CUDA;
+  constexpr unsigned int LARGE_TILE = SweepCfg<4, false, SWEEP_LARGE>::TILE;
+  const unsigned int tiles = rows ? seg.tiles : which == SELFTEST_LONG ? (ONE + LARGE_TILE - 1) / LARGE_TILE : one.tiles;
+  const SegGeom geo = rows ? SegGeom{ROW, seg.tiles_per_seg, ROWS, 4, sh} : SegGeom{ONE, tiles, 1u, 4, nullptr};
+  return selftest_sweeps(which, ctrl, lb, tiles, geo, stream) == cudaSuccess ? B2S_OK : B2S_ERR_CUDA;
+}
+
+int b2s_selftest_wait_timeout(void* ws, size_t ws_bytes, void* cuda_stream)
+{
+  return b2s_selftest_wait_timeout_in(SELFTEST_SHORT, ws, ws_bytes, cuda_stream);
 }
 
 int b2s_check_status(void* ws, void* cuda_stream)

@@ -50,6 +50,11 @@ template <int KB, bool PAIRS, int SIZE = SWEEP_MEDIUM> struct SweepCfg {
   static constexpr int WINDOW  = SIZE == SWEEP_SMALL ? 16 : LB_WINDOW;
 };
 
+// Where the look-back table of every workspace starts: behind the control block and nothing else, since the short
+// window of a first tile's successors reads that far in front of the table (look_back), without using what it finds.
+constexpr size_t LOOKBACK_OFFSET = (sizeof(Ctrl) + 255) / 256 * 256;
+static_assert(LOOKBACK_OFFSET >= (LB_WINDOW - 1) * RADIX * sizeof(unsigned int), "a short window may read the control block");
+
 struct Radix1dLayout {
   size_t off_lookback, lookback_used, off_keys[2], off_idx[2], total;
   unsigned int tiles;
@@ -70,7 +75,7 @@ inline Radix1dLayout radix_1d_layout(size_t n, bool pairs)
   size_t rows = tiles_of(n);
   if (n > SMALL_MAX && tiles_of(SMALL_MAX) > rows) rows = tiles_of(SMALL_MAX);
   if (n > MEDIUM_MAX && tiles_of(MEDIUM_MAX) > rows) rows = tiles_of(MEDIUM_MAX);
-  size_t off           = align_up(sizeof(Ctrl), 256);
+  size_t off           = LOOKBACK_OFFSET;
   l.off_lookback       = off;
   l.lookback_used      = align_up((size_t)KB * l.tiles * RADIX * sizeof(unsigned int), 256);
   off += align_up((size_t)KB * rows * RADIX * sizeof(unsigned int), 256);
@@ -223,7 +228,7 @@ inline RadixSegLayout radix_seg_layout(size_t seg_len, size_t nseg, bool pairs)
   l.tiles_per_seg         = (unsigned int)((seg_len + tile - 1) / tile);
   l.tiles                 = (unsigned int)(l.tiles_per_seg * nseg);
   const size_t volume     = seg_len * nseg;
-  size_t off              = align_up(sizeof(Ctrl), 256);
+  size_t off              = LOOKBACK_OFFSET;
   l.off_lookback          = off;
   off += align_up((size_t)KB * l.tiles * RADIX * sizeof(unsigned int), 256);
   l.off_seghist = off;
@@ -290,6 +295,11 @@ inline cudaError_t radix_seg_xf(const void* in, void* out, int64_t* idx_out, uns
   return cudaGetLastError();
 }
 
+// The self-test's way to the passes of uint32 keys as the sorts launch them: of short 1-D arrays (dependent launches),
+// of rows longer than SEG_CAP, of long 1-D arrays.
+enum : int { SELFTEST_SHORT = 0, SELFTEST_ROWS = 1, SELFTEST_LONG = 2 };
+cudaError_t selftest_sweeps(int which, Ctrl* ctrl, unsigned int* lookback, unsigned int tiles, SegGeom geo, cudaStream_t stream);
+
 // Segments of more than SEG_CAP elements (each below 2^30, fewer than 2^32 elements in all).
 template <int KB>
 cudaError_t launch_radix_seg(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
@@ -338,7 +348,7 @@ inline cudaError_t segsort_cfg(int xf, const void* in, void* out, int64_t* idx_o
   return cudaGetLastError();
 }
 
-// The merge-sort form of the on-chip row sort (4- and 8-byte keys, rows of more than 256 elements).
+// Rows of one block: buckets, merging where the keys crowd (4- and 8-byte keys, rows of more than 512 elements).
 template <int KB, bool PAIRS, int THREADS, int FORM>
 inline cudaError_t segmerge_cfg(int xf, const void* in, void* out, int64_t* idx_out, unsigned int seg_len,
                                 unsigned long long nseg, int64_t index_offset, unsigned int* status, cudaStream_t stream)
@@ -419,7 +429,7 @@ inline cudaError_t segmerge_any(int xf, const void* in, void* out, int64_t* idx_
 
 inline bool seg_merge_enabled()
 {
-  const char* e = std::getenv("B2S_SEG_MERGE");  // 0: keep every row on the radix kernel (comparisons)
+  const char* e = std::getenv("B2S_SEG_MERGE");  // 0: rows above 512 stay on the radix kernel (comparisons)
   return e == nullptr || e[0] != '0';
 }
 

@@ -446,13 +446,12 @@ constexpr int LB_WINDOW             = 4;         // predecessors inspected per r
 // always does, so the walk never leaves the segment.  WINDOW entries are loaded per round trip: the
 // loads are independent, so a run of tiles that have only published their counts costs one memory
 // latency per window.  A window may reach beyond the segment's first tile, `left` entries further down: it
-// then reads what lies in front (another segment's or pass's entries, or the control block, which is as
-// large as a short window), never to be counted; a longer window reads the first tile's entry again.
+// then reads what lies in front (another segment's or pass's entries, or the control block: LOOKBACK_OFFSET in
+// b2s_launch.cuh), never to be counted; a longer window reads the first tile's entry again.
 // The walk is on the critical path of every tile, and its instructions cost more of that than its loads:
 // hence the straight-line form (2^28 float32 argsort 5.92 -> 5.84 ms, Zipf int64 sort 7.50 -> 7.38 against a
 // branch per entry; windows of 8 and 16 were slower on long arrays).
 // Returns false when the poll limit ran out.
-static_assert(sizeof(Ctrl) >= (LB_WINDOW - 1) * RADIX * sizeof(unsigned int), "a short window may read the control block");
 template <int WINDOW>
 __device__ __forceinline__ bool look_back(const Ctrl* ctrl, const unsigned int* entry, int left, unsigned int* excl_out)
 {

@@ -105,6 +105,10 @@ int b2s_check_status(void* ws, void* cuda_stream);
  * has no bounded waits to test: its library kernels are not its own.) */
 int b2s_selftest_wait_timeout(void* ws, size_t ws_bytes, void* cuda_stream);
 
+/* The same for a choice of the kernels that sort uint32 keys: which = 0 the passes of short 1-D arrays (what
+ * b2s_selftest_wait_timeout runs), 1 those of rows too long to be sorted on chip, 2 those of long 1-D arrays. */
+int b2s_selftest_wait_timeout_in(int which, void* ws, size_t ws_bytes, void* cuda_stream);
+
 /* Same contract as b2s_local_sort, for callers that cannot hand over a workspace because they
  * cannot allocate one: for instance a task body under a runtime that forbids cudaMalloc while
  * tasks are in flight, or a thread whose memory pool is exhausted.  It has no counterpart in the

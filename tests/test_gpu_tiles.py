@@ -88,3 +88,24 @@ def test_a_captured_sort_replays_on_new_keys(cuda_device, n):
         want = torch.sort(keys, stable=True).indices
         assert torch.equal(idx, want)
     del graph
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_a_wait_that_runs_out_in_each_form_of_the_pass(cuda_device, which):
+    """The library's own self-test in the passes of short arrays (dependent launches, a look-back window of 16),
+    of long rows and of long arrays (a window of 4): the status is reported, and the workspace serves correct
+    sorts of every form afterwards."""
+    import torch
+
+    lib, stream, code = _lib.lib(), torch.cuda.current_stream().cuda_stream, _lib.DTYPE_CODE[np.dtype(np.uint32)]
+    ws = torch.empty(16 << 20, dtype=torch.uint8, device="cuda")
+    assert lib.b2s_selftest_wait_timeout_in(which, ws.data_ptr(), 2 << 20, stream) == 0
+    assert lib.b2s_check_status(ws.data_ptr(), stream) == 5          # B2S_ERR_TIMEOUT
+    keys = torch.randint(0, 1 << 31, (600_000,), device="cuda").to(torch.int32)
+    out = torch.empty_like(keys)
+    for n, seg in ((100_000, 100_000), (600_000, 20_000), (600_000, 600_000)):
+        _lib.check(lib.b2s_local_sort(code, keys.data_ptr(), out.data_ptr(), None, n, seg, 0, int(n == seg), 1, ws.data_ptr(),
+                                      ws.numel(), stream), "b2s_local_sort")
+        assert lib.b2s_check_status(ws.data_ptr(), stream) == 0
+        assert torch.equal(out[:n].reshape(-1, seg), torch.sort(keys[:n].reshape(-1, seg), dim=1).values)
