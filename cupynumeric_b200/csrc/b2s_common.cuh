@@ -104,7 +104,8 @@ __host__ __device__ __forceinline__ typename KeyOf<KB>::type pad_raw(int xf)
 }
 
 // ---------------------------------------------------------------------------------------------
-// Control block at the start of a workspace (zeroed by one memset per sort call).
+// Control block at the start of a workspace.  Radix sorts clear it by one memset; sorts on chip, which wait for
+// nothing, write its status word and leave the rest alone.
 // ---------------------------------------------------------------------------------------------
 constexpr int RADIX_BITS = 8;
 constexpr int RADIX      = 1 << RADIX_BITS;

@@ -54,7 +54,7 @@ extern "C" int b2s_local_sort_noalloc(int dtype, const void* keys_in, void* keys
   unsigned char* scratch = nullptr;
   rc = scratch_of_current_device(&scratch);
   if (rc != B2S_OK) return rc;
-  // b2s_local_sort clears the control block and the look-back table of the scratch on every call
+  // every sort starts by clearing what it reads of the scratch (on-chip sorts write the status word only)
   return b2s_local_sort(dtype, keys_in, keys_out, idx_out, volume, segment, index_offset, ndim_is_1, 1, scratch,
                         (size_t)B2S_NOALLOC_SCRATCH_BYTES, cuda_stream);
 }
