@@ -45,7 +45,8 @@ L2_BYTES = 126 << 20
 
 # name -> description.  hbm_bytes: algorithmic bytes per key on one GPU / on several (the second
 # adds the k-way merge); nvlink_bytes: bytes per key that cross NVLink per direction, before the
-# (P-1)/P factor; sweep_bytes: algorithmic bytes per key of one launch of the dominant kernel.
+# (P-1)/P factor; sweep_bytes: algorithmic bytes per key of one launch of the dominant kernel.  Only what runs is
+# counted: the keys of c4 leave five passes of eight (8 for the histogram, 5 x 16), those of c5 four (8 + 20 + 24 + 24 + 20).
 CONFIGS = {
     "c1": dict(label="1-D int32 sort, N=2^{log2} per GPU, keys uniform over the full int32 range", dtype="i32", log2=24,
                argsort=False, hbm_bytes=(36.0, 36.0), nvlink_bytes=4.0, sweep_bytes=8.0, kernel="onesweep_kernel",
@@ -57,10 +58,10 @@ CONFIGS = {
                log2=28, argsort=False, hbm_bytes=(16.0, 16.0), nvlink_bytes=0.0, sweep_bytes=16.0,
                kernel="segmerge_kernel", multi="rows"),
     "c4": dict(label="1-D int64 distributed sort, 2^{log2} keys per GPU, Zipf(1.2) clipped to [0,2^40)", dtype="i64",
-               log2=28, argsort=False, hbm_bytes=(136.0, 152.0), nvlink_bytes=8.0, sweep_bytes=16.0,
+               log2=28, argsort=False, hbm_bytes=(88.0, 104.0), nvlink_bytes=8.0, sweep_bytes=16.0,
                kernel="onesweep_kernel", multi="distributed"),
     "c5": dict(label="1-D uint64 distributed stable argsort -> int64, 2^{log2} keys per GPU, ascending with 1% pair swaps",
-               dtype="u64", log2=28, argsort=True, hbm_bytes=(248.0, 272.0), nvlink_bytes=16.0, sweep_bytes=31.0,
+               dtype="u64", log2=28, argsort=True, hbm_bytes=(96.0, 120.0), nvlink_bytes=16.0, sweep_bytes=22.0,
                kernel="onesweep_kernel", multi="distributed"),
 }
 

@@ -303,7 +303,7 @@ __device__ __forceinline__ unsigned int digit_fast(typename KeyOf<KB>::type raw,
 {
   if (XF == XF_FLOAT) {
     // one byte permutation in place of a shift and a mask (float32 argsort of 2^28 5.86 -> 5.81 ms, sort of 2^27
-    // 2.51 -> 2.48); the same on the chosen half of an 8-byte image slowed float64 by 4 %
+    // 2.51 -> 2.48), although the argsort instance spills more with it; the same on the chosen half of an 8-byte image slowed float64 by 4 %
     if (KB == 4) return __byte_perm((unsigned int)to_ordered<KB, XF>(raw), 0u, s.prmt);
     return (unsigned int)(to_ordered<KB, XF>(raw) >> shift) & (RADIX - 1);
   } else if (XF == XF_CFLOAT) {

@@ -649,10 +649,11 @@ onesweep_kernel(Ctrl* ctrl, unsigned int* __restrict__ lookback, int pass, SegGe
     rd[k] = (d << 16) | (old + __popc(peers & lt));
   }
 #else
-  // PIN keeps the compiler from computing many elements' digits ahead of their turn.  For short float keys
-  // without positions the registers saved are worth more than the overlap (float32 2^27 2.57 -> 2.51 ms,
-  // float16 1.52 -> 1.41, columns of 10^5 float32 0.694 -> 0.672); integers, 8-byte keys and pairs lose by it
-  // (int32 2^28 4.59 -> 4.64, float64 2^27 6.10 -> 6.35, uint16 argsort 1.37 -> 1.44).
+  // PIN keeps the compiler from computing many elements' digits ahead of their turn.  Short float keys without
+  // positions gain by it (float32 2^27 2.57 -> 2.51 ms, float16 1.52 -> 1.41, columns of 10^5 float32 0.694 -> 0.672),
+  // though not through fewer registers: the float32 instance of 24 keys per thread spills more with it (36 + 20
+  // bytes per thread become 252 + 232).  Integers, 8-byte keys and pairs lose by it (int32 2^28 4.59 -> 4.64, float64
+  // 2^27 6.10 -> 6.35, uint16 argsort 1.37 -> 1.44).
   constexpr bool PIN = XF == XF_FLOAT && !PAIRS && KB <= 4;
 #pragma unroll
   for (int k = 0; k < IPC; ++k) {
