@@ -440,7 +440,9 @@ inline cudaError_t segsort_pairs(int xf, const void* in, void* out, int64_t* idx
   // Short rows go to the warp kernel (2^24 float32 keys with positions, against the one-CTA-per-row radix
   // and merge kernels they took before: rows of 2 19.2 ms -> 0.07 ms, of 32 1.31 -> 0.10, of 100 0.47 -> 0.17, of
   // 200 1.42 -> 0.15, of 512 0.34 -> 0.12).  One-byte rows of 65 to 128 stay with the radix kernel, which
-  // needs a single pass for them (0.140 ms against 0.146 when this kernel still merged them).
+  // needs a single pass for them whatever they hold.  2^24 uint8 keys in rows of 100, radix against warp kernel: spread
+  // over 256 values 127 and 125 us, of three values 120 and 144, of one 45 and 74; the argsort 140 and 117, 132
+  // and 137, 60 and 68.
   // Keys of a sort are mapped back from their images, which the complex64 image does not allow: those
   // rows are sorted with positions and the keys fetched through them.  So are keys below 4 bytes, whose
   // words have room for the position anyway.
