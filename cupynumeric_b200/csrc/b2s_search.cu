@@ -14,8 +14,8 @@
 namespace b2s {
 
 constexpr int SS_SAMPLES  = 4096;
-constexpr size_t SS_MANY  = (size_t)1 << 19;  // values from which on a search goes through samples
-constexpr size_t SS_BYTES = (size_t)1 << 28;  // longest tile for which it does
+constexpr size_t SS_MANY  = (size_t)1 << 20;  // values from which on a long tile is searched without samples
+constexpr size_t SS_BYTES = (size_t)1 << 28;  // longest tile that the L2 holds well enough
 
 // SAMPLES > 0: every CTA first puts SS_SAMPLES evenly spaced keys of the tile (their images) into shared memory and
 // searches there; only the levels below go to memory.  A warp's 32 probes at different places of
@@ -90,12 +90,13 @@ static cudaError_t searchsorted_launch(const void* sorted, size_t n, int64_t glo
                                                      reinterpret_cast<long long*>(positions));
     return cudaGetLastError();
   };
-  // The samples pay where a CTA has several rounds of values for the ones it fetched, and where the probes below
-  // them find the tile in the L2: 10^5 values in 2^24 doubles take 19 us with them and 13 without, 2 * 10^5 26 and 20,
-  // 3 * 10^5 35 and 31, 2^20 95 and 110; in 2^26 doubles (512 MiB) 2^22 values take 1071 us with them and 994 without.
-  if (num_values >= SS_MANY && n <= SS_BYTES / KB) {
-    size_t grid = (num_values + 511) / 512;
-    if (grid > (size_t)sms * 4) grid = (size_t)sms * 4;  // all resident: the samples are fetched once per CTA
+  // The samples pay where a CTA has more than one round of values for the ones it fetched (10^5 values in 2^24 doubles
+  // take 19 us with them and 13 without, 2 * 10^5 26 and 20, 4 * 10^5 47 and 50, 2^20 95 and 110), and, for many
+  // values, where the probes below them find the tile in the L2: in 2^26 doubles (512 MiB) 4 * 10^5 values take 111
+  // us with them and 138 without, but 2^22 values 1071 and 994.
+  const size_t grid_all = (size_t)sms * 4;  // all resident: the samples are fetched once per CTA
+  if (num_values > grid_all * 512 && (num_values < SS_MANY || n <= SS_BYTES / KB)) {
+    const size_t grid = grid_all;
     return whole ? launch(searchsorted_kernel<KB, true, SS_SAMPLES, 512>, 512, grid)
                  : launch(searchsorted_kernel<KB, false, SS_SAMPLES, 512>, 512, grid);
   }

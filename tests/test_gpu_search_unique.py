@@ -70,9 +70,9 @@ def test_unique_reports_a_wait_that_runs_out(cuda_device):
 @pytest.mark.parametrize("dtype", [np.uint8, np.float32, np.int64])
 @pytest.mark.parametrize("n", [1, 4095, 4097, 12_289, 300_001])
 def test_searchsorted_of_many_values(cuda_device, n, dtype):
-    """From 2^19 values on the upper levels are searched in samples."""
+    """Beyond one round of values per block the upper levels are searched in samples."""
     rng = np.random.default_rng(n)
-    for m in ((1 << 19) - 1, 1 << 19, (1 << 19) + 301):
+    for m in (148 * 2048, 148 * 2048 + 1, (1 << 19) + 301):
         a = np.sort(rng.integers(0, 200, n).astype(dtype) if dtype == np.uint8 else rng.integers(0, 2 * n, n).astype(dtype))
         v = np.concatenate([a[:500], a[-500:], rng.integers(0, 250, m).astype(dtype)])[:m]
         d_a, d_v = to_device(a), to_device(v)
