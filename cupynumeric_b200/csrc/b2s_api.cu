@@ -363,7 +363,7 @@ int b2s_selftest_wait_timeout_in(int which, void* ws, size_t ws_bytes, void* cud
   ra.key_bytes   = 4;
   if (rows) {
     const unsigned int chunks = (ROW + SEG_HIST_CHUNK - 1) / SEG_HIST_CHUNK;
-    seg_hist_kernel<4, XF_UNSIGNED><<<ROWS * chunks, 256, 0, stream>>>(in, ROW, chunks, sh);
+    seg_hist_kernel<4, XF_UNSIGNED><<<ROWS * chunks, 256, 0, stream>>>(in, ROW, chunks, sh, ctrl, nullptr, 0);
     seg_scan_kernel<<<ROWS * 4, RADIX, 0, stream>>>(sh);
     scan_route_kernel<<<1, RADIX, 0, stream>>>(ctrl, ra);
   } else {

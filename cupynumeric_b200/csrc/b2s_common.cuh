@@ -132,13 +132,17 @@ struct FixDesc {
   const uint32_t* widen_src;  // with synth_idx: the caller's 32-bit payload takes the place of i
 };
 
+enum : unsigned int { ROUTE_OPEN = 0, ROUTE_SPLIT = 1, ROUTE_RADIX = 2 };
+
 struct Ctrl {
   unsigned int status;                  // 0 or a b2s_status_t, written by kernels
   unsigned int abort;                   // set with status; every later wait gives up at once
   unsigned int tile_counter[MAX_PASSES];
   unsigned int hist_done;               // CTAs of the histogram kernel that have added their counts
   unsigned int spin_limit;              // 0: SPIN_LIMIT; else the poll limit of the look-back wait (self-test)
-  unsigned int pad_[4];
+  unsigned int route;                   // who sorts: the splitting kernels (b2s_split.cuh) or the radix passes
+  unsigned int split_nleaf;             // buckets to be sorted on chip, so far
+  unsigned int split_nseg, split_ntiles;  // what the second split takes
   unsigned int hist[MAX_PASSES][RADIX]; // digit counts, then (after the scan kernel) exclusive bases
   PassDesc pass[MAX_PASSES];
   FixDesc fix;
@@ -332,6 +336,23 @@ template <int KB, int XF>
 __device__ __forceinline__ unsigned int digit_of(typename KeyOf<KB>::type raw, int shift)
 {
   return (unsigned int)(to_ordered<KB, XF>(raw) >> shift) & (RADIX - 1);
+}
+
+// Launches a kernel that calls chain_wait() before it reads anything its predecessor in the stream wrote.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kern)(P...), unsigned int grid, unsigned int block, size_t smem, cudaStream_t stream, A... args)
+{
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim          = dim3(grid);
+  cfg.blockDim         = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream           = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs    = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }

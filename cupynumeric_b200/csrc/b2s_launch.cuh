@@ -7,6 +7,7 @@
 #include "b2s_segsort.cuh"
 #include "b2s_segmerge.cuh"
 #include "b2s_segwarp.cuh"
+#include "b2s_split_plan.cuh"
 
 #include <cstdlib>
 #include <type_traits>
@@ -99,22 +100,6 @@ inline Radix1dLayout radix_1d_layout(size_t n, bool pairs)
 // wait loses more than it hides (Zipf int64 sort of 2^28 7.17 -> 7.29 ms; at 2^22 keys int64 argsort still
 // gains, 343 -> 320 us): those sorts, and segments, launch their passes the plain way.
 constexpr size_t CHAIN_MAX = (size_t)1 << 23;
-template <typename... P, typename... A>
-inline cudaError_t launch_chained(void (*kern)(P...), unsigned int grid, unsigned int block, size_t smem, cudaStream_t stream, A... args)
-{
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim          = dim3(grid);
-  cfg.blockDim         = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream           = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs    = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-
 template <int KB, int XF, bool PAIRS, int SIZE = SWEEP_MEDIUM, bool CHAINED = false>
 inline cudaError_t launch_sweeps(Ctrl* ctrl, unsigned int* lookback, unsigned int tiles, SegGeom geo,
                                  int64_t index_offset, cudaStream_t stream)
@@ -134,6 +119,46 @@ inline cudaError_t launch_sweeps(Ctrl* ctrl, unsigned int* lookback, unsigned in
   return cudaGetLastError();
 }
 
+// Testing aid and comparisons: B2S_SPLIT=0 leaves every sort to the radix passes, another number is the length from which
+// 1-D sorts are tried by the splitting kernels, whatever the keys.
+inline long long split_override()
+{
+  const char* e = std::getenv("B2S_SPLIT");
+  return e == nullptr ? -1 : std::atoll(e);
+}
+
+// Whether a 1-D sort is tried by the splitting kernels first, and which keys the sample then sends back to the radix
+// passes.  Measured on one GPU, radix passes -> splits, us per call:
+//   int32 sort, full range         9 * 10^5 (one split) 62 -> 59, 2 * 10^6 (two) 85 -> 85, 3.5 116 -> 112, 6 188 -> 142,
+//                                  2^24 368 -> 280, 8 * 10^7 1450 -> 1016
+//   float32 sort, normal           1.1 * 10^6 69 -> 61, 3.5 117 -> 119, 6 191 -> 177, 20 450 -> 371, 80 1517 -> 1163
+//   float32 argsort                7 * 10^5 97 -> 61, 2 * 10^6 99 -> 100, 6 230 -> 209, 20 583 -> 517, 80 1853 -> 1747
+//   int64 sort, full range         7 * 10^5 128 -> 73, 3.5 * 10^6 284 -> 152, 20 1065 -> 524, 80 3780 -> 1875
+//   int64 sort, 4 bytes differ     7 * 10^5 67 -> 84, 2 * 10^6 84 -> 110, 3.5 169 -> 168, 20 574 -> 527
+//   int64 argsort, full range      7 * 10^5 147 -> 71, 6 * 10^6 456 -> 257, 80 4495 -> 2435
+//   float64 sort, normal           6 * 10^4 73 -> 68, 1.5 * 10^5 81 -> 69, 7 131 -> 70, 80 * 10^6 3702 -> 2006
+//   float64 argsort                2 * 10^4 79 -> 70, 4 * 10^5 103 -> 75, 80 * 10^6 4587 -> 2536
+// Whether bytes are constant is not known before the sample; keys that are sent back have paid for it and for the
+// launches (about 13 us for one split, 25 for two).  8-byte integers, whose upper bytes often are constant, are
+// tried only where that is a small part.
+template <int KB, int XF>
+inline SplitPlan split_plan_1d(size_t n, bool pairs, bool keys_too, size_t room)
+{
+  const long long over = split_override();
+  if (!(KB == 4 || KB == 8) || XF == XF_CFLOAT || (pairs && keys_too) || over == 0) return SplitPlan{};
+  SplitPlan p = split_plan(n, 1, pairs, room);
+  size_t least;
+  if (KB == 4) least = p.levels != 1 ? 5000000 : pairs ? 600000 : 900000;
+  else if (XF == XF_FLOAT) least = pairs ? 20000 : 100000;
+  else least = pairs ? 6000000 : 3000000;
+  if (n < (over > 0 ? (size_t)over : least)) p.ok = false;
+  // (float32 argsort of 2^28 5.80 -> 5.85 ms)
+  if (KB == 4 && pairs && n > 100000000 && over < 0) p.ok = false;
+  // each byte in which the keys differ is a radix pass
+  if (over <= 0) p.radix_if = KB == 4 ? (pairs || p.levels == 1 ? 0xEu : 0xCu) : (pairs || n < 6000000 ? 0xEu : 0u);
+  return p;
+}
+
 #ifndef B2S_HIST_LANES
 #define B2S_HIST_LANES 1
 #endif
@@ -150,8 +175,30 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
   unsigned int* lb   = reinterpret_cast<unsigned int*>(ws + lay.off_lookback);
   // control block; the look-back tables too unless the histogram kernel clears them
   const bool own_hist = hist_parts == nullptr;
-  cudaError_t e       = cudaMemsetAsync(ws, 0, lay.off_lookback + (own_hist ? 0 : lay.lookback_used), stream);
+  const SplitPlan plan = own_hist ? split_plan_1d<KB, XF>(n, pairs, out != nullptr, lay.off_keys[0] - lay.off_lookback) : SplitPlan{};
+  cudaError_t e        = cudaMemsetAsync(ws, 0, lay.off_lookback + (plan.ok ? plan.zero_bytes : own_hist ? 0 : lay.lookback_used), stream);
   if (e != cudaSuccess) return e;
+  if constexpr ((KB == 4 || KB == 8) && XF != XF_CFLOAT) {
+    // the splitting kernels first; the radix passes behind them find out whether anything is left to do
+    if (plan.ok) {
+      SplitJob job{};
+      job.in           = in;
+      job.out          = out;
+      job.idx64        = idx32 ? nullptr : idx_out;
+      job.idx32        = idx32 ? reinterpret_cast<uint32_t*>(idx_out) : nullptr;
+      job.payload      = idx_in;
+      job.seg_len      = n;
+      job.nseg         = 1;
+      job.index_offset = index_offset;
+      for (int i = 0; i < 2; ++i) {
+        job.tmp_keys[i] = ws + lay.off_keys[i];
+        job.tmp_pos[i]  = reinterpret_cast<uint32_t*>(ws + lay.off_idx[i]);
+      }
+      job.tables = ws + lay.off_lookback;
+      e = launch_split<KB>(XF, plan, job, ctrl, stream);
+      if (e != cudaSuccess) return e;
+    }
+  }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -255,12 +302,41 @@ inline cudaError_t radix_seg_xf(const void* in, void* out, int64_t* idx_out, uns
   Ctrl* ctrl       = reinterpret_cast<Ctrl*>(ws);
   unsigned int* lb = reinterpret_cast<unsigned int*>(ws + lay.off_lookback);
   unsigned int* sh = reinterpret_cast<unsigned int*>(ws + lay.off_seghist);
-  cudaError_t e    = cudaMemsetAsync(ws, 0, lay.off_keys[0], stream);  // control block, look-back table, histograms
+  // control block and histograms; the look-back table is cleared by the histogram kernel, since the tables of the
+  // splitting kernels take its place until then
+  cudaError_t e = cudaMemsetAsync(ws, 0, lay.off_lookback, stream);
   if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(ws + lay.off_seghist, 0, lay.off_keys[0] - lay.off_seghist, stream);
+  if (e != cudaSuccess) return e;
+  if constexpr ((KB == 4 || KB == 8) && XF != XF_CFLOAT) {
+    if (!(pairs && out != nullptr) && split_override() != 0) {
+      const SplitPlan plan = split_plan(seg_len, nseg, pairs, lay.off_seghist - lay.off_lookback);
+      if (plan.ok) {
+        e = cudaMemsetAsync(ws + lay.off_lookback, 0, plan.zero_bytes, stream);
+        if (e != cudaSuccess) return e;
+        SplitJob job{};
+        job.in           = in;
+        job.out          = out;
+        job.idx64        = idx_out;
+        job.seg_len      = seg_len;
+        job.nseg         = nseg;
+        job.index_offset = index_offset;
+        for (int i = 0; i < 2; ++i) {
+          job.tmp_keys[i] = ws + lay.off_keys[i];
+          job.tmp_pos[i]  = reinterpret_cast<uint32_t*>(ws + lay.off_idx[i]);
+        }
+        job.tables = ws + lay.off_lookback;
+        e = launch_split<KB>(XF, plan, job, ctrl, stream);
+        if (e != cudaSuccess) return e;
+      }
+    }
+  }
   const unsigned int chunks = (seg_len + SEG_HIST_CHUNK - 1) / SEG_HIST_CHUNK;
   {
     prof::Scope ps(prof::K_HIST, stream);
-    seg_hist_kernel<KB, XF><<<nseg * chunks, 256, 0, stream>>>(static_cast<const K*>(in), seg_len, chunks, sh);
+    seg_hist_kernel<KB, XF><<<nseg * chunks, 256, 0, stream>>>(static_cast<const K*>(in), seg_len, chunks, sh, ctrl,
+                                                                  reinterpret_cast<uint4*>(ws + lay.off_lookback),
+                                                                  (lay.off_seghist - lay.off_lookback) / 16);
   }
   {
     prof::Scope ps(prof::K_SCAN, stream);

@@ -108,7 +108,11 @@ __device__ __forceinline__ void scan_route_body(Ctrl* ctrl, const RouteArgs& a)
   ctrl->fix = fix;
 }
 
-static __global__ void __launch_bounds__(RADIX) scan_route_kernel(Ctrl* ctrl, RouteArgs a) { scan_route_body(ctrl, a); }
+static __global__ void __launch_bounds__(RADIX) scan_route_kernel(Ctrl* ctrl, RouteArgs a)
+{
+  if (ctrl->route == ROUTE_SPLIT) return;  // sorted already; the passes, not routed, have nothing to do
+  scan_route_body(ctrl, a);
+}
 
 // The digit histograms arrive ready-made in `nparts` pieces ([part][npass][RADIX] counts, e.g. one
 // per rank that sent this GPU keys): add them up, then scan and route as usual.  Takes the place
@@ -168,6 +172,7 @@ hist_kernel(const typename KeyOf<KB>::type* __restrict__ keys, unsigned int n, C
 {
   using K = typename KeyOf<KB>::type;
   __shared__ unsigned int sh[KB][RADIX];
+  if (ctrl->route == ROUTE_SPLIT) return;  // sorted already; the passes, not routed, have nothing to do
   for (int i = threadIdx.x; i < KB * RADIX; i += HIST_THREADS) (&sh[0][0])[i] = 0;
   __syncthreads();
 
@@ -233,6 +238,7 @@ hist_lanes_kernel(const typename KeyOf<KB>::type* __restrict__ keys, unsigned in
   using K = typename KeyOf<KB>::type;
   constexpr int COPIES = HistLanes<KB>::COPIES;
   extern __shared__ __align__(16) unsigned int histl_smem[];
+  if (ctrl->route == ROUTE_SPLIT) return;  // sorted already; the passes, not routed, have nothing to do
   unsigned int* sh = histl_smem;  // [(pass * RADIX + digit) * COPIES + copy]
   for (int i = threadIdx.x; i < KB * RADIX * COPIES; i += HISTL_THREADS) sh[i] = 0;
   for (unsigned long long i = (unsigned long long)blockIdx.x * HISTL_THREADS + threadIdx.x; i < route.zero_vecs;
@@ -313,9 +319,12 @@ constexpr unsigned int SEG_HIST_CHUNK = 8192;
 template <int KB, int XF>
 __global__ void __launch_bounds__(256)
 seg_hist_kernel(const typename KeyOf<KB>::type* __restrict__ keys, unsigned int seg_len, unsigned int chunks_per_seg,
-                unsigned int* __restrict__ seg_hist)
+                unsigned int* __restrict__ seg_hist, const Ctrl* ctrl, uint4* zero_ptr, unsigned long long zero_vecs)
 {
   __shared__ unsigned int sh[KB][RADIX];
+  if (ctrl->route == ROUTE_SPLIT) return;  // sorted already
+  for (unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x; i < zero_vecs; i += (unsigned long long)gridDim.x * 256)
+    zero_ptr[i] = make_uint4(0u, 0u, 0u, 0u);
   for (int i = threadIdx.x; i < KB * RADIX; i += 256) (&sh[0][0])[i] = 0;
   __syncthreads();
   const unsigned int seg = blockIdx.x / chunks_per_seg, chunk = blockIdx.x - seg * chunks_per_seg;

@@ -1,0 +1,170 @@
+"""The splitting sort of long arrays and long rows (csrc/b2s_split.cuh) against NumPy's stable sort, bit for bit: one
+input per mapping of keys to cells, per edge of its tables and per way out of it."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _values(how: str, n: int, dtype: np.dtype, seed: int) -> np.ndarray:
+    rng = np.random.default_rng(seed)
+    if dtype.kind == "f":
+        if how == "normal":
+            a = rng.standard_normal(n)
+        elif how == "nans":          # three values in a hundred, and one pattern of them
+            a = rng.standard_normal(n)
+            a[rng.integers(0, n, n // 33)] = np.nan
+        elif how == "patterns":      # zeros of both signs, several NaN patterns: input order among equal images
+            a = np.round(rng.standard_normal(n) * 4) / 4
+            a = a.astype(dtype)
+            u = a.view(f"u{dtype.itemsize}")
+            at = rng.integers(0, n, n // 50)
+            u[at] = np.array(np.nan, dtype).view(u.dtype) + (at % 5).astype(u.dtype)
+            return a
+        elif how == "wide":          # every magnitude, and infinities
+            a = np.exp2(rng.uniform(-140 if dtype.itemsize == 4 else -1000, 120, n)) * rng.choice([-1.0, 1.0], n)
+            a[rng.integers(0, n, 9)] = np.inf
+            a[rng.integers(0, n, 9)] = -np.inf
+        elif how == "spike":         # half of the keys are one value, the others around it
+            a = np.where(rng.random(n) < 0.5, 0.75, rng.standard_normal(n))
+        elif how == "few":           # values far apart, each with many copies
+            a = rng.integers(0, 37, n) * 1.37e5
+        elif how == "crowded":       # two clusters that a linear function does not take apart
+            a = np.where(rng.random(n) < 0.5, 1.0, 1e30) * (1 + rng.random(n) * 1e-4)
+        elif how == "equal":
+            a = np.full(n, 2.5)
+        else:
+            a = np.full(n, np.nan)
+        return a.astype(dtype)
+    info = np.iinfo(dtype)
+    if how == "normal":
+        return rng.integers(info.min, info.max, n, dtype=dtype, endpoint=True)
+    if how == "nans":                # the ends of the range
+        a = rng.integers(info.min, info.max, n, dtype=dtype, endpoint=True)
+        a[rng.integers(0, n, n // 30)] = info.max
+        a[rng.integers(0, n, n // 30)] = info.min
+        return a
+    if how == "patterns":            # Zipf: crowded at the lower end, the largest value often
+        return np.minimum(rng.zipf(1.2, n).astype(np.float64), min(info.max, 2**40 - 1)).astype(dtype)
+    if how == "wide":
+        return np.exp2(rng.uniform(0, 8 * dtype.itemsize - 2, n)).astype(dtype)
+    if how == "spike":
+        return np.where(rng.random(n) < 0.5, 12345, rng.integers(0, 2**31 - 1, n)).astype(dtype)
+    if how == "few":
+        return (rng.integers(0, 100, n) * (1 if seed % 2 else info.max // 128)).astype(dtype)
+    if how == "crowded":             # almost in order
+        a = np.arange(n).astype(dtype)
+        i, j = rng.integers(0, n, n // 100), rng.integers(0, n, n // 100)
+        a[i], a[j] = a[j], a[i]
+        return a
+    return np.full(n, 7 if how == "equal" else info.max, dtype)
+
+
+def _check(a: np.ndarray, op: str) -> None:
+    import cupynumeric_b200 as num
+
+    d = torch.from_numpy(a.view(f"i{a.dtype.itemsize}") if a.dtype.kind == "u" else a).cuda()
+    d = d.view({"u4": torch.uint32, "u8": torch.uint64}[a.dtype.str[1:]]) if a.dtype.kind == "u" else d
+    order = np.argsort(a, axis=-1, kind="stable")
+    if op == "argsort":
+        got = num.argsort(num.array(d), axis=-1, kind="stable").to_numpy()
+        assert np.array_equal(got, order)
+    else:
+        got  = num.sort(num.array(d), axis=-1).to_numpy()
+        want = np.take_along_axis(a, order, axis=-1)
+        assert np.array_equal(got.view(f"u{a.dtype.itemsize}"), want.view(f"u{a.dtype.itemsize}"))
+
+
+HOW = ["normal", "nans", "patterns", "wide", "spike", "few", "crowded", "equal", "last"]
+
+
+@pytest.fixture
+def split_all(monkeypatch):
+    """1-D sorts of every length and of all keys are tried by the splitting kernels."""
+    monkeypatch.setenv("B2S_SPLIT", "8193")
+
+
+@pytest.mark.parametrize("how", HOW)
+@pytest.mark.parametrize("op", ["sort", "argsort"])
+@pytest.mark.parametrize("dtype", ["int32", "uint32", "float32", "int64", "uint64", "float64"])
+def test_two_splits(split_all, dtype, op, how):
+    # (more keys than one split takes apart)
+    _check(_values(how, 2_100_019, np.dtype(dtype), 11), op)
+
+
+@pytest.mark.parametrize("how", HOW)
+@pytest.mark.parametrize("op", ["sort", "argsort"])
+@pytest.mark.parametrize("dtype", ["int32", "float32", "uint64", "float64"])
+def test_one_split(split_all, dtype, op, how):
+    _check(_values(how, 300_007, np.dtype(dtype), 13), op)
+
+
+@pytest.mark.parametrize("how", HOW)
+@pytest.mark.parametrize("op", ["sort", "argsort"])
+@pytest.mark.parametrize("dtype", ["int32", "float32", "uint64", "float64"])
+def test_long_rows(dtype, op, how):
+    n, rows = 20_011, 37
+    _check(_values(how, n * rows, np.dtype(dtype), 12).reshape(rows, n), op)
+
+
+# around the lengths where the buckets' size, the number of splits and the tables change: 200 buckets of 2048, 4096, 6144
+# (with positions) and 8192 keys
+@pytest.mark.parametrize("n", [8193, 8704, 16384, 30011, 409_600, 409_601, 819_201, 1_100_003, 1_228_801, 1_638_401])
+@pytest.mark.parametrize("dtype", ["int32", "float32", "int64", "float64"])
+def test_lengths(split_all, dtype, n):
+    for op in ("sort", "argsort"):
+        _check(_values("nans", n, np.dtype(dtype), n), op)
+    if n < 100_000:
+        _check(_values("nans", n * 3, np.dtype(dtype), n).reshape(3, n), "argsort")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "int64"])
+def test_as_it_is_dispatched(dtype):
+    # (above every border of the dispatch)
+    for how in ("normal", "patterns"):
+        a = _values(how, 6_000_011, np.dtype(dtype), 3)
+        for op in ("sort", "argsort"):
+            _check(a, op)
+
+
+def test_in_place_and_other_streams(split_all):
+    """The input stays whole until the last kernel writes; two sorts on two streams do not meet."""
+    import cupynumeric_b200 as num
+
+    a, b = (_values("normal", 2_500_001, np.dtype("int64"), k) for k in (5, 6))
+    x = num.array(torch.from_numpy(a).cuda())
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        y = num.sort(num.array(torch.from_numpy(b).cuda()))
+    x.sort()
+    torch.cuda.synchronize()
+    assert np.array_equal(x.to_numpy(), np.sort(a))
+    assert np.array_equal(y.to_numpy(), np.sort(b))
+
+
+def test_under_capture(split_all):
+    """The launches and their chaining can be captured and replayed on other keys."""
+    import ctypes
+
+    from cupynumeric_b200 import _lib
+
+    n, lib, need = 700_001, _lib.lib(), ctypes.c_size_t()
+    code = _lib.DTYPE_CODE[np.dtype("float64")]
+    _lib.check(lib.b2s_workspace_bytes(code, n, n, 1, ctypes.byref(need)), "ws")
+    keys = torch.empty(n, dtype=torch.float64, device="cuda")
+    idx = torch.empty(n, dtype=torch.int64, device="cuda")
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        _lib.check(lib.b2s_local_sort(code, keys.data_ptr(), None, idx.data_ptr(), n, n, 0, 1, 1, ws.data_ptr(), need.value,
+                                      torch.cuda.current_stream().cuda_stream), "sort")
+    for how in ("normal", "few", "wide"):
+        a = _values(how, n, np.dtype("float64"), 8)
+        keys.copy_(torch.from_numpy(a))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(idx.cpu().numpy(), np.argsort(a, kind="stable")), how
