@@ -4,6 +4,11 @@
 // through the radix passes of every key as the payload, so a key costs one gather and one sort;
 // nothing leaves the library between the keys (the reference chains argsort tasks and index
 // gathers from Python, cupynumeric/_module/ssc_sorting.py:423-444).
+//
+// Neighbouring keys of at most eight bytes together are one key to the radix passes: the gather puts their
+// order-preserving images side by side.  The passes are those of the bytes that differ, as before; a gather, a histogram and
+// the passes that find nothing to do are saved for every key that joins another (4000037 rows of float64, int32, int16:
+// the two integers 220 -> 150 us).
 #include <cuda_runtime.h>
 
 #include "../../include/b200sort.h"
@@ -46,6 +51,53 @@ __global__ void lex_compose_kernel(const int64_t* __restrict__ order_in, const i
     order_out[i] = order_in[(i / segment) * segment + (size_t)pick[i]];
 }
 
+// Several keys as one 8-byte key: images side by side, the major key uppermost.
+struct LexPart {
+  const void* keys;
+  int bytes, xf, shift;
+};
+struct LexParts {
+  LexPart part[8];
+  int n;
+};
+
+__device__ __forceinline__ unsigned long long lex_image(const LexPart& p, size_t i)
+{
+  if (p.bytes == 4) return to_ordered_rt<4>(__ldg(static_cast<const unsigned int*>(p.keys) + i), p.xf);
+  if (p.bytes == 2) return to_ordered_rt<2>(__ldg(static_cast<const unsigned short*>(p.keys) + i), p.xf);
+  return to_ordered_rt<1>(__ldg(static_cast<const unsigned char*>(p.keys) + i), p.xf);
+}
+
+// out[i] = the parts' images of row order[i] (null: i)
+__global__ void lex_join_kernel(LexParts parts, const uint32_t* __restrict__ order, size_t volume, unsigned long long* __restrict__ out)
+{
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < volume; i += stride) {
+    const size_t row     = order != nullptr ? order[i] : i;
+    unsigned long long k = 0;
+    for (int p = 0; p < parts.n; ++p) k |= lex_image(parts.part[p], row) << parts.part[p].shift;
+    out[i] = k;
+  }
+}
+
+// Keys k .. k + lex_group() - 1 are sorted as one.
+static int lex_group(int nkeys, const int* dtypes, int k)
+{
+  size_t bytes = 0;
+  int m        = 0;
+  while (k + m < nkeys && m < 8 && bytes + lex_elem_bytes(dtypes[k + m]) <= 8) bytes += lex_elem_bytes(dtypes[k + m++]);
+  return m > 1 ? m : 1;
+}
+
+static int lex_xf(int dtype)
+{
+  switch (dtype) {
+    case B2S_INT8: case B2S_INT16: case B2S_INT32: return XF_SIGNED;
+    case B2S_FLOAT16: case B2S_FLOAT32: return XF_FLOAT;
+    default: return XF_UNSIGNED;
+  }
+}
+
 template <typename I>
 static cudaError_t lex_gather(size_t eb, const void* in, const I* order, size_t volume, size_t segment, void* out,
                               cudaStream_t stream)
@@ -68,9 +120,18 @@ struct LexLayout {
   size_t off_gather, off_ord[2], off_pick, off_sort, sort_bytes, total;
 };
 
-static int lex_layout(int nkeys, const int* dtypes, size_t volume, size_t segment, LexLayout* l)
+// `joined`: with room for joined keys.
+static int lex_layout(int nkeys, const int* dtypes, size_t volume, size_t segment, LexLayout* l, bool joined)
 {
   size_t max_eb = 0, max_ws = 0;
+  if (joined) {
+    for (int k = 0; k < nkeys; k += lex_group(nkeys, dtypes, k)) {
+      if (lex_group(nkeys, dtypes, k) < 2) continue;
+      const int rc = b2s_workspace_bytes(B2S_UINT64, volume, segment, 1, &max_ws);
+      if (rc != B2S_OK) return rc;
+      max_eb = 8;
+    }
+  }
   for (int k = 0; k < nkeys; ++k) {
     const size_t eb = lex_elem_bytes(dtypes[k]);
     if (eb == 0) return B2S_ERR_UNSUPPORTED;
@@ -91,6 +152,17 @@ static int lex_layout(int nkeys, const int* dtypes, size_t volume, size_t segmen
   return B2S_OK;
 }
 
+// Whether neighbouring keys may be sorted as one: 1-D tiles whose order is carried through the passes.
+static bool lex_joins(const int* dtypes, int nkeys, size_t volume, size_t segment)
+{
+  bool some = false;
+  for (int k = 0; k < nkeys; ++k) {
+    if (dtypes[k] == B2S_COMPLEX128) return false;
+    some = some || lex_group(nkeys, dtypes, k) > 1;
+  }
+  return some && volume == segment && local_sort_pos32_supported(volume);
+}
+
 }  // namespace b2s
 
 using namespace b2s;
@@ -102,7 +174,7 @@ int b2s_lexsort_workspace_bytes(int nkeys, const int* dtypes, size_t volume, siz
   if (nkeys < 1 || dtypes == nullptr || bytes == nullptr) return B2S_ERR_INVALID_ARG;
   if (volume > 0 && (segment == 0 || volume % segment != 0)) return B2S_ERR_INVALID_ARG;
   LexLayout l{};
-  const int rc = lex_layout(nkeys, dtypes, volume, segment ? segment : 1, &l);
+  const int rc = lex_layout(nkeys, dtypes, volume, segment ? segment : 1, &l, lex_joins(dtypes, nkeys, volume, segment));
   if (rc == B2S_OK) *bytes = l.total;
   return rc;
 }
@@ -116,8 +188,15 @@ int b2s_lexsort(int nkeys, const int* dtypes, const void* const* keys, int64_t* 
   for (int k = 0; k < nkeys; ++k)
     if (keys[k] == nullptr) return B2S_ERR_INVALID_ARG;
   LexLayout l{};
-  int rc = lex_layout(nkeys, dtypes, volume, segment, &l);
+  bool joined = lex_joins(dtypes, nkeys, volume, segment);
+  int rc      = lex_layout(nkeys, dtypes, volume, segment, &l, joined);
   if (rc != B2S_OK) return rc;
+  if (joined && ws_bytes < l.total) {
+    // a workspace without that room: key by key
+    joined = false;
+    rc     = lex_layout(nkeys, dtypes, volume, segment, &l, joined);
+    if (rc != B2S_OK) return rc;
+  }
   if (ws == nullptr || ws_bytes < l.total || (reinterpret_cast<uintptr_t>(ws) & 255u) != 0) return B2S_ERR_WORKSPACE;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   unsigned char* base = static_cast<unsigned char*>(ws);
@@ -134,18 +213,34 @@ int b2s_lexsort(int nkeys, const int* dtypes, const void* const* keys, int64_t* 
   if (carry) {
     uint32_t* pos[2] = {reinterpret_cast<uint32_t*>(ord[0]), reinterpret_cast<uint32_t*>(ord[1])};
     int cur = 0;
-    for (int k = 0; k < nkeys; ++k) {
-      const bool last = k == nkeys - 1;
+    for (int k = 0, step = 1; k < nkeys; k += step) {
+      step = joined ? lex_group(nkeys, dtypes, k) : 1;
+      const bool last = k + step == nkeys;
+      const int dtype = step > 1 ? (int)B2S_UINT64 : dtypes[k];
       const void* src = keys[k];
-      if (k > 0) {
+      if (step > 1) {
+        LexParts parts{};
+        int shift = 0;
+        for (int i = 0; i < step; ++i) {
+          parts.part[i] = LexPart{keys[k + i], (int)lex_elem_bytes(dtypes[k + i]), lex_xf(dtypes[k + i]), shift};
+          shift += 8 * parts.part[i].bytes;
+        }
+        parts.n           = step;
+        unsigned int grid = (unsigned int)((volume + 1023) / 1024);
+        if (grid > 148 * 16) grid = 148 * 16;
+        prof::Scope ps(prof::K_FIXUP, stream);
+        lex_join_kernel<<<grid, 256, 0, stream>>>(parts, k > 0 ? pos[cur] : nullptr, volume, static_cast<unsigned long long*>(gathered));
+        if (cudaGetLastError() != cudaSuccess) return B2S_ERR_CUDA;
+        src = gathered;
+      } else if (k > 0) {
         if (lex_gather<uint32_t>(lex_elem_bytes(dtypes[k]), keys[k], pos[cur], volume, segment, gathered, stream) != cudaSuccess)
           return B2S_ERR_CUDA;
         src = gathered;
       }
       if (last) {
-        rc = local_sort_payload32(dtypes[k], src, k == 0 ? nullptr : pos[cur], idx_out, volume, 0, sort_ws, l.sort_bytes, stream);
+        rc = local_sort_payload32(dtype, src, k == 0 ? nullptr : pos[cur], idx_out, volume, 0, sort_ws, l.sort_bytes, stream);
       } else {
-        rc = local_sort_payload32(dtypes[k], src, k == 0 ? nullptr : pos[cur], reinterpret_cast<int64_t*>(pos[cur ^ 1]), volume, 0,
+        rc = local_sort_payload32(dtype, src, k == 0 ? nullptr : pos[cur], reinterpret_cast<int64_t*>(pos[cur ^ 1]), volume, 0,
                                   sort_ws, l.sort_bytes, stream, 1);
         cur ^= 1;
       }
