@@ -46,10 +46,12 @@ L2_BYTES = 126 << 20
 # name -> description.  hbm_bytes: algorithmic bytes per key on one GPU / on several (the second
 # adds the k-way merge); nvlink_bytes: bytes per key that cross NVLink per direction, before the
 # (P-1)/P factor; sweep_bytes: algorithmic bytes per key of one launch of the dominant kernel.  Only what runs is
-# counted: the keys of c4 leave five passes of eight (8 for the histogram, 5 x 16), those of c5 four (8 + 20 + 24 + 24 + 20).
+# counted.  c2 runs a histogram and four radix passes; the others with a split_move_kernel two splits, each counted and moved, and the
+# leaves: c1 4 + 8 + 4 + 8 + 8; c4, of whose keys 0.39 are moved and the others filled in, 8 + 11.1 + 3.1 + 6.2 + 11.1;
+# c5 8 + 20 + 8 + 24 + 20.
 CONFIGS = {
     "c1": dict(label="1-D int32 sort, N=2^{log2} per GPU, keys uniform over the full int32 range", dtype="i32", log2=24,
-               argsort=False, hbm_bytes=(36.0, 36.0), nvlink_bytes=4.0, sweep_bytes=8.0, kernel="onesweep_kernel",
+               argsort=False, hbm_bytes=(32.0, 32.0), nvlink_bytes=4.0, sweep_bytes=8.0, kernel="split_move_kernel",
                multi="distributed"),
     "c2": dict(label="1-D float32 stable argsort -> int64, N=2^{log2} per GPU, N(0,1) + 0.1% NaN + 1% duplicates",
                dtype="f32", log2=28, argsort=True, hbm_bytes=(88.0, 108.0), nvlink_bytes=12.0, sweep_bytes=21.0,
@@ -58,11 +60,11 @@ CONFIGS = {
                log2=28, argsort=False, hbm_bytes=(16.0, 16.0), nvlink_bytes=0.0, sweep_bytes=16.0,
                kernel="segmerge_kernel", multi="rows"),
     "c4": dict(label="1-D int64 distributed sort, 2^{log2} keys per GPU, Zipf(1.2) clipped to [0,2^40)", dtype="i64",
-               log2=28, argsort=False, hbm_bytes=(88.0, 104.0), nvlink_bytes=8.0, sweep_bytes=16.0,
-               kernel="onesweep_kernel", multi="distributed"),
+               log2=28, argsort=False, hbm_bytes=(39.5, 55.5), nvlink_bytes=8.0, sweep_bytes=8.65,
+               kernel="split_move_kernel", multi="distributed"),
     "c5": dict(label="1-D uint64 distributed stable argsort -> int64, 2^{log2} keys per GPU, ascending with 1% pair swaps",
-               dtype="u64", log2=28, argsort=True, hbm_bytes=(96.0, 120.0), nvlink_bytes=16.0, sweep_bytes=22.0,
-               kernel="onesweep_kernel", multi="distributed"),
+               dtype="u64", log2=28, argsort=True, hbm_bytes=(80.0, 104.0), nvlink_bytes=16.0, sweep_bytes=22.0,
+               kernel="split_move_kernel", multi="distributed"),
 }
 
 
@@ -553,7 +555,7 @@ class Bench:
         })
         if multi:
             rec["exchange"] = os.environ.get("B2S_DIST_P2P", "1") != "0" and "peer" or "nccl"
-        dom = {"onesweep_kernel": "sweep", "segmerge_kernel": "segsort"}[c["kernel"]]
+        dom = {"onesweep_kernel": "sweep", "split_move_kernel": "sweep", "segmerge_kernel": "segsort"}[c["kernel"]]
         if dom in kernels:
             avg_ms = kernels[dom]["avg_working_launch_ms"]
             achieved = c["sweep_bytes"] * n_local / (avg_ms * 1e-3) / 1e9
@@ -561,7 +563,7 @@ class Bench:
             rec["dominant_kernel"] = {"bound": "hbm", "kernel": c["kernel"], "achieved": achieved, "peak": self.peak,
                                       "unit": "GB/s", "frac": achieved / self.peak, "peak_source": f"of {self.peak_kind}",
                                       "avg_launch_ms": avg_ms, "launches_per_step": kernels[dom]["working_launches_per_step"],
-                                      "launches": "passes that moved data (a pass the routing skipped returns at once and is left out)",
+                                      "launches": "passes or splits that moved data (a pass the routing skipped returns at once and is left out)",
                                       "algorithmic_bytes_per_launch": c["sweep_bytes"] * n_local,
                                       "traffic": traffic * n_local if traffic else None}
         if nranks == 1 and not args.no_cub:
