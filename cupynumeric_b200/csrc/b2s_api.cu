@@ -150,8 +150,8 @@ bool local_sort_pos32_supported(size_t n) { return n > SEG_CAP && n < single_sor
 
 // Stable 1-D argsort of keys that carry a 32-bit payload each (pay_in[i] belongs to keys_in[i];
 // null: the payload of element i is i).  out32 == 0: idx_out[k] = index_offset + payload of the
-// k-th smallest key, as int64; out32 != 0: idx_out points to n uint32 values that receive the bare
-// payloads.  The distributed sort uses it on what a rank received (payload = global position minus a
+// k-th smallest key, as int64; out32 (IDX_32): idx_out points to n uint32 values that receive the bare
+// payloads; IDX_PASSES_ONLY beside it: by the radix passes alone.  The distributed sort uses it on what a rank received (payload = global position minus a
 // common base), the lexicographic sort to carry its order from key to key: travelling as 32 bits the
 // payload costs the radix passes no more than a plain argsort.
 int local_sort_payload32(int dtype, const void* keys_in, const uint32_t* pay_in, int64_t* idx_out, size_t n,
@@ -165,7 +165,7 @@ int local_sort_payload32(int dtype, const void* keys_in, const uint32_t* pay_in,
   if (rc != B2S_OK) return rc;
   if (ws == nullptr || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u) != 0) return B2S_ERR_WORKSPACE;
   const cudaError_t e = radix_any(di.kb, di.xf, keys_in, nullptr, idx_out, (unsigned int)n, index_offset,
-                                  static_cast<unsigned char*>(ws), stream, out32 ? 1 : 0, pay_in);
+                                  static_cast<unsigned char*>(ws), stream, out32, pay_in);
   return e == cudaSuccess ? B2S_OK : B2S_ERR_CUDA;
 }
 

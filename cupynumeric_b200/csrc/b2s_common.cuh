@@ -132,6 +132,7 @@ struct FixDesc {
   const uint32_t* widen_src;  // with synth_idx: the caller's 32-bit payload takes the place of i
 };
 
+enum : int { IDX_32 = 1, IDX_PASSES_ONLY = 2 };  // how an argsort is asked for (launch_radix_1d)
 enum : unsigned int { ROUTE_OPEN = 0, ROUTE_SPLIT = 1, ROUTE_RADIX = 2 };
 
 struct Ctrl {

@@ -129,33 +129,34 @@ inline long long split_override()
 
 // Whether a 1-D sort is tried by the splitting kernels first, and which keys the sample then sends back to the radix
 // passes.  Measured on one GPU, radix passes -> splits, us per call:
-//   int32 sort, full range         9 * 10^5 (one split) 62 -> 59, 2 * 10^6 (two) 85 -> 85, 3.5 116 -> 112, 6 188 -> 142,
-//                                  2^24 368 -> 280, 8 * 10^7 1450 -> 1016
-//   float32 sort, normal           1.1 * 10^6 69 -> 61, 3.5 117 -> 119, 6 191 -> 177, 20 450 -> 371, 80 1517 -> 1163
+//   int32 sort, full range         10^7 253 -> 195, 2^24 371 -> 272, 8 * 10^7 1450 -> 1016
+//   float32 sort, normal           1.1 * 10^6 (one split) 69 -> 61, 3.5 (two) 117 -> 119, 6 191 -> 177, 20 450 -> 371, 80 1517 -> 1163
 //   float32 argsort                7 * 10^5 97 -> 61, 2 * 10^6 99 -> 100, 6 230 -> 209, 20 583 -> 517, 80 1853 -> 1747
-//   int64 sort, full range         7 * 10^5 128 -> 73, 3.5 * 10^6 284 -> 152, 20 1065 -> 524, 80 3780 -> 1875
-//   int64 sort, 4 bytes differ     7 * 10^5 67 -> 84, 2 * 10^6 84 -> 110, 3.5 169 -> 168, 20 574 -> 527
-//   int64 argsort, full range      7 * 10^5 147 -> 71, 6 * 10^6 456 -> 257, 80 4495 -> 2435
-//   float64 sort, normal           6 * 10^4 73 -> 68, 1.5 * 10^5 81 -> 69, 7 131 -> 70, 80 * 10^6 3702 -> 2006
-//   float64 argsort                2 * 10^4 79 -> 70, 4 * 10^5 103 -> 75, 80 * 10^6 4587 -> 2536
+//   int32 argsort, full range      2 * 10^7 579 -> 459, 4 1002 -> 843, 8 1819 -> 1583
+//   int64 sort, full range         10^7 601 -> 309, 2 * 10^7 1065 -> 524, 8 3780 -> 1875
+//   int64 argsort, full range      2 * 10^7 1273 -> 676, 8 4495 -> 2435
+//   float64 sort, normal           2 * 10^5 84 -> 69, 7 131 -> 70, 80 * 10^6 3702 -> 2006
+//   float64 argsort                2 * 10^5 87 -> 70, 4 103 -> 75, 80 * 10^6 4587 -> 2536
+//   uint64 argsort, almost in order  8 * 10^6 248 -> 271, 30 940 -> 769, 2^28 8094 -> 6225
+//   int64 sort, Zipf               8 * 10^6 319 -> 445 (given up late), 30 921 -> 468, 2^28 7174 -> 3120
 // Whether bytes are constant is not known before the sample; keys that are sent back have paid for it and for the
-// launches (about 13 us for one split, 25 for two).  8-byte integers, whose upper bytes often are constant, are
-// tried only where that is a small part.
+// launches (about 15 us for one split, 25 for two; int32 argsort of a hundred values, 6 * 10^6 keys 74 -> 100, 50 346 -> 373).
+// Integers, whose upper bytes often are constant, are tried only where that is a small part.
 template <int KB, int XF>
 inline SplitPlan split_plan_1d(size_t n, bool pairs, bool keys_too, size_t room)
 {
   const long long over = split_override();
   if (!(KB == 4 || KB == 8) || XF == XF_CFLOAT || (pairs && keys_too) || over == 0) return SplitPlan{};
-  SplitPlan p = split_plan(n, 1, pairs, room);
+  SplitPlan p          = split_plan(n, 1, pairs, room);
+  constexpr bool FLOAT = XF == XF_FLOAT;
   size_t least;
-  if (KB == 4) least = p.levels != 1 ? 5000000 : pairs ? 600000 : 900000;
-  else if (XF == XF_FLOAT) least = pairs ? 20000 : 100000;
-  else least = pairs ? 6000000 : 3000000;
+  if (KB == 4) least = !FLOAT ? (pairs ? 40000000 : 16000000) : p.levels != 1 ? 5000000 : pairs ? 600000 : 900000;
+  else least = FLOAT ? 200000 : pairs ? 12000000 : 8000000;
   if (n < (over > 0 ? (size_t)over : least)) p.ok = false;
   // (float32 argsort of 2^28 5.80 -> 5.85 ms)
   if (KB == 4 && pairs && n > 100000000 && over < 0) p.ok = false;
   // each byte in which the keys differ is a radix pass
-  if (over <= 0) p.radix_if = KB == 4 ? (pairs || p.levels == 1 ? 0xEu : 0xCu) : (pairs || n < 6000000 ? 0xEu : 0u);
+  if (over <= 0) p.radix_if = KB == 4 ? (pairs || p.levels == 1 ? 0xEu : 0xCu) : FLOAT || pairs ? 0xEu : n < 24000000 ? 0x3Eu : 0u;
   return p;
 }
 
@@ -175,7 +176,7 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
   unsigned int* lb   = reinterpret_cast<unsigned int*>(ws + lay.off_lookback);
   // control block; the look-back tables too unless the histogram kernel clears them
   const bool own_hist = hist_parts == nullptr;
-  const SplitPlan plan = own_hist ? split_plan_1d<KB, XF>(n, pairs, out != nullptr, lay.off_keys[0] - lay.off_lookback) : SplitPlan{};
+  const SplitPlan plan = own_hist && !(idx32 & IDX_PASSES_ONLY) ? split_plan_1d<KB, XF>(n, pairs, out != nullptr, lay.off_keys[0] - lay.off_lookback) : SplitPlan{};
   cudaError_t e        = cudaMemsetAsync(ws, 0, lay.off_lookback + (plan.ok ? plan.zero_bytes : own_hist ? 0 : lay.lookback_used), stream);
   if (e != cudaSuccess) return e;
   if constexpr ((KB == 4 || KB == 8) && XF != XF_CFLOAT) {
@@ -184,8 +185,8 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
       SplitJob job{};
       job.in           = in;
       job.out          = out;
-      job.idx64        = idx32 ? nullptr : idx_out;
-      job.idx32        = idx32 ? reinterpret_cast<uint32_t*>(idx_out) : nullptr;
+      job.idx64        = (idx32 & IDX_32) ? nullptr : idx_out;
+      job.idx32        = (idx32 & IDX_32) ? reinterpret_cast<uint32_t*>(idx_out) : nullptr;
       job.payload      = idx_in;
       job.seg_len      = n;
       job.nseg         = 1;
@@ -208,8 +209,8 @@ inline cudaError_t radix_1d_xf(const void* in, void* out, int64_t* idx_out, unsi
   RouteArgs ra{};
   ra.keys_in     = in;
   ra.keys_out    = out;
-  ra.idx_out     = idx32 ? nullptr : idx_out;
-  ra.idx_out32   = idx32 ? reinterpret_cast<uint32_t*>(idx_out) : nullptr;
+  ra.idx_out     = (idx32 & IDX_32) ? nullptr : idx_out;
+  ra.idx_out32   = (idx32 & IDX_32) ? reinterpret_cast<uint32_t*>(idx_out) : nullptr;
   ra.idx_in      = idx_in;
   ra.tmp_keys[0] = ws + lay.off_keys[0];
   ra.tmp_keys[1] = ws + lay.off_keys[1];
@@ -309,7 +310,9 @@ inline cudaError_t radix_seg_xf(const void* in, void* out, int64_t* idx_out, uns
   e = cudaMemsetAsync(ws + lay.off_seghist, 0, lay.off_keys[0] - lay.off_seghist, stream);
   if (e != cudaSuccess) return e;
   if constexpr ((KB == 4 || KB == 8) && XF != XF_CFLOAT) {
-    if (!(pairs && out != nullptr) && split_override() != 0) {
+    // (float32 sort of 7 rows of 90000 66 -> 73 us, of 10 rows of 10^6 271 -> 177)
+    const bool enough = KB == 8 || pairs || (size_t)seg_len * nseg >= 1000000 || split_override() > 0;
+    if (!(pairs && out != nullptr) && split_override() != 0 && enough) {
       const SplitPlan plan = split_plan(seg_len, nseg, pairs, lay.off_seghist - lay.off_lookback);
       if (plan.ok) {
         e = cudaMemsetAsync(ws + lay.off_lookback, 0, plan.zero_bytes, stream);
@@ -382,7 +385,8 @@ cudaError_t launch_radix_seg(int xf, const void* in, void* out, int64_t* idx_out
                              unsigned int nseg, int64_t index_offset, unsigned char* ws, cudaStream_t stream);
 
 // 1-D stable sort of n < 2^30 keys. `ws` must hold radix_1d_layout<KB>(n, idx_out != null).total bytes.
-// idx32 != 0: idx_out points to n uint32 values and receives positions 0..n-1 without the offset.
+// idx32: IDX_32: idx_out points to n uint32 values and receives positions 0..n-1 without the offset; IDX_PASSES_ONLY: by the
+// radix passes alone.
 // idx_in != null: the payload of element i is idx_in[i] instead of i (stable argsort of data that
 // already carries 32-bit payloads); the output index is index_offset + payload.
 // hist_parts != null: hist_nparts ready-made digit histograms ([part][KB][256]) to add up instead

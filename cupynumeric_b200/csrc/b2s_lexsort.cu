@@ -217,6 +217,9 @@ int b2s_lexsort(int nkeys, const int* dtypes, const void* const* keys, int64_t* 
       step = joined ? lex_group(nkeys, dtypes, k) : 1;
       const bool last = k + step == nkeys;
       const int dtype = step > 1 ? (int)B2S_UINT64 : dtypes[k];
+      // joined keys lie in clusters and later keys have few values: the splits give up on them, late (two int32 keys of 100000 and 200
+      // values by 1.6 * 10^7 rows 631 us by the passes, 851 after the splits)
+      const int how = step > 1 || k > 0 ? IDX_PASSES_ONLY : 0;
       const void* src = keys[k];
       if (step > 1) {
         LexParts parts{};
@@ -238,10 +241,10 @@ int b2s_lexsort(int nkeys, const int* dtypes, const void* const* keys, int64_t* 
         src = gathered;
       }
       if (last) {
-        rc = local_sort_payload32(dtype, src, k == 0 ? nullptr : pos[cur], idx_out, volume, 0, sort_ws, l.sort_bytes, stream);
+        rc = local_sort_payload32(dtype, src, k == 0 ? nullptr : pos[cur], idx_out, volume, 0, sort_ws, l.sort_bytes, stream, how);
       } else {
         rc = local_sort_payload32(dtype, src, k == 0 ? nullptr : pos[cur], reinterpret_cast<int64_t*>(pos[cur ^ 1]), volume, 0,
-                                  sort_ws, l.sort_bytes, stream, 1);
+                                  sort_ws, l.sort_bytes, stream, how | IDX_32);
         cur ^= 1;
       }
       if (rc != B2S_OK) return rc;

@@ -3,9 +3,12 @@
 //
 // Why: a stable 8-bit radix pass costs 105 to 115 thread instructions per key, most of them for ranking
 // equal digits in input order, and 4-byte keys need four of them.  A split needs no order inside a bucket: one
-// shared-memory atomic takes the place of the ranking (about 40 instructions per key), two splits of a few hundred
+// shared-memory atomic takes the place of the ranking (53 instructions per int32 key), two splits of a few hundred
 // buckets each leave rows of a few thousand keys, and the last step orders those by (key, position), so that
 // an argsort is stable although the splits are not.  Equal keys of a sort have nothing to be told apart by.
+// 2^24 int32 keys: four passes of 84 us and a histogram of 26 against two splits of 51 and 57, counts of 21 and 18 and leaves
+// of 68; 2^28 int64 Zipf keys 7174 -> 3120 us.  Pairs of 4-byte keys, with four passes to save, gain least (float32 argsort of
+// 2 * 10^7 keys 583 -> 517 us).
 //
 // Steps, all on the stream, with no word back to the host:
 //   sample    per segment (the array, a row, or a bucket of the first split): bounds of 4096 keys, from
@@ -50,7 +53,7 @@ struct SplitLevel {
   SplitSeg* segs;
   unsigned int* hist;         // [segment][cells]
   unsigned short* lut;        // [segment][cells]: bucket
-  unsigned int* cursor;       // [segment][nb]: next free place of the bucket
+  unsigned int* cursor;       // [segment][SPLIT_BINS]: next free place of the bucket
   const unsigned short* tile_seg;  // tile -> segment; null: tiles_per_seg each
   unsigned int nseg, tiles_per_seg, seg_len;  // (of equal segments)
   unsigned int cells, cap;
@@ -146,6 +149,9 @@ __device__ __forceinline__ TileRange my_tiles(unsigned int ntiles)
 }
 
 // ---- sample: one block per segment ----
+// Latency of scattered loads: 7 to 13 us for an array, 33 us for the 187 segments of 2^28 keys.  More samples would narrow
+// what lies outside their range: with 1024 per segment of the second split one sort of 2^27 keys in a few had a cell
+// of outsiders that no bucket holds.
 template <int KB, int FORM, bool PAIRS, int SAMPLES>
 __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl, SplitLevel L, unsigned int decide, typename KeyOf<KB>::type flip)
 {
@@ -372,7 +378,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
         const unsigned long long d = (unsigned long long)(img[j] ^ lo_seen);
 #pragma unroll
         for (int k = 0; k < KB; ++k) bytes |= (d >> (8 * k) & 0xFFu) ? 1u << k : 0u;
-        if (PAIRS && !(FORM != FORM_INT && img[j] == (K)~(K)0)) {
+        if ((PAIRS || FORM != FORM_INT) && !(FORM != FORM_INT && img[j] == (K)~(K)0)) {
           unsigned int h = (unsigned int)img[j] * 2654435761u ^ (unsigned int)((unsigned long long)img[j] >> 32) * 2246822519u;
           h ^= h >> 15;
           h = h * 3266489917u | 1u;
@@ -392,7 +398,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
       unsigned int route = ROUTE_SPLIT;
       // (a sample finds its copies among those before it: half of the square)
       const unsigned long long copies = (unsigned long long)sh_n[0] * 2 * len / ((unsigned long long)ns * ns);
-      if (PAIRS && m.mode != MAP_POS && sh_n[0] >= 16 && copies > 512) route = ROUTE_RADIX;
+      // (of an argsort equal keys have to be taken apart; in a sort of floats, whose cells cannot be seen to hold one value, they
+      // fill cells that nothing splits)
+      if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && sh_n[0] >= 16 && copies > 512) route = ROUTE_RADIX;
       if (PAIRS) {
         // a cell that holds more than the next split takes apart could not be handled later
         const unsigned long long est = (unsigned long long)(most >> 16) * len / ns;
@@ -406,6 +414,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
 }
 
 // ---- cells: counts per cell; a block takes a run of consecutive tiles ----
+// One shared-memory reduction per key.  8-byte keys are bound by memory (2^28 uint64 keys 332 us, 6.5 TB/s), 4-byte keys by
+// issue (2^26 int32 keys 62 us, 4.3 TB/s).
 template <int KB, int FORM, bool PAIRS>
 __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctrl, SplitLevel L, typename KeyOf<KB>::type flip)
 {
@@ -552,6 +562,10 @@ __device__ __forceinline__ bool cell_bounds(const SplitMap& m, unsigned int c0, 
 }
 
 // ---- pack: one block per segment cuts its cells into buckets ----
+// Latency of a handful of dependent steps on chip: 8 to 9 us, up to 50 where many values are filled in.  Walking from bucket to
+// bucket costs 35 cycles each with one lookup per step (220 with the four it takes to tell what a bucket is, hence
+// the list that the block looks at afterwards: float32 sort of 7 * 10^5 keys, this kernel 30 -> 8 us); cells that are small
+// need no walk at all.
 constexpr int PACK_THREADS = 1024;
 inline size_t pack_smem(unsigned int cells) { return (size_t)(cells + 1) * 4 + (size_t)cells * 6; }
 
@@ -784,7 +798,14 @@ split_pack_kernel(Ctrl* ctrl, SplitLevel L, SplitLeaf* leaves, SplitSeg* next_se
 }
 
 // ---- split: moves the keys of a tile to their buckets ----
-// What bounds it is the shared-memory pipe: 32 random words lie three or four deep in the banks.  So every lane
+// What bounds it is the shared-memory pipe (81 % busy for int32 keys, 17.5 wavefronts per 32 keys) and, with two blocks of 64
+// registers per thread on an SM, latency; DRAM is 30 to 40 % busy.  2^28 int32 keys: shared counters and staged
+// bucket numbers 1.12 ms, the counters below 0.99, the next tile's keys on their way while a tile goes out 0.79; 2^28 uint64 keys
+// with positions in order 2.5 -> 1.9 -> 1.6.  Three blocks with smaller tiles lose (int32 2^25 96 -> 122 us: shorter runs, and
+// the counters' scan is shared by fewer keys); a product instead of the table where keys lie evenly takes three
+// wavefronts away and 2 % of the time.
+//
+// 32 random words lie three or four deep in the banks.  So every lane
 // has counters of its own, in its own bank: counting a key and looking its place up take one wavefront each, whatever
 // the keys (keys that come in order would meet in one counter, at two cycles per lane).  The order inside
 // a bucket is the lanes'; bucket and destination of a staged key are found once more from the key, by neighbours that
@@ -972,6 +993,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 2) split_move_kernel(Ctrl* ctrl
 }
 
 // ---- leaves: sorts a bucket on chip ----
+// Like rows of one block (segmerge_kernel): a bucket per key, then networks of 16; bound by issue (81 thread instructions per
+// int32 key, 140 per int64 key, 147 per float32 key with its position) and the shared-memory pipe.  2^26 int32 keys 281 us, 2^25
+// int64 keys 228, 2^25 float32 keys with positions 257.  Bounds that the cells imply save the search for them (int64
+// 2^27 1097 -> 893 us), and buckets of one word each the networks (uint64 argsort of 2^28 keys almost in order 2.7 -> 1.9 ms).  8-byte
+// words get the registers of 24 warps per SM (80): with 64 they spill (int64 2^27 1271 -> 1058 us).  Fetching the next bucket's
+// keys early gained nothing and made 8-byte pairs spill.
 constexpr int LEAF_VT = 16;
 template <int KB, bool PAIRS, int THREADS> struct LeafSmem {
   static constexpr int TILE   = THREADS * LEAF_VT;

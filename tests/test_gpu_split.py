@@ -121,11 +121,11 @@ def test_lengths(split_all, dtype, n):
         _check(_values("nans", n * 3, np.dtype(dtype), n).reshape(3, n), "argsort")
 
 
-@pytest.mark.parametrize("dtype", ["float32", "int64"])
-def test_as_it_is_dispatched(dtype):
-    # (above every border of the dispatch)
+@pytest.mark.parametrize("dtype,n", [("float32", 6_000_011), ("int64", 12_000_017)])
+def test_as_it_is_dispatched(dtype, n):
+    # (above the borders of the dispatch)
     for how in ("normal", "patterns"):
-        a = _values(how, 6_000_011, np.dtype(dtype), 3)
+        a = _values(how, n, np.dtype(dtype), 3)
         for op in ("sort", "argsort"):
             _check(a, op)
 
