@@ -132,16 +132,19 @@ inline long long split_override()
 //   int32 sort, full range         10^7 253 -> 195, 2^24 371 -> 272, 8 * 10^7 1450 -> 1016
 //   float32 sort, normal           1.1 * 10^6 (one split) 69 -> 61, 3.5 (two) 117 -> 119, 6 191 -> 177, 20 450 -> 371, 80 1517 -> 1163
 //   float32 argsort                7 * 10^5 97 -> 61, 2 * 10^6 99 -> 100, 6 230 -> 209, 20 583 -> 517, 80 1853 -> 1747
-//   int32 argsort, full range      2 * 10^7 579 -> 459, 4 1002 -> 843, 8 1819 -> 1583
-//   int64 sort, full range         10^7 601 -> 309, 2 * 10^7 1065 -> 524, 8 3780 -> 1875
-//   int64 argsort, full range      2 * 10^7 1273 -> 676, 8 4495 -> 2435
+//   int64 sort, full range         2.5 * 10^7 1298 -> 586, 8 3780 -> 1875
+//   int64 argsort, full range      2.5 * 10^7 1541 -> 807, 8 4495 -> 2435
 //   float64 sort, normal           2 * 10^5 84 -> 69, 7 131 -> 70, 80 * 10^6 3702 -> 2006
 //   float64 argsort                2 * 10^5 87 -> 70, 4 103 -> 75, 80 * 10^6 4587 -> 2536
-//   uint64 argsort, almost in order  8 * 10^6 248 -> 271, 30 940 -> 769, 2^28 8094 -> 6225
-//   int64 sort, Zipf               8 * 10^6 319 -> 445 (given up late), 30 921 -> 468, 2^28 7174 -> 3120
+//   uint64 argsort, almost in order  3 * 10^7 940 -> 769, 2^28 8094 -> 6225
+//   int64 sort, Zipf               3 * 10^7 921 -> 468, 2^28 7174 -> 3120
 // Whether bytes are constant is not known before the sample; keys that are sent back have paid for it and for the
-// launches (about 15 us for one split, 25 for two; int32 argsort of a hundred values, 6 * 10^6 keys 74 -> 100, 50 346 -> 373).
-// Integers, whose upper bytes often are constant, are tried only where that is a small part.
+// launches (about 15 us for one split, 25 for two).  Integers, whose upper bytes often are constant, are tried only
+// where that is a small part or the splits win all the same.  So int32 argsorts are not tried (full range 4 * 10^7
+// 1002 -> 843 us, but a hundred values 5 * 10^7 346 -> 373), and 8-byte integers not below 2.4 * 10^7 (full range sort 10^7
+// 601 -> 309, but Zipf 8 * 10^6 317 -> 344, almost in order 214 -> 236).  Float64 keys that hold whole numbers differ in
+// five bytes; many copies crowd their cells, which the splits find out late (unique of ids, 5 * 10^6:
+// 334 -> 450 us, sent back by the sample 361).
 template <int KB, int XF>
 inline SplitPlan split_plan_1d(size_t n, bool pairs, bool keys_too, size_t room)
 {
@@ -150,13 +153,13 @@ inline SplitPlan split_plan_1d(size_t n, bool pairs, bool keys_too, size_t room)
   SplitPlan p          = split_plan(n, 1, pairs, room);
   constexpr bool FLOAT = XF == XF_FLOAT;
   size_t least;
-  if (KB == 4) least = !FLOAT ? (pairs ? 40000000 : 16000000) : p.levels != 1 ? 5000000 : pairs ? 600000 : 900000;
-  else least = FLOAT ? 200000 : pairs ? 12000000 : 8000000;
+  if (KB == 4) least = !FLOAT ? (pairs ? SIZE_MAX : 16000000) : p.levels != 1 ? 5000000 : pairs ? 600000 : 900000;
+  else least = FLOAT ? 200000 : 24000000;
   if (n < (over > 0 ? (size_t)over : least)) p.ok = false;
   // (float32 argsort of 2^28 5.80 -> 5.85 ms)
   if (KB == 4 && pairs && n > 100000000 && over < 0) p.ok = false;
   // each byte in which the keys differ is a radix pass
-  if (over <= 0) p.radix_if = KB == 4 ? (pairs || p.levels == 1 ? 0xEu : 0xCu) : FLOAT || pairs ? 0xEu : n < 24000000 ? 0x3Eu : 0u;
+  if (over <= 0) p.radix_if = KB == 4 ? (pairs || p.levels == 1 ? 0xEu : 0xCu) : FLOAT ? 0x3Eu : pairs ? 0xEu : 0u;
   return p;
 }
 

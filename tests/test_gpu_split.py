@@ -121,7 +121,7 @@ def test_lengths(split_all, dtype, n):
         _check(_values("nans", n * 3, np.dtype(dtype), n).reshape(3, n), "argsort")
 
 
-@pytest.mark.parametrize("dtype,n", [("float32", 6_000_011), ("int64", 12_000_017)])
+@pytest.mark.parametrize("dtype,n", [("float32", 6_000_011), ("int64", 24_000_017)])
 def test_as_it_is_dispatched(dtype, n):
     # (above the borders of the dispatch)
     for how in ("normal", "patterns"):
