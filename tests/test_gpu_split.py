@@ -131,15 +131,22 @@ def test_as_it_is_dispatched(dtype, n):
 
 
 def test_in_place_and_other_streams(split_all):
-    """The input stays whole until the last kernel writes; two sorts on two streams do not meet."""
+    """The input stays whole until the last kernel writes; two sorts on two streams, which run at the same time, have a
+    workspace each."""
     import cupynumeric_b200 as num
+    from cupynumeric_b200.runtime import runtime
 
     a, b = (_values("normal", 2_500_001, np.dtype("int64"), k) for k in (5, 6))
     x = num.array(torch.from_numpy(a).cuda())
-    torch.cuda.synchronize()
+    z = num.array(torch.from_numpy(b).cuda())
     side = torch.cuda.Stream()
+    own = runtime.workspace(1 << 16)
     with torch.cuda.stream(side):
-        y = num.sort(num.array(torch.from_numpy(b).cuda()))
+        assert runtime.workspace(1 << 16).data_ptr() != own.data_ptr()
+    del own
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        y = num.sort(z)
     x.sort()
     torch.cuda.synchronize()
     assert np.array_equal(x.to_numpy(), np.sort(a))
