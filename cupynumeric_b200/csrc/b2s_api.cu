@@ -148,6 +148,19 @@ inline int chunk_layout(int dtype, int kb, size_t n, bool argsort, ChunkLayout* 
 // Sizes the single radix sort takes with 32-bit payloads carried through its passes.
 bool local_sort_pos32_supported(size_t n) { return n > SEG_CAP && n < single_sort_limit(); }
 
+// Rounds of resident blocks that a radix pass of a 1-D argsort of n keys takes (4- or 8-byte keys, 148 SMs).
+unsigned int argsort_pass_waves(int kb, size_t n)
+{
+  auto waves = [&](size_t tile, size_t resident) { return (unsigned int)((n + tile * resident - 1) / (tile * resident)); };
+  using M4 = SweepCfg<4, true>;
+  using M8 = SweepCfg<8, true>;
+  using L4 = SweepCfg<4, true, SWEEP_LARGE>;
+  using L8 = SweepCfg<8, true, SWEEP_LARGE>;
+  const bool large = n > MEDIUM_MAX;
+  if (kb == 8) return large ? waves(L8::TILE, 148 * L8::MINCTAS) : waves(M8::TILE, 148 * M8::MINCTAS);
+  return large ? waves(L4::TILE, 148 * L4::MINCTAS) : waves(M4::TILE, 148 * M4::MINCTAS);
+}
+
 // Stable 1-D argsort of keys that carry a 32-bit payload each (pay_in[i] belongs to keys_in[i];
 // null: the payload of element i is i).  out32 == 0: idx_out[k] = index_offset + payload of the
 // k-th smallest key, as int64; out32 (IDX_32): idx_out points to n uint32 values that receive the bare

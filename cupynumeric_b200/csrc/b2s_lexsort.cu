@@ -8,7 +8,7 @@
 // Neighbouring keys of at most eight bytes together are one key to the radix passes: the gather puts their
 // order-preserving images side by side.  The passes are those of the bytes that differ, as before; a gather, a histogram and
 // the passes that find nothing to do are saved for every key that joins another (4000037 rows of float64, int32, int16:
-// the two integers 220 -> 150 us).
+// the two integers 220 -> 150 us), but every pass moves 8-byte keys: see lex_worth.
 #include <cuda_runtime.h>
 
 #include "../../include/b200sort.h"
@@ -19,6 +19,7 @@ namespace b2s {
 bool local_sort_pos32_supported(size_t n);
 int local_sort_payload32(int dtype, const void* keys_in, const uint32_t* pay_in, int64_t* idx_out, size_t n,
                          int64_t index_offset, void* ws, size_t ws_bytes, cudaStream_t stream, int out32 = 0);
+unsigned int argsort_pass_waves(int kb, size_t n);
 
 static size_t lex_elem_bytes(int dtype)
 {
@@ -80,13 +81,30 @@ __global__ void lex_join_kernel(LexParts parts, const uint32_t* __restrict__ ord
   }
 }
 
+// Whether joining `m` keys of `bytes` together pays.  A joined pass moves 8-byte keys: a round of its resident blocks takes
+// 15 us where one of a 4-byte pass takes 18.7 for 1.7 times the keys, so it pays where the rounds are about as many, and what
+// joining saves besides, a gather and a histogram per key, tells where both last one round.  Key by key against joined,
+// us, every byte differing:
+//   int32, int32      3 * 10^5 rows 103 -> 93, 8 * 10^5 210 -> 143, 2 * 10^6 (a round each) 215 -> 205, 3 (one, two) 262 -> 297,
+//                     4 (two each) 403 -> 333, 5 (two, three) 439 -> 459, 7 (two, four) 525 -> 602, 16 (five, eight) 1069 -> 1126;
+//                     2^20 rows, whose 4-byte tiles are all full, 151 -> 160
+//   float32, uint16   2 * 10^6 182 -> 161, 3 219 -> 234, 4 317 -> 262, 16 * 10^6 707 -> 866
+//   uint8, uint8      3 * 10^5 45 -> 47, 2 * 10^6 72 -> 81, 16 * 10^6 287 -> 394: short keys have cheap passes of their own
+//   eight of uint8    3 * 10^5 198 -> 99, 3 * 10^6 405 -> 327, 7 711 -> 671, 16 * 10^6 1401 -> 1289: many keys save many gathers
+static bool lex_worth(int m, size_t bytes, size_t volume)
+{
+  if (m >= 5) return true;
+  if (m == 2 && bytes <= 4) return false;
+  return argsort_pass_waves(8, volume) * 4 <= argsort_pass_waves(4, volume) * 5;
+}
+
 // Keys k .. k + lex_group() - 1 are sorted as one.
-static int lex_group(int nkeys, const int* dtypes, int k)
+static int lex_group(int nkeys, const int* dtypes, int k, size_t volume)
 {
   size_t bytes = 0;
   int m        = 0;
   while (k + m < nkeys && m < 8 && bytes + lex_elem_bytes(dtypes[k + m]) <= 8) bytes += lex_elem_bytes(dtypes[k + m++]);
-  return m > 1 ? m : 1;
+  return m > 1 && lex_worth(m, bytes, volume) ? m : 1;
 }
 
 static int lex_xf(int dtype)
@@ -125,8 +143,8 @@ static int lex_layout(int nkeys, const int* dtypes, size_t volume, size_t segmen
 {
   size_t max_eb = 0, max_ws = 0;
   if (joined) {
-    for (int k = 0; k < nkeys; k += lex_group(nkeys, dtypes, k)) {
-      if (lex_group(nkeys, dtypes, k) < 2) continue;
+    for (int k = 0; k < nkeys; k += lex_group(nkeys, dtypes, k, volume)) {
+      if (lex_group(nkeys, dtypes, k, volume) < 2) continue;
       const int rc = b2s_workspace_bytes(B2S_UINT64, volume, segment, 1, &max_ws);
       if (rc != B2S_OK) return rc;
       max_eb = 8;
@@ -158,7 +176,7 @@ static bool lex_joins(const int* dtypes, int nkeys, size_t volume, size_t segmen
   bool some = false;
   for (int k = 0; k < nkeys; ++k) {
     if (dtypes[k] == B2S_COMPLEX128) return false;
-    some = some || lex_group(nkeys, dtypes, k) > 1;
+    some = some || lex_group(nkeys, dtypes, k, volume) > 1;
   }
   return some && volume == segment && local_sort_pos32_supported(volume);
 }
@@ -214,7 +232,7 @@ int b2s_lexsort(int nkeys, const int* dtypes, const void* const* keys, int64_t* 
     uint32_t* pos[2] = {reinterpret_cast<uint32_t*>(ord[0]), reinterpret_cast<uint32_t*>(ord[1])};
     int cur = 0;
     for (int k = 0, step = 1; k < nkeys; k += step) {
-      step = joined ? lex_group(nkeys, dtypes, k) : 1;
+      step = joined ? lex_group(nkeys, dtypes, k, volume) : 1;
       const bool last = k + step == nkeys;
       const int dtype = step > 1 ? (int)B2S_UINT64 : dtypes[k];
       // joined keys lie in clusters and later keys have few values: the splits give up on them, late (two int32 keys of 100000 and 200

@@ -7,8 +7,6 @@ import numpy as np
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
-
 KEYS = [("float64", "int32", "int16"), ("int32", "int32"), ("float32", "uint16"), ("bool", "int8", "float16", "uint32", "int64"),
         ("int8",) * 9, ("uint16", "float32", "int16", "float64", "uint8", "int8"), ("int64", "int32", "uint64"), ("int32", "int64", "uint32", "float32")]
 
@@ -30,6 +28,28 @@ def _columns(names, n, seed):
     return out
 
 
+def _row_bytes(names, n):
+    from cupynumeric_b200 import _lib
+
+    need, codes = ctypes.c_size_t(), (ctypes.c_int * len(names))(*[_lib.DTYPE_CODE[np.dtype(d)] for d in names])
+    _lib.check(_lib.lib().b2s_lexsort_workspace_bytes(len(names), codes, n, n, ctypes.byref(need)), "ws")
+    return need.value / n
+
+
+@pytest.mark.parametrize("names,joined", [
+    # rows at which keys are joined; the others' workspace has no room for an 8-byte key
+    (("int32", "int32"), [2_000_003, 4_000_037]),
+    (("float32", "uint16"), [2_000_003, 4_000_037]),
+    (("uint8", "uint8"), []),
+    (("int16", "int16"), []),
+    (("uint8",) * 8, [2_000_003, 3_000_017, 4_000_037, 16_000_057]),
+], ids=lambda v: "-".join(v) if isinstance(v, tuple) else "")
+def test_what_is_joined(names, joined):
+    for n in (2_000_003, 3_000_017, 4_000_037, 16_000_057):
+        assert (_row_bytes(names, n) > 50) == (n in joined), n
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [8192, 8193, 100_003])
 @pytest.mark.parametrize("names", KEYS, ids="-".join)
 def test_joined_keys(names, n):
@@ -39,6 +59,18 @@ def test_joined_keys(names, n):
     assert np.array_equal(num.lexsort(cols).to_numpy(), np.lexsort(cols))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2_121_728, 2_121_729])
+def test_around_the_length_where_joining_ends(n):
+    import cupynumeric_b200 as num
+
+    names = ("float64", "int32", "uint16", "int8")
+    assert (_row_bytes(names[1:], n) > 50) == (n == 2_121_728)
+    cols = _columns(names, n, 4)
+    assert np.array_equal(num.lexsort(cols).to_numpy(), np.lexsort(cols))
+
+
+@pytest.mark.gpu
 def test_a_workspace_without_room_for_joined_keys():
     from cupynumeric_b200 import _lib
 
