@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 // float32 digit extraction through one floating-point add (see to_ordered)
@@ -133,7 +134,8 @@ struct FixDesc {
 };
 
 enum : int { IDX_32 = 1, IDX_PASSES_ONLY = 2 };  // how an argsort is asked for (launch_radix_1d)
-enum : unsigned int { ROUTE_OPEN = 0, ROUTE_SPLIT = 1, ROUTE_RADIX = 2 };
+// Who sorts: open, the splitting kernels, the radix passes since the sample, the radix passes since a later kernel gave up.
+enum : unsigned int { ROUTE_OPEN = 0, ROUTE_SPLIT = 1, ROUTE_RADIX = 2, ROUTE_LATE = 3 };
 
 struct Ctrl {
   unsigned int status;                  // 0 or a b2s_status_t, written by kernels
@@ -148,6 +150,7 @@ struct Ctrl {
   PassDesc pass[MAX_PASSES];
   FixDesc fix;
 };
+static_assert(offsetof(Ctrl, route) == 48, "the tests read who sorted there");
 
 constexpr unsigned int DEV_ERR_TIMEOUT = 5;  // == B2S_ERR_TIMEOUT
 

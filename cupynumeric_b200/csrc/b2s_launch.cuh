@@ -144,7 +144,11 @@ inline long long split_override()
 // 1002 -> 843 us, but a hundred values 5 * 10^7 346 -> 373), and 8-byte integers not below 2.4 * 10^7 (full range sort 10^7
 // 601 -> 309, but Zipf 8 * 10^6 317 -> 344, almost in order 214 -> 236).  Float64 keys that hold whole numbers differ in
 // five bytes; many copies crowd their cells, which the splits find out late (unique of ids, 5 * 10^6:
-// 334 -> 450 us, sent back by the sample 361).
+// 334 -> 450 us, sent back by the sample 361).  Of int64 sorts two differing bytes go back (65536 values, 8 * 10^7 1110 -> 1655),
+// one and three do not (a hundred values 670 -> 644, 2^24 values 2.4 * 10^7 544 -> 503, 8 1559 -> 1629).
+// Argsorts of keys that are alike as far as the sample sees need few passes, and the splits, which cut them by position, give up
+// late: they go back (one value, 2.4 * 10^7 int64 148 us by the passes, by the splits 519; 8 * 10^6 float64 73, 935).  Sorts of such
+// integers stay: one value costs more (2.4 * 10^7 int64 176 -> 245, int32 of 1.6 * 10^7 70 -> 130), but one value and a few others less.
 template <int KB, int XF>
 inline SplitPlan split_plan_1d(size_t n, bool pairs, bool keys_too, size_t room)
 {
@@ -159,7 +163,7 @@ inline SplitPlan split_plan_1d(size_t n, bool pairs, bool keys_too, size_t room)
   // (float32 argsort of 2^28 5.80 -> 5.85 ms)
   if (KB == 4 && pairs && n > 100000000 && over < 0) p.ok = false;
   // each byte in which the keys differ is a radix pass
-  if (over <= 0) p.radix_if = KB == 4 ? (pairs || p.levels == 1 ? 0xEu : 0xCu) : FLOAT ? 0x3Eu : pairs ? 0xEu : 0u;
+  if (over <= 0) p.radix_if = KB == 4 ? (pairs ? 0xFu : p.levels == 1 ? 0xEu : 0xCu) : FLOAT ? (pairs ? 0x3Fu : 0x3Eu) : pairs ? 0xFu : 0x4u;
   return p;
 }
 

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
     });
   }
   flush();
-  if (FORM == FORM_FLOAT && !PAIRS && special) atomicMax(&ctrl->route, (unsigned int)ROUTE_RADIX);
+  if (FORM == FORM_FLOAT && !PAIRS && special) atomicMax(&ctrl->route, (unsigned int)ROUTE_LATE);
 }
 
 // The only image of a cell, where it has one.
@@ -758,7 +758,7 @@ split_pack_kernel(Ctrl* ctrl, SplitLevel L, SplitLeaf* leaves, SplitSeg* next_se
     tiles   = L.last ? 0 : (len + next_tile - 1) / next_tile;
   }
   if (__syncthreads_or(fail)) {
-    if (tid == 0) atomicMax(&ctrl->route, (unsigned int)ROUTE_RADIX);
+    if (tid == 0) atomicMax(&ctrl->route, (unsigned int)ROUTE_LATE);
     return;
   }
   unsigned int all_entries, all_tiles;

@@ -63,11 +63,25 @@ def _values(how: str, n: int, dtype: np.dtype, seed: int) -> np.ndarray:
     return np.full(n, 7 if how == "equal" else info.max, dtype)
 
 
-def _check(a: np.ndarray, op: str) -> None:
+OPEN, SPLIT, RADIX, LATE = range(4)   # who sorted: nobody tried, the splits, the passes since the sample, since later
+
+
+def _device(a: np.ndarray) -> torch.Tensor:
+    d = torch.from_numpy(a.view(f"i{a.dtype.itemsize}") if a.dtype.kind == "u" else a).cuda()
+    return d.view({"u4": torch.uint32, "u8": torch.uint64}[a.dtype.str[1:]]) if a.dtype.kind == "u" else d
+
+
+def _route() -> int:
+    """Of the last sort of this thread: a word of the control block at the head of its workspace."""
+    from cupynumeric_b200.runtime import runtime
+
+    return int(runtime.workspace(1)[48:52].view(torch.int32).item())
+
+
+def _check(a: np.ndarray, op: str) -> int:
     import cupynumeric_b200 as num
 
-    d = torch.from_numpy(a.view(f"i{a.dtype.itemsize}") if a.dtype.kind == "u" else a).cuda()
-    d = d.view({"u4": torch.uint32, "u8": torch.uint64}[a.dtype.str[1:]]) if a.dtype.kind == "u" else d
+    d = _device(a)
     order = np.argsort(a, axis=-1, kind="stable")
     if op == "argsort":
         got = num.argsort(num.array(d), axis=-1, kind="stable").to_numpy()
@@ -76,6 +90,7 @@ def _check(a: np.ndarray, op: str) -> None:
         got  = num.sort(num.array(d), axis=-1).to_numpy()
         want = np.take_along_axis(a, order, axis=-1)
         assert np.array_equal(got.view(f"u{a.dtype.itemsize}"), want.view(f"u{a.dtype.itemsize}"))
+    return _route()
 
 
 HOW = ["normal", "nans", "patterns", "wide", "spike", "few", "crowded", "equal", "last"]
@@ -128,6 +143,18 @@ def test_as_it_is_dispatched(dtype, n):
         a = _values(how, n, np.dtype(dtype), 3)
         for op in ("sort", "argsort"):
             _check(a, op)
+
+
+@pytest.mark.parametrize("dtype,op,n", [("float32", "argsort", 700_001), ("float32", "argsort", 5_000_011), ("float64", "argsort", 250_007),
+                                        ("int64", "argsort", 24_000_017), ("int64", "sort", 24_000_017)])
+def test_sent_back_with_the_sample(dtype, op, n):
+    """Keys that need few passes: alike as far as the sample sees, or, in a sort of int64, of two differing bytes."""
+    if op == "argsort":
+        a = np.full(n, 3, np.dtype(dtype))
+        a[n // 2] = 4
+    else:
+        a = np.random.default_rng(5).integers(0, 65536, n).astype(dtype)
+    assert _check(a, op) == RADIX
 
 
 def test_in_place_and_other_streams(split_all):
