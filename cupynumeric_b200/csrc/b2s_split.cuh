@@ -20,8 +20,8 @@
 //
 // A cell that holds a single value of which a sort has many copies is not moved at all: its place in the
 // result is filled in at the end.  What cannot be cut finely enough (a heavily repeated key of an argsort,
-// values that crowd at a scale of their own) or needs input order among keys of equal image (-0.0, several NaN
-// patterns) is left to the radix passes: `route` in the control block says so before anything of the output is
+// values that crowd at a scale of their own) or needs input order among keys of equal image (zeros of both signs, NaNs of
+// several patterns) is left to the radix passes: `route` in the control block says so before anything of the output is
 // written, and the radix kernels, launched behind, return at once where it says otherwise.
 #pragma once
 
@@ -60,6 +60,7 @@ struct SplitLevel {
   unsigned int last;          // buckets are leaves (else segments of the next level)
   unsigned int pos_n;         // positions lie below this
   unsigned int radix_if;      // bit k: keys that differ in k bytes are left to the radix passes
+  SplitMarks* marks;
   const void* src_keys;
   const uint32_t* src_pos;    // null: the place inside the segment
   void* dst_keys;
@@ -78,6 +79,51 @@ __device__ __forceinline__ typename KeyOf<KB>::type split_image(typename KeyOf<K
   if constexpr (FORM == FORM_FLOAT) return to_ordered<KB, XF_FLOAT>(raw);
   else if constexpr (FORM == FORM_IMAGE) return raw;
   else return (typename KeyOf<KB>::type)(raw ^ flip);
+}
+
+// Zeros of both signs have one image, and so have all NaNs.  Where a sort holds one pattern of each, that is what its result gets;
+// of several it would have to keep the input order, which the radix passes do.  The patterns of a warp's threads:
+template <int KB> struct MarksSeen {
+  using K        = typename KeyOf<KB>::type;
+  K nan          = 0;
+  unsigned int zeros = 0;
+  bool mixed     = false;
+  __device__ __forceinline__ void see(K raw, K image)
+  {
+    if (image == (K)~(K)0) {
+      mixed |= nan != 0 && nan != raw;
+      nan = raw;
+    } else if (image == (K)((K)1 << (8 * KB - 1))) {
+      zeros |= raw == 0 ? 1u : 2u;
+    }
+  }
+  // into `to` (of the block, or of the sort); by whole warps
+  __device__ __forceinline__ void into(SplitMarks* to)
+  {
+    const unsigned int with = __ballot_sync(0xFFFFFFFFu, nan != 0);
+    zeros                   = __reduce_or_sync(0xFFFFFFFFu, zeros);
+    const unsigned int from = with ? __ffs(with) - 1 : 0;
+    const K first           = __shfl_sync(0xFFFFFFFFu, nan, from);
+    mixed |= nan != 0 && nan != first;
+    mixed = __any_sync(0xFFFFFFFFu, mixed);
+    if ((threadIdx.x & 31) == from) {
+      if (with) {
+        const unsigned long long old = atomicCAS(&to->nan, 0ull, (unsigned long long)first);
+        mixed |= old != 0 && old != (unsigned long long)first;
+      }
+      if (zeros) zeros |= atomicOr(&to->zeros, zeros);
+      mixed |= zeros == 3;
+    }
+  }
+};
+template <int KB>
+__device__ __forceinline__ typename KeyOf<KB>::type split_raw(typename KeyOf<KB>::type o, typename KeyOf<KB>::type nan, typename KeyOf<KB>::type zero)
+{
+  using K        = typename KeyOf<KB>::type;
+  constexpr K SB = (K)((K)1 << (8 * KB - 1));
+  if (o == (K)~(K)0) return nan;
+  if (o == SB) return zero;
+  return (o & SB) ? (K)(o ^ SB) : (K)~o;
 }
 
 template <int KB> struct FloatOf { using type = float; };
@@ -160,6 +206,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
   __shared__ K sh_b[2 * SPLIT_THREADS / 32];
   __shared__ unsigned int sh_n[2], sh_most[2], sh_eq[2];
   __shared__ unsigned long long sh_lo, sh_hi;
+  __shared__ SplitMarks sh_marks;
   const unsigned int seg = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   chain_wait();
   if (!decide && ctrl->route != ROUTE_SPLIT) return;
@@ -192,9 +239,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
   }
   auto mine = [&](int j) { return j * SPLIT_THREADS + tid < ns; };
   K lo = (K)~(K)0, hi = 0;
+  MarksSeen<KB> seen;
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
+    const K raw = img[j];
     img[j] = split_image<KB, FORM>(img[j], flip);
+    if (FORM == FORM_FLOAT && !PAIRS && mine(j)) seen.see(raw, img[j]);
     // (of floats the finite ones count)
     if (mine(j) && !(FORM != FORM_INT && (unsigned int)(img[j] >> (8 * KB - 32)) - FIN_LO >= 0u - 2u * FIN_LO)) {
       lo = img[j] < lo ? img[j] : lo;
@@ -213,8 +263,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
   }
   if (tid < 2) sh_n[tid] = sh_most[tid] = sh_eq[tid] = 0;
   if (tid == 0) {
-    sh_lo = ~0ull;
-    sh_hi = 0;
+    sh_lo    = ~0ull;
+    sh_hi    = 0;
+    sh_marks = SplitMarks{};
   }
   for (unsigned int i = tid; i < L.cells; i += SPLIT_THREADS) sh_cells[i] = 0;
   __syncthreads();
@@ -371,6 +422,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
     for (unsigned int i = tid; i < SPLIT_PRINTS; i += SPLIT_THREADS) table[i] = 0;
     if (tid == 0) sh_n[0] = sh_n[1] = 0;
     __syncthreads();
+    if (FORM == FORM_FLOAT && !PAIRS) seen.into(&sh_marks);
+    const bool mixed = __syncthreads_or(seen.mixed);
     unsigned int same = 0, bytes = 0;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
@@ -395,7 +448,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
     }
     __syncthreads();
     if (tid == 0) {
-      unsigned int route = ROUTE_SPLIT;
+      unsigned int route = mixed ? ROUTE_RADIX : ROUTE_SPLIT;
       // (a sample finds its copies among those before it: half of the square)
       const unsigned long long copies = (unsigned long long)sh_n[0] * 2 * len / ((unsigned long long)ns * ns);
       // (of an argsort equal keys have to be taken apart; in a sort of floats, whose cells cannot be seen to hold one value, they
@@ -422,17 +475,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
   using K             = typename KeyOf<KB>::type;
   constexpr int ITEMS = SplitCfg<KB, PAIRS>::ITEMS, TILE = SplitCfg<KB, PAIRS>::TILE;
   extern __shared__ unsigned int h[];
+  __shared__ SplitMarks sh_marks;
   chain_wait();
   if (__syncthreads_or(ld_relaxed(&ctrl->route) != ROUTE_SPLIT)) return;  // (other blocks may be changing it)
   const unsigned int tid = threadIdx.x;
   const TileRange r = my_tiles(L.tile_seg ? ctrl->split_ntiles : L.nseg * L.tiles_per_seg);
   if (r.first >= r.end) return;
   for (unsigned int i = tid; i < L.cells; i += SPLIT_THREADS) h[i] = 0;
+  if (tid == 0) sh_marks = SplitMarks{};
   __syncthreads();
   const unsigned int ci = L.cells - 2 - split_nan_cells(FORM, PAIRS, L.cells);
   unsigned int cur = 0xFFFFFFFFu;
   SplitSeg s{};
-  bool special = false;
+  MarksSeen<KB> seen;
   auto flush = [&] {
     __syncthreads();
     unsigned int* out = L.hist + (size_t)cur * L.cells;
@@ -471,10 +526,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
         const unsigned int e = j * SPLIT_THREADS + tid;
         if (PART && e >= valid) continue;
         const K x = split_image<KB, FORM>(key[j], flip);
-        if (FORM == FORM_FLOAT && !PAIRS) {
-          // images that fold several bit patterns: the radix passes keep their input order
-          if (x == (K)~(K)0 || x == (K)((K)1 << (8 * KB - 1))) special |= sm_is_special<KB>(key[j], XF_FLOAT);
-        }
+        if (FORM == FORM_FLOAT && !PAIRS) seen.see(key[j], x);
         if (PAIRS && MODE != MAP_POS && FORM != FORM_INT && x == (K)~(K)0) {
           nans |= 1u << j;   // ordered by position, which is fetched for them alone
           continue;
@@ -497,7 +549,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
     });
   }
   flush();
-  if (FORM == FORM_FLOAT && !PAIRS && special) atomicMax(&ctrl->route, (unsigned int)ROUTE_LATE);
+  if (FORM == FORM_FLOAT && !PAIRS) {
+    // the warps' patterns to the block's, and those to the sort's
+    seen.into(&sh_marks);
+    bool mixed = __syncthreads_or(seen.mixed);
+    if (tid < 32 && (sh_marks.nan != 0 || sh_marks.zeros != 0)) {
+      seen.nan   = (K)sh_marks.nan;
+      seen.zeros = sh_marks.zeros;
+      seen.mixed = false;
+      seen.into(L.marks);
+      mixed |= seen.mixed;
+    }
+    if (mixed && tid < 32) atomicMax(&ctrl->route, (unsigned int)ROUTE_LATE);
+  }
 }
 
 // The only image of a cell, where it has one.
@@ -695,7 +759,8 @@ split_pack_kernel(Ctrl* ctrl, SplitLevel L, SplitLeaf* leaves, SplitSeg* next_se
       if (b == c && filled(c, &image)) {
         const unsigned int len = pre[c + 1] - pre[c], begin = s.begin + pre[c];
         unsigned long long raw;
-        if constexpr (FORM != FORM_INT) raw = (unsigned long long)sm_from_ordered<KB>((K)image, XF_FLOAT);
+        if constexpr (FORM != FORM_INT)
+          raw = (unsigned long long)split_raw<KB>((K)image, (K)L.marks->nan, (L.marks->zeros & 2u) ? (K)((K)1 << (8 * KB - 1)) : (K)0);
         else raw = (unsigned long long)(K)((K)image ^ flip);
         const unsigned int parts = (len + FILL_CHUNK - 1) / FILL_CHUNK, e = atomicAdd(&ctrl->split_nleaf, parts);
         for (unsigned int i = 0; i < parts; ++i)
@@ -1013,6 +1078,7 @@ template <int KB, bool PAIRS, int THREADS> struct LeafSmem {
 
 struct LeafArgs {
   const SplitLeaf* leaves;
+  const SplitMarks* marks;
   const void* keys;
   const uint32_t* pos;
   void* out;
@@ -1202,6 +1268,9 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
   if (ctrl->route != ROUTE_SPLIT) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned int nleaf = ctrl->split_nleaf;
+  // the patterns of NaNs and zeros
+  const K nan  = FORM != FORM_INT && !PAIRS ? (K)A.marks->nan : (K)0;
+  const K zero = FORM != FORM_INT && !PAIRS && (A.marks->zeros & 2u) ? (K)((K)1 << (8 * KB - 1)) : (K)0;
   for (unsigned int l = blockIdx.x; l < nleaf; l += gridDim.x) {
     const SplitLeaf leaf = A.leaves[l];
     if (leaf.len & LEAF_FILL) {
@@ -1243,7 +1312,7 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
           if (count[mid] > i) b = mid; else a = mid + 1;
         }
         const K o = (K)((K)leaf.lo + a);
-        if constexpr (FORM != FORM_INT) to[i] = sm_from_ordered<KB>(o, XF_FLOAT);
+        if constexpr (FORM != FORM_INT) to[i] = split_raw<KB>(o, nan, zero);
         else to[i] = (K)(o ^ flip);
       }
       __syncthreads();
@@ -1379,7 +1448,7 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
         leaf_order<W, false, THREADS>(img, none, bk, exact && FORM == FORM_INT, sw, sp, cnt, wsum);
         for (unsigned int e = tid; e < n; e += THREADS) {
           const K o = (K)sw[smpad(e)];
-          if constexpr (FORM != FORM_INT) dst[e] = sm_from_ordered<KB>(o, XF_FLOAT);
+          if constexpr (FORM != FORM_INT) dst[e] = split_raw<KB>(o, nan, zero);
           else dst[e] = (K)(o ^ flip);
         }
       }
@@ -1429,6 +1498,7 @@ inline cudaError_t split_form(typename KeyOf<KB>::type flip, const SplitPlan& pl
     L.last          = l == plan.levels - 1;
     L.pos_n         = job.seg_len;
     L.radix_if      = plan.radix_if;
+    L.marks         = reinterpret_cast<SplitMarks*>(job.tables + plan.off_marks);
     L.src_keys      = l == 0 ? job.in : job.tmp_keys[0];
     L.src_pos       = PAIRS && l > 0 ? job.tmp_pos[0] : nullptr;
     L.dst_keys      = job.tmp_keys[l];
@@ -1474,6 +1544,7 @@ inline cudaError_t split_form(typename KeyOf<KB>::type flip, const SplitPlan& pl
   }
   LeafArgs A{};
   A.leaves       = leaves;
+  A.marks        = reinterpret_cast<const SplitMarks*>(job.tables + plan.off_marks);
   A.keys         = job.tmp_keys[plan.levels - 1];
   A.pos          = PAIRS ? job.tmp_pos[plan.levels - 1] : nullptr;
   A.out          = job.out;

@@ -44,6 +44,12 @@ struct SplitLeaf {
   unsigned long long lo, span;
 };
 
+// What the float keys of a sort without positions hold, of the two images that stand for several bit patterns each.
+struct SplitMarks {
+  unsigned long long nan;  // the NaNs' pattern; 0: none seen
+  unsigned int zeros;      // 1: zeros seen, 2: negative zeros
+};
+
 // Shape of one split.
 struct SplitShape {
   unsigned int nseg;   // most segments
@@ -56,7 +62,7 @@ struct SplitPlan {
   unsigned int radix_if;     // bit k: keys that differ in k bytes are left to the radix passes
   SplitShape lev[2];
   size_t zero_bytes;  // from the start: what has to be clear
-  size_t off_hist[2], off_segs[2], off_lut[2], off_cursor[2], off_tile_seg, off_leaves, total;
+  size_t off_marks, off_hist[2], off_segs[2], off_lut[2], off_cursor[2], off_tile_seg, off_leaves, total;
 };
 
 // nseg segments of seg_len keys; `room` bytes for the tables (the look-back tables of the radix passes, which are
@@ -87,7 +93,8 @@ inline SplitPlan split_plan(size_t seg_len, size_t nseg, bool pairs, size_t room
     p.lev[0] = SplitShape{1u, b1 > 100 ? 8192u : 4096u, (unsigned int)(seg_len / b1)};
     p.lev[1] = SplitShape{2 * b1 + 2 < SPLIT_BINS ? 2 * b1 + 2 : SPLIT_BINS, b1 > 100 && !pairs ? 8192u : 4096u, cap};
   }
-  size_t off = 0;
+  p.off_marks = 0;
+  size_t off  = 256;
   for (int l = 0; l < p.levels; ++l) {
     p.off_hist[l] = off;
     off += align_up((size_t)p.lev[l].nseg * p.lev[l].cells * 4, 256);

@@ -157,6 +157,35 @@ def test_sent_back_with_the_sample(dtype, op, n):
     assert _check(a, op) == RADIX
 
 
+@pytest.mark.parametrize("dtype,rows,n", [("float64", 1, 250_007), ("float32", 1, 5_000_011), ("float64", 37, 20_011), ("float32", 60, 20_011)])
+def test_patterns_of_zeros_and_nans(dtype, rows, n):
+    """A sort keeps the one pattern that its zeros have, and its NaNs; where there are several the passes take it, at once if
+    the sample sees them."""
+    t, bits = np.dtype(dtype), np.dtype(dtype).itemsize * 8
+    rng = np.random.default_rng(n)
+    base = (rng.standard_normal(rows * n) + 0.5).astype(t)
+    odd = np.array((1 << (bits - 1)) - 1, f"u{t.itemsize}").view(t)       # what arithmetic on a GPU gives
+    neg = np.array(((1 << bits) - 1) ^ 4, f"u{t.itemsize}").view(t)
+
+    def case(*parts):
+        a = base.copy()
+        for value, places in parts:
+            a[places] = value
+        return _check(a.reshape((rows, n) if rows > 1 else n), "sort")
+
+    some, more = (rng.integers(0, rows * n, rows * n // 50) for _ in range(2))
+    few = rng.integers(0, rows * n, 500)     # (no more copies of a zero than a leaf holds)
+    one = np.array([rows * n // 3])
+    assert case() == SPLIT
+    assert case((-0.0, few), (odd, more)) == SPLIT
+    assert case((0.0, few), (neg, one)) == SPLIT
+    assert case((-0.0, one)) == SPLIT
+    assert case((odd, some), (np.nan, more)) == RADIX
+    assert case((0.0, some), (-0.0, more)) == RADIX
+    assert case((odd, one), (np.nan, one + 1)) in (RADIX, LATE)
+    assert case((0.0, one), (-0.0, one + n // 3)) in (RADIX, LATE)
+
+
 def test_in_place_and_other_streams(split_all):
     """The input stays whole until the last kernel writes; two sorts on two streams, which run at the same time, have a
     workspace each."""
