@@ -46,14 +46,15 @@ def local_sort_tile(tile: torch.Tensor, argsort: bool, stable: bool, index_offse
     need = ctypes.c_size_t(0)
     _lib.check(lib.b2s_workspace_bytes(code, volume, segment, int(argsort), ctypes.byref(need)),
                "b2s_workspace_bytes")
-    ws = runtime.workspace(need.value)
+    device = torch.cuda.current_device()
+    stream = torch.cuda.current_stream(device).cuda_stream
+    own = runtime.scratch(need.value, device, stream)
     st = lib.b2s_local_sort(code, tile.data_ptr(), None if argsort else out.data_ptr(),
                             out.data_ptr() if argsort else None, volume, segment, int(index_offset),
-                            int(tile.ndim == 1), int(stable), ws.data_ptr(), ws.numel(),
-                            runtime.stream_handle())
+                            int(tile.ndim == 1), int(stable), own.ptr, own.nbytes, stream)
     _lib.check(st, "b2s_local_sort")
     if segment > ON_CHIP and tile.dtype != torch.complex128:  # (its inner sorts keep their control blocks elsewhere)
-        runtime.note_sort(ws)
+        runtime.note_sort(own)
     return out
 
 

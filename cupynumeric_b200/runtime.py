@@ -9,7 +9,6 @@ Plays the role the Legate runtime plays for the reference's SORT task: it owns d
 from __future__ import annotations
 
 import threading
-from collections import OrderedDict
 
 import torch
 import torch.distributed as dist
@@ -17,16 +16,27 @@ import torch.distributed as dist
 from . import _lib
 
 
+class Scratch:
+    """What the calls of one thread on one stream sort with: a workspace, and the word that keeps the status of its sorts."""
+
+    __slots__ = ("ws", "ptr", "nbytes", "status", "failed", "used")
+
+    def __init__(self, ws: torch.Tensor, failed: torch.Tensor) -> None:
+        self.ws, self.failed, self.used = ws, failed, 0
+        self.ptr, self.nbytes, self.status = ws.data_ptr(), ws.numel(), ws[:4].view(torch.int32)
+
+
 class Runtime:
     KEPT = 8       # workspaces kept per process, least recently used first out
     STICKY = 64    # status words kept per process
 
     def __init__(self) -> None:
-        # (device, stream, thread) -> the workspace and the status word at its head
-        self._ws: OrderedDict[tuple[int, int, int], tuple[torch.Tensor, torch.Tensor]] = OrderedDict()
-        self._sticky: dict[tuple[int, int], torch.Tensor] = {}   # (device, stream) -> status of its sorts so far
-        self._failed: dict[int, int] = {}                        # device -> status read but not raised yet
+        # by (device, stream, thread)
+        self._kept: dict[tuple[int, int, int], Scratch] = {}
+        self._sticky: dict[tuple[int, int, int], torch.Tensor] = {}   # status of the sorts so far
+        self._failed: dict[int, int] = {}                             # device -> status read but not raised yet
         self._lock = threading.Lock()
+        self._calls = 0
         self._comm = None
 
     # --- topology -------------------------------------------------------------------------
@@ -52,60 +62,61 @@ class Runtime:
         return torch.cuda.current_stream().cuda_stream
 
     # --- scratch memory -------------------------------------------------------------------
-    def _scratch(self, nbytes: int) -> torch.Tensor:
+    def _bytes(self, nbytes: int) -> torch.Tensor:
         return torch.empty(nbytes, dtype=torch.uint8, device=self.device)
 
-    def workspace(self, nbytes: int) -> torch.Tensor:
-        """A 256-byte aligned device buffer of at least ``nbytes``, reused by the calls of one thread on
-        one stream of one device.  These are ordered.  Sorts of two streams run at the same time, and two
-        threads enqueue the kernels of their sorts in any order even on one stream; the kernels of a sort take
-        their store addresses from its workspace, so such sorts never share one.  A buffer that goes returns to the
-        allocator, which hands it out again on the stream it was made on."""
-        key = (torch.cuda.current_device(), self.stream_handle(), threading.get_ident())
+    def scratch(self, nbytes: int, device: int, stream: int) -> Scratch:
+        """A workspace of at least ``nbytes``, 256-byte aligned, for a call on this stream, the current one of
+        the current device.  It is reused by the calls of one thread on one stream: these are ordered.  Sorts of two streams
+        run at the same time, and two threads enqueue the kernels of their sorts in any order even on one
+        stream; the kernels of a sort take their store addresses from its workspace, so such sorts never share one.  A buffer
+        that goes returns to the allocator, which hands it out again on the stream it was made on."""
+        key = (device, stream, threading.get_ident())
+        self._calls += 1
+        own = self._kept.get(key)
+        if own is None or own.nbytes < nbytes:
+            own = self._renew(key, max(int(nbytes), 1 << 16))
+        own.used = self._calls
+        return own
+
+    def _renew(self, key: tuple[int, int, int], nbytes: int) -> Scratch:
         with self._lock:
-            cur = self._ws.get(key)
-            if cur is not None and cur[0].numel() >= nbytes:
-                self._ws.move_to_end(key)
-                return cur[0]
-            self._ws.pop(key, None)
-            cur = None
-            while len(self._ws) >= self.KEPT:
-                self._ws.popitem(last=False)
-            size = max(int(nbytes), 1 << 16)
+            self._kept.pop(key, None)
+            while len(self._kept) >= self.KEPT:
+                del self._kept[min(self._kept, key=lambda k: self._kept[k].used)]
             try:
-                ws = self._scratch(size)
+                ws = self._bytes(nbytes)
             except torch.cuda.OutOfMemoryError:
-                self._ws.clear()   # what other streams and threads keep for their next call
-                ws = self._scratch(size)
+                self._kept.clear()   # what other streams and threads keep for their next call
+                ws = self._bytes(nbytes)
             assert ws.data_ptr() % 256 == 0
-            self._ws[key] = (ws, ws[:4].view(torch.int32))
-            return ws
+            if key not in self._sticky:
+                if len(self._sticky) >= self.STICKY:
+                    self._collect()
+                self._sticky[key] = torch.zeros(1, dtype=torch.int32, device=self.device)
+            own = self._kept[key] = Scratch(ws, self._sticky[key])
+            return own
+
+    def workspace(self, nbytes: int) -> torch.Tensor:
+        """The workspace of a call on the current stream."""
+        return self.scratch(nbytes, torch.cuda.current_device(), self.stream_handle()).ws
 
     def release_workspace(self) -> None:
         with self._lock:
-            self._ws.clear()
+            self._kept.clear()
 
     # --- device-side status of the sorts enqueued so far ------------------------------------
-    def note_sort(self, ws: torch.Tensor) -> None:
+    def note_sort(self, own: Scratch) -> None:
         """Folds the status word at the head of a workspace (0, or the code a kernel left when a
-        bounded wait ran out) into a word per stream that survives the workspace's reuse.  Stream
+        bounded wait ran out) into a word that survives the workspace's reuse.  Stream
         ordered, no synchronisation."""
-        dev, stream = torch.cuda.current_device(), self.stream_handle()
-        with self._lock:
-            acc = self._sticky.get((dev, stream))
-            if acc is None:
-                if len(self._sticky) >= self.STICKY:
-                    self._collect()
-                acc = self._sticky[(dev, stream)] = torch.zeros(1, dtype=torch.int32, device=self.device)
-            own = self._ws.get((dev, stream, threading.get_ident()))
-        torch.maximum(acc, own[1] if own is not None and own[0] is ws else ws[:4].view(torch.int32), out=acc)
+        torch.maximum(own.failed, own.status, out=own.failed)
 
     def _collect(self) -> None:
-        """Reads the status words of all streams and lets go of them."""
-        for (dev, _), acc in self._sticky.items():
-            torch.cuda.synchronize(dev)
-            self._failed[dev] = max(self._failed.get(dev, 0), int(acc.item()))
-        self._sticky.clear()
+        """Reads the status words whose workspaces are gone and lets go of them."""
+        for key in [k for k in self._sticky if k not in self._kept]:
+            torch.cuda.synchronize(key[0])
+            self._failed[key[0]] = max(self._failed.get(key[0], 0), int(self._sticky.pop(key).item()))
 
     def raise_pending(self) -> None:
         """Called where a result reaches the host: raises if any sort of this device since the last call reported
@@ -115,12 +126,12 @@ class Runtime:
             return
         dev = torch.cuda.current_device()
         with self._lock:
-            words = [acc for (d, _), acc in self._sticky.items() if d == dev]
+            words = [word for key, word in self._sticky.items() if key[0] == dev]
             status = self._failed.pop(dev, 0)
-        for acc in words:
-            own = int(acc.item())
+        for word in words:
+            own = int(word.item())
             if own != 0:
-                acc.zero_()
+                word.zero_()
             status = max(status, own)
         if status != 0:
             raise _lib.B2SError(status, "a sort kernel")

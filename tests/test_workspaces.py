@@ -27,8 +27,8 @@ class Fake(Runtime):
     def stream_handle(self):
         return self.stream
 
-    def _scratch(self, nbytes):
-        if self.full_at is not None and sum(w.numel() for w, _ in self._ws.values()) + nbytes > self.full_at:
+    def _bytes(self, nbytes):
+        if self.full_at is not None and sum(s.nbytes for s in self._kept.values()) + nbytes > self.full_at:
             raise torch.cuda.OutOfMemoryError("no room")
         raw = torch.zeros(nbytes + 256, dtype=torch.uint8)
         at = -raw.data_ptr() % 256
@@ -67,15 +67,15 @@ def test_what_is_kept_is_bounded_and_given_back(run):
     ws = {}
     for run.stream in range(Runtime.KEPT + 3):
         ws[run.stream] = run.workspace(1000)
-    assert len(run._ws) == Runtime.KEPT
+    assert len(run._kept) == Runtime.KEPT
     run.stream = 0
     assert run.workspace(1000) is not ws[0]        # (it went first)
     run.stream = Runtime.KEPT + 2
     assert run.workspace(1000) is ws[run.stream]
     run.full_at = 1 << 20
-    assert run.workspace(1 << 20).numel() == 1 << 20 and len(run._ws) == 1   # room is made of what the others keep
+    assert run.workspace(1 << 20).numel() == 1 << 20 and len(run._kept) == 1   # room is made of what the others keep
     run.release_workspace()
-    assert not run._ws
+    assert not run._kept
     with pytest.raises(torch.cuda.OutOfMemoryError):
         run.workspace((1 << 20) + 1)
 
@@ -83,9 +83,9 @@ def test_what_is_kept_is_bounded_and_given_back(run):
 @pytest.mark.parametrize("streams", [2, 66])
 def test_a_failure_on_any_stream_is_raised_once(run, streams):
     for run.stream in range(streams):
-        ws = run.workspace(1000)
-        ws[:4].view(torch.int32).fill_(5 if run.stream == 1 else 0)
-        run.note_sort(ws)
+        own = run.scratch(1000, run.dev, run.stream)
+        own.status.fill_(5 if run.stream == 1 else 0)
+        run.note_sort(own)
     assert len(run._sticky) <= Runtime.STICKY < 66
     with pytest.raises(_lib.B2SError):
         run.raise_pending()
