@@ -82,48 +82,41 @@ __device__ __forceinline__ typename KeyOf<KB>::type split_image(typename KeyOf<K
 }
 
 // Zeros of both signs have one image, and so have all NaNs.  Where a sort holds one pattern of each, that is what its result gets;
-// of several it would have to keep the input order, which the radix passes do.  The patterns of a warp's threads:
-template <int KB> struct MarksSeen {
-  using K        = typename KeyOf<KB>::type;
-  K nan          = 0;
-  unsigned int zeros = 0;
-  bool mixed     = false;
-  __device__ __forceinline__ void see(K raw, K image)
-  {
-    if (image == (K)~(K)0) {
-      mixed |= nan != 0 && nan != raw;
-      nan = raw;
-    } else if (image == (K)((K)1 << (8 * KB - 1))) {
-      zeros |= raw == 0 ? 1u : 2u;
-    }
-  }
-  // into `to` (of the block, or of the sort); by whole warps
-  __device__ __forceinline__ void into(SplitMarks* to)
-  {
-    const unsigned int with = __ballot_sync(0xFFFFFFFFu, nan != 0);
-    zeros                   = __reduce_or_sync(0xFFFFFFFFu, zeros);
-    const unsigned int from = with ? __ffs(with) - 1 : 0;
-    const K first           = __shfl_sync(0xFFFFFFFFu, nan, from);
-    mixed |= nan != 0 && nan != first;
-    mixed = __any_sync(0xFFFFFFFFu, mixed);
-    if ((threadIdx.x & 31) == from) {
-      if (with) {
-        const unsigned long long old = atomicCAS(&to->nan, 0ull, (unsigned long long)first);
-        mixed |= old != 0 && old != (unsigned long long)first;
-      }
-      if (zeros) zeros |= atomicOr(&to->zeros, zeros);
-      mixed |= zeros == 3;
-    }
-  }
-};
+// of several it would have to keep the input order, which the radix passes do.  Key j of a thread: the usual patterns
+// into `flags`, others into `odd`, to be looked at by mark().
 template <int KB>
-__device__ __forceinline__ typename KeyOf<KB>::type split_raw(typename KeyOf<KB>::type o, typename KeyOf<KB>::type nan, typename KeyOf<KB>::type zero)
+__device__ __forceinline__ void mark_usual(typename KeyOf<KB>::type raw, typename KeyOf<KB>::type image, unsigned int& flags, unsigned int& odd, int j)
+{
+  using K = typename KeyOf<KB>::type;
+  if (image == (K)~(K)0 || image == (K)((K)1 << (8 * KB - 1))) {
+    if (sm_is_special<KB>(raw, XF_FLOAT)) odd |= 1u << j;
+    else flags |= image == (K)~(K)0 ? MARK_NAN : MARK_ZERO;
+  }
+}
+// `block` lies in shared memory.
+template <int KB>
+__device__ __forceinline__ void mark(typename KeyOf<KB>::type raw, typename KeyOf<KB>::type image, unsigned int& flags, SplitMarks* block)
+{
+  if (image != (typename KeyOf<KB>::type)~(typename KeyOf<KB>::type)0) {
+    flags |= MARK_NEG_ZERO;
+  } else if (*reinterpret_cast<volatile unsigned long long*>(&block->nan) != (unsigned long long)raw) {
+    const unsigned long long old = atomicCAS(&block->nan, 0ull, (unsigned long long)raw);
+    if (old != 0 && old != (unsigned long long)raw) flags |= MARK_MIXED;
+  }
+}
+__device__ __forceinline__ bool marks_mixed(unsigned long long nan, unsigned int flags)
+{
+  return (flags & MARK_MIXED) != 0 || (flags & (MARK_ZERO | MARK_NEG_ZERO)) == (MARK_ZERO | MARK_NEG_ZERO) || ((flags & MARK_NAN) != 0 && nan != 0);
+}
+// A key from its image.
+template <int KB>
+__device__ __forceinline__ typename KeyOf<KB>::type marked_raw(typename KeyOf<KB>::type o, const SplitMarks* m)
 {
   using K        = typename KeyOf<KB>::type;
   constexpr K SB = (K)((K)1 << (8 * KB - 1));
-  if (o == (K)~(K)0) return nan;
-  if (o == SB) return zero;
-  return (o & SB) ? (K)(o ^ SB) : (K)~o;
+  if (o == (K)~(K)0 && m->nan != 0) return (K)m->nan;
+  if (o == SB && (m->flags & MARK_NEG_ZERO) != 0) return SB;
+  return sm_from_ordered<KB>(o, XF_FLOAT);
 }
 
 template <int KB> struct FloatOf { using type = float; };
@@ -226,25 +219,28 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
   constexpr unsigned int FIN_LO = KB == 8 ? 0x00100000u : 0x00800000u;  // upper words of finite images start here
   K img[PER];
   unsigned int at[PER];
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const unsigned int i = j * SPLIT_THREADS + tid;
-    // one key of every stretch of len / SAMPLES, at a scattered place inside it
+  // one key of every stretch of len / SAMPLES, at a scattered place inside it
+  auto place = [&](unsigned int i) {
     unsigned int h = i * 2654435761u;
     h ^= h >> 15;
     h *= 2246822519u;
-    at[j]  = len <= SAMPLES ? i : (unsigned int)(((unsigned long long)i * len) / SAMPLES) + __umulhi(h, len / SAMPLES);
+    return len <= SAMPLES ? i : (unsigned int)(((unsigned long long)i * len) / SAMPLES) + __umulhi(h, len / SAMPLES);
+  };
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const unsigned int i = j * SPLIT_THREADS + tid;
+    at[j]  = place(i);
     img[j] = i < ns ? src[at[j]] : (K)0;
     if (PAIRS && L.src_pos != nullptr) at[j] = i < ns ? L.src_pos[begin + at[j]] : 0u;
   }
   auto mine = [&](int j) { return j * SPLIT_THREADS + tid < ns; };
   K lo = (K)~(K)0, hi = 0;
-  MarksSeen<KB> seen;
+  unsigned int flags = 0, odd = 0;
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
     const K raw = img[j];
     img[j] = split_image<KB, FORM>(img[j], flip);
-    if (FORM == FORM_FLOAT && !PAIRS && mine(j)) seen.see(raw, img[j]);
+    if (FORM == FORM_FLOAT && !PAIRS && mine(j)) mark_usual<KB>(raw, img[j], flags, odd, j);
     // (of floats the finite ones count)
     if (mine(j) && !(FORM != FORM_INT && (unsigned int)(img[j] >> (8 * KB - 32)) - FIN_LO >= 0u - 2u * FIN_LO)) {
       lo = img[j] < lo ? img[j] : lo;
@@ -263,9 +259,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
   }
   if (tid < 2) sh_n[tid] = sh_most[tid] = sh_eq[tid] = 0;
   if (tid == 0) {
-    sh_lo    = ~0ull;
-    sh_hi    = 0;
-    sh_marks = SplitMarks{};
+    sh_lo = ~0ull;
+    sh_hi = 0;
   }
   for (unsigned int i = tid; i < L.cells; i += SPLIT_THREADS) sh_cells[i] = 0;
   __syncthreads();
@@ -420,10 +415,20 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
     __syncthreads();
     unsigned int* table = sh_cells;
     for (unsigned int i = tid; i < SPLIT_PRINTS; i += SPLIT_THREADS) table[i] = 0;
-    if (tid == 0) sh_n[0] = sh_n[1] = 0;
+    if (tid == 0) {
+      sh_n[0] = sh_n[1] = 0;
+      sh_marks = SplitMarks{};
+    }
     __syncthreads();
-    if (FORM == FORM_FLOAT && !PAIRS) seen.into(&sh_marks);
-    const bool mixed = __syncthreads_or(seen.mixed);
+    if (FORM == FORM_FLOAT && !PAIRS) {
+      while (odd) {
+        const K raw = src[place((__ffs(odd) - 1) * SPLIT_THREADS + tid)];
+        odd &= odd - 1;
+        mark<KB>(raw, split_image<KB, FORM>(raw, flip), flags, &sh_marks);
+      }
+      flags = __reduce_or_sync(0xFFFFFFFFu, flags);
+      if (lane == 0 && flags) atomicOr(&sh_marks.flags, flags);
+    }
     unsigned int same = 0, bytes = 0;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
     }
     __syncthreads();
     if (tid == 0) {
-      unsigned int route = mixed ? ROUTE_RADIX : ROUTE_SPLIT;
+      unsigned int route = FORM == FORM_FLOAT && !PAIRS && marks_mixed(sh_marks.nan, sh_marks.flags) ? ROUTE_RADIX : ROUTE_SPLIT;
       // (a sample finds its copies among those before it: half of the square)
       const unsigned long long copies = (unsigned long long)sh_n[0] * 2 * len / ((unsigned long long)ns * ns);
       // (of an argsort equal keys have to be taken apart; in a sort of floats, whose cells cannot be seen to hold one value, they
@@ -487,7 +492,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
   const unsigned int ci = L.cells - 2 - split_nan_cells(FORM, PAIRS, L.cells);
   unsigned int cur = 0xFFFFFFFFu;
   SplitSeg s{};
-  MarksSeen<KB> seen;
+  unsigned int flags = 0;
   auto flush = [&] {
     __syncthreads();
     unsigned int* out = L.hist + (size_t)cur * L.cells;
@@ -515,7 +520,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
     auto count = [&](auto md, auto part) {
       constexpr unsigned int MODE = decltype(md)::value;
       constexpr bool PART         = decltype(part)::value;
-      unsigned int nans           = 0;
+      unsigned int nans = 0, odd = 0;
 #pragma unroll
       for (int j = 0; j < ITEMS; ++j) {
         const unsigned int e = j * SPLIT_THREADS + tid;
@@ -526,13 +531,21 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
         const unsigned int e = j * SPLIT_THREADS + tid;
         if (PART && e >= valid) continue;
         const K x = split_image<KB, FORM>(key[j], flip);
-        if (FORM == FORM_FLOAT && !PAIRS) seen.see(key[j], x);
+        if (FORM == FORM_FLOAT && !PAIRS) mark_usual<KB>(key[j], x, flags, odd, j);
         if (PAIRS && MODE != MAP_POS && FORM != FORM_INT && x == (K)~(K)0) {
           nans |= 1u << j;   // ordered by position, which is fetched for them alone
           continue;
         }
         const unsigned int pos = !PAIRS || MODE != MAP_POS ? 0u : psrc == nullptr ? at + e : psrc[e];
         atomicAdd(&h[cell_of<KB, FORM, PAIRS, MODE>(x, pos, s.map, ci)], 1u);
+      }
+      if (FORM == FORM_FLOAT && !PAIRS) {
+        while (odd) {   // negative zeros and other NaNs, fetched once more: kept until here they would spill
+          const int j = __ffs(odd) - 1;
+          odd &= odd - 1;
+          const K raw = src[j * SPLIT_THREADS + tid];
+          mark<KB>(raw, split_image<KB, FORM>(raw, flip), flags, &sh_marks);
+        }
       }
       if (PAIRS && FORM != FORM_INT) {
         while (nans) {
@@ -550,17 +563,17 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
   }
   flush();
   if (FORM == FORM_FLOAT && !PAIRS) {
-    // the warps' patterns to the block's, and those to the sort's
-    seen.into(&sh_marks);
-    bool mixed = __syncthreads_or(seen.mixed);
-    if (tid < 32 && (sh_marks.nan != 0 || sh_marks.zeros != 0)) {
-      seen.nan   = (K)sh_marks.nan;
-      seen.zeros = sh_marks.zeros;
-      seen.mixed = false;
-      seen.into(L.marks);
-      mixed |= seen.mixed;
+    flags = __reduce_or_sync(0xFFFFFFFFu, flags);
+    if ((tid & 31) == 0 && flags) atomicOr(&sh_marks.flags, flags);
+    __syncthreads();
+    if (tid == 0) {
+      flags = sh_marks.flags;
+      if (sh_marks.nan != 0) {
+        const unsigned long long old = atomicCAS(&L.marks->nan, 0ull, sh_marks.nan);
+        if (old != 0 && old != sh_marks.nan) flags |= MARK_MIXED;
+      }
+      if (flags & ~ld_relaxed(&L.marks->flags)) atomicOr(&L.marks->flags, flags);
     }
-    if (mixed && tid < 32) atomicMax(&ctrl->route, (unsigned int)ROUTE_LATE);
   }
 }
 
@@ -648,6 +661,10 @@ split_pack_kernel(Ctrl* ctrl, SplitLevel L, SplitLeaf* leaves, SplitSeg* next_se
   const unsigned int seg = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   chain_wait();
   if (__syncthreads_or(ld_relaxed(&ctrl->route) != ROUTE_SPLIT)) return;  // (other blocks may be changing it)
+  if (FORM == FORM_FLOAT && !PAIRS && marks_mixed(L.marks->nan, L.marks->flags)) {
+    if (tid == 0) atomicMax(&ctrl->route, (unsigned int)ROUTE_LATE);
+    return;
+  }
   if (L.tile_seg != nullptr && seg >= ctrl->split_nseg) return;
   const SplitSeg s = L.segs[seg];
   if (s.len == 0) return;
@@ -760,7 +777,7 @@ split_pack_kernel(Ctrl* ctrl, SplitLevel L, SplitLeaf* leaves, SplitSeg* next_se
         const unsigned int len = pre[c + 1] - pre[c], begin = s.begin + pre[c];
         unsigned long long raw;
         if constexpr (FORM != FORM_INT)
-          raw = (unsigned long long)split_raw<KB>((K)image, (K)L.marks->nan, (L.marks->zeros & 2u) ? (K)((K)1 << (8 * KB - 1)) : (K)0);
+          raw = (unsigned long long)marked_raw<KB>((K)image, L.marks);
         else raw = (unsigned long long)(K)((K)image ^ flip);
         const unsigned int parts = (len + FILL_CHUNK - 1) / FILL_CHUNK, e = atomicAdd(&ctrl->split_nleaf, parts);
         for (unsigned int i = 0; i < parts; ++i)
@@ -1268,9 +1285,8 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
   if (ctrl->route != ROUTE_SPLIT) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned int nleaf = ctrl->split_nleaf;
-  // the patterns of NaNs and zeros
-  const K nan  = FORM != FORM_INT && !PAIRS ? (K)A.marks->nan : (K)0;
-  const K zero = FORM != FORM_INT && !PAIRS && (A.marks->zeros & 2u) ? (K)((K)1 << (8 * KB - 1)) : (K)0;
+  // (other patterns than the usual ones of NaNs and zeros: a loop of its own, so that the usual one costs no more for it)
+  const bool marked = FORM != FORM_INT && !PAIRS && (A.marks->nan != 0 || (A.marks->flags & MARK_NEG_ZERO) != 0);
   for (unsigned int l = blockIdx.x; l < nleaf; l += gridDim.x) {
     const SplitLeaf leaf = A.leaves[l];
     if (leaf.len & LEAF_FILL) {
@@ -1312,7 +1328,7 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
           if (count[mid] > i) b = mid; else a = mid + 1;
         }
         const K o = (K)((K)leaf.lo + a);
-        if constexpr (FORM != FORM_INT) to[i] = split_raw<KB>(o, nan, zero);
+        if constexpr (FORM != FORM_INT) to[i] = marked_raw<KB>(o, A.marks);
         else to[i] = (K)(o ^ flip);
       }
       __syncthreads();
@@ -1446,10 +1462,14 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
       }
       if (!narrow) {
         leaf_order<W, false, THREADS>(img, none, bk, exact && FORM == FORM_INT, sw, sp, cnt, wsum);
-        for (unsigned int e = tid; e < n; e += THREADS) {
-          const K o = (K)sw[smpad(e)];
-          if constexpr (FORM != FORM_INT) dst[e] = split_raw<KB>(o, nan, zero);
-          else dst[e] = (K)(o ^ flip);
+        if (FORM != FORM_INT && marked) {
+          for (unsigned int e = tid; e < n; e += THREADS) dst[e] = marked_raw<KB>((K)sw[smpad(e)], A.marks);
+        } else {
+          for (unsigned int e = tid; e < n; e += THREADS) {
+            const K o = (K)sw[smpad(e)];
+            if constexpr (FORM != FORM_INT) dst[e] = sm_from_ordered<KB>(o, XF_FLOAT);
+            else dst[e] = (K)(o ^ flip);
+          }
         }
       }
     }

@@ -44,10 +44,11 @@ struct SplitLeaf {
   unsigned long long lo, span;
 };
 
-// What the float keys of a sort without positions hold, of the two images that stand for several bit patterns each.
+// Bit patterns among the float keys of a sort without positions whose image stands for several.
+enum : unsigned int { MARK_ZERO = 1, MARK_NEG_ZERO = 2, MARK_NAN = 4 /* the canonical one */, MARK_MIXED = 8 /* several others */ };
 struct SplitMarks {
-  unsigned long long nan;  // the NaNs' pattern; 0: none seen
-  unsigned int zeros;      // 1: zeros seen, 2: negative zeros
+  unsigned long long nan;  // NaNs of another pattern; 0: none
+  unsigned int flags;
 };
 
 // Shape of one split.
