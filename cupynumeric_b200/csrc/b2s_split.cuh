@@ -38,7 +38,10 @@ constexpr unsigned short LUT_DROP = 0xFFFF;
 constexpr int SPLIT_THREADS       = 512;
 constexpr int SPLIT_SAMPLES       = 4096;  // of a segment of the input
 constexpr int SPLIT_SAMPLES_NEXT  = 2048;  // of a bucket of the first split
-constexpr unsigned int SPLIT_PRINTS = 8192;
+// Places for the samples' fingerprints by how often the samples are drawn: of keys of an argsort, whose copies decide (below),
+// more samples from 8 * 10^6 keys on, where 16 copies of each value are too few pairs among 4096.
+inline unsigned int split_rounds(unsigned int len, unsigned int nseg, bool pairs) { return !pairs || nseg != 1 || len <= 8000000u ? 1 : len <= 32000000u ? 2 : 4; }
+__host__ __device__ constexpr unsigned int split_prints(unsigned int rounds) { return rounds == 1 ? 8192 : 32768; }
 
 template <int KB, bool PAIRS> struct SplitCfg {
   // (two blocks per SM, each with its tile, the counters and the table of up to 8192 cells)
@@ -60,6 +63,8 @@ struct SplitLevel {
   unsigned int last;          // buckets are leaves (else segments of the next level)
   unsigned int pos_n;         // positions lie below this
   unsigned int radix_if;      // bit k: keys that differ in k bytes are left to the radix passes
+  unsigned int rounds;        // of samples
+  unsigned int most_copies;   // of a key, above which the radix passes are faster
   SplitMarks* marks;
   const void* src_keys;
   const uint32_t* src_pos;    // null: the place inside the segment
@@ -413,8 +418,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
     // Who sorts.  Copies of a key among the samples, by a table of fingerprints (NaNs apart), as if every value
     // had as many
     __syncthreads();
-    unsigned int* table = sh_cells;
-    for (unsigned int i = tid; i < SPLIT_PRINTS; i += SPLIT_THREADS) table[i] = 0;
+    unsigned int* table       = sh_cells;
+    const unsigned int prints = split_prints(L.rounds);
+    for (unsigned int i = tid; i < prints; i += SPLIT_THREADS) table[i] = 0;
     if (tid == 0) {
       sh_n[0] = sh_n[1] = 0;
       sh_marks = SplitMarks{};
@@ -430,19 +436,39 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
       if (lane == 0 && flags) atomicOr(&sh_marks.flags, flags);
     }
     unsigned int same = 0, bytes = 0;
+    auto print = [&](K image) {
+      if (FORM != FORM_INT && image == (K)~(K)0) return;
+      unsigned int h = (unsigned int)image * 2654435761u ^ (unsigned int)((unsigned long long)image >> 32) * 2246822519u;
+      h ^= h >> 15;
+      h = h * 3266489917u | 1u;
+      const unsigned int old = atomicCAS(&table[__umulhi(h, prints)], 0u, h);
+      same += old == h ? 1u : 0u;
+    };
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       if (mine(j)) {
         const unsigned long long d = (unsigned long long)(img[j] ^ lo_seen);
 #pragma unroll
         for (int k = 0; k < KB; ++k) bytes |= (d >> (8 * k) & 0xFFu) ? 1u << k : 0u;
-        if ((PAIRS || FORM != FORM_INT) && !(FORM != FORM_INT && img[j] == (K)~(K)0)) {
-          unsigned int h = (unsigned int)img[j] * 2654435761u ^ (unsigned int)((unsigned long long)img[j] >> 32) * 2246822519u;
-          h ^= h >> 15;
-          h = h * 3266489917u | 1u;
-          const unsigned int old = atomicCAS(&table[h >> 19], 0u, h);
-          same += old == h ? 1u : 0u;
+        if (PAIRS || FORM != FORM_INT) print(img[j]);
+      }
+    }
+    if (PAIRS) {
+      // one more key of every stretch per round, from parts of it that do not meet
+      for (unsigned int r = 1; r < L.rounds; ++r) {
+        const unsigned int part = len / SAMPLES / (L.rounds - 1);
+        K more[PER];
+        bool other[PER];
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+          const unsigned int i = j * SPLIT_THREADS + tid;
+          const unsigned int p = (unsigned int)(((unsigned long long)i * len) / SAMPLES) + (r - 1) * part + __umulhi((i + r) * 2654435761u, part);
+          other[j]             = p != place(i);
+          more[j]              = src[p];
         }
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+          if (other[j]) print(split_image<KB, FORM>(more[j], flip));
       }
     }
     same  = __reduce_add_sync(0xFFFFFFFFu, same);
@@ -454,11 +480,14 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
     __syncthreads();
     if (tid == 0) {
       unsigned int route = FORM == FORM_FLOAT && !PAIRS && marks_mixed(sh_marks.nan, sh_marks.flags) ? ROUTE_RADIX : ROUTE_SPLIT;
-      // (a sample finds its copies among those before it: half of the square)
-      const unsigned long long copies = (unsigned long long)sh_n[0] * 2 * len / ((unsigned long long)ns * ns);
+      // A sample finds its copies among those before it: half of the square, as long as few have any; then what counts is how many
+      // others there are.
+      const unsigned int drawn    = ns * L.rounds, eq = sh_n[0];
+      unsigned long long copies   = (unsigned long long)eq * 2 * len / ((unsigned long long)drawn * drawn);
+      if (2 * eq > drawn) copies  = max(copies, (unsigned long long)(len / max(drawn - eq, 1u)));
       // (of an argsort equal keys have to be taken apart; in a sort of floats, whose cells cannot be seen to hold one value, they
       // fill cells that nothing splits)
-      if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && sh_n[0] >= 16 && copies > 512) route = ROUTE_RADIX;
+      if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && eq >= 6 && copies > L.most_copies) route = ROUTE_RADIX;
       if (PAIRS) {
         // a cell that holds more than the next split takes apart could not be handled later
         const unsigned long long est = (unsigned long long)(most >> 16) * len / ns;
@@ -1491,6 +1520,22 @@ inline cudaError_t split_smem(Kern kern, size_t smem)
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
+// Copies of each key above which the passes are faster: the positions of equal keys are put in order by the networks and the merging of
+// leaf_order.  Time of the splits in parts of the passes' for argsorts of n / c evenly used values:
+//   float32, 6 * 10^6 (two splits)   c = 8 0.90, 20 1.25, 100 1.50, 400 1.68;  2 * 10^7  0.89, 1.30, 1.75, 1.97
+//   float32, 7 * 10^5 (one split)    c = 20 0.90, 100 0.93, 150 1.02, 400 1.06
+//   float64, 2.5 * 10^5              c = 8 0.79, 20 1.04, 100 1.21;  8 * 10^6  c = 8 0.63, 20 0.92, 40 1.07, 250 1.43
+//   int64, 2.4 * 10^7                c = 8 0.66, 20 0.93, 40 1.19, 400 1.46
+//   float32, 300 rows of 16400       c = 8 0.85, 20 1.16, 40 1.34 (int32 0.81, 1.10, 1.30);  sent back 1.15
+//   float64, rows                    30000 of 300 copies 1.09, 100003 of 1000 0.95; sent back 1.06 to 1.12
+// Sorts have no positions to be put in order, but of floats values that fill cells.
+inline unsigned int split_most_copies(int kb, bool pairs, unsigned int nseg, const SplitPlan& plan)
+{
+  if (!pairs) return plan.lev[plan.levels - 1].cap / 2;
+  if (kb == 8) return nseg != 1 ? 2048 : 24;
+  return nseg != 1 ? 24 : plan.levels == 1 ? 128 : 12;
+}
+
 template <int KB, int FORM0, bool PAIRS>
 inline cudaError_t split_form(typename KeyOf<KB>::type flip, const SplitPlan& plan, const SplitJob& job, Ctrl* ctrl, cudaStream_t stream)
 {
@@ -1518,6 +1563,8 @@ inline cudaError_t split_form(typename KeyOf<KB>::type flip, const SplitPlan& pl
     L.last          = l == plan.levels - 1;
     L.pos_n         = job.seg_len;
     L.radix_if      = plan.radix_if;
+    L.rounds        = l == 0 ? split_rounds(job.seg_len, job.nseg, PAIRS) : 1;
+    L.most_copies   = split_most_copies(KB, PAIRS, job.nseg, plan);
     L.marks         = reinterpret_cast<SplitMarks*>(job.tables + plan.off_marks);
     L.src_keys      = l == 0 ? job.in : job.tmp_keys[0];
     L.src_pos       = PAIRS && l > 0 ? job.tmp_pos[0] : nullptr;
@@ -1527,7 +1574,8 @@ inline cudaError_t split_form(typename KeyOf<KB>::type flip, const SplitPlan& pl
     {
       prof::Scope ps(prof::K_HIST, stream);
       auto sample = l == 0 ? split_sample_kernel<KB, FORM0, PAIRS, SPLIT_SAMPLES> : split_sample_kernel<KB, FORM1, PAIRS, SPLIT_SAMPLES_NEXT>;
-      const size_t smem = (size_t)(sh.cells > SPLIT_PRINTS ? sh.cells : SPLIT_PRINTS) * 4;
+      const unsigned int prints = split_prints(L.rounds);
+      const size_t smem         = (size_t)(sh.cells > prints ? sh.cells : prints) * 4;
       e = split_smem(sample, smem);
       if (e != cudaSuccess) return e;
       e = launch_chained(sample, sh.nseg, SPLIT_THREADS, smem, stream, ctrl, L, l > 0 ? 0u : job.nseg == 1 ? 2u : 1u, flip);

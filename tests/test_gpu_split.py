@@ -157,6 +157,19 @@ def test_sent_back_with_the_sample(dtype, op, n):
     assert _check(a, op) == RADIX
 
 
+@pytest.mark.parametrize("dtype,rows,n,copies", [("float64", 1, 250_007, 60), ("float32", 1, 700_001, 400), ("float32", 1, 5_000_011, 60),
+                                                 ("int64", 1, 24_000_017, 60), ("float32", 1, 32_000_003, 40), ("float32", 60, 20_011, 80)])
+def test_copies_send_argsorts_back(dtype, rows, n, copies):
+    """Evenly used values: two copies of each stay with the splits, many go back with the sample, which draws more keys of long arrays."""
+    rng = np.random.default_rng(n)
+    for c in (2, copies):
+        if c == 2 and n > 5_000_011:
+            continue   # (test_as_it_is_dispatched)
+        names = rng.standard_normal((rows, n // c)) * (2.0**40 if dtype == "int64" else 1.0)
+        a = np.take_along_axis(names, rng.integers(0, n // c, (rows, n)), axis=1).astype(dtype)
+        assert _check(a if rows > 1 else a[0], "argsort") == (SPLIT if c == 2 else RADIX)
+
+
 @pytest.mark.parametrize("dtype,rows,n", [("float64", 1, 250_007), ("float32", 1, 5_000_011), ("float64", 37, 20_011), ("float32", 60, 20_011)])
 def test_patterns_of_zeros_and_nans(dtype, rows, n):
     """A sort keeps the one pattern that its zeros have, and its NaNs; where there are several the passes take it, at once if
