@@ -317,8 +317,11 @@ inline cudaError_t radix_seg_xf(const void* in, void* out, int64_t* idx_out, uns
   e = cudaMemsetAsync(ws + lay.off_seghist, 0, lay.off_keys[0] - lay.off_seghist, stream);
   if (e != cudaSuccess) return e;
   if constexpr ((KB == 4 || KB == 8) && XF != XF_CFLOAT) {
-    // (float32 sort of 7 rows of 90000 66 -> 73 us, of 10 rows of 10^6 271 -> 177)
-    const bool enough = KB == 8 || pairs || (size_t)seg_len * nseg >= 1000000 || split_override() > 0;
+    // 8-byte keys and argsorts gain at every length (time in parts of the passes': int64 and float64 sorts 0.65 for 3 rows of 8200,
+    // 0.37 to 0.5 for 1000 rows; argsorts of float32 0.7 for 3 rows of 20011, 0.6 for 1000 of 16400).  4-byte sorts need 10^6 keys
+    // (float32, 7 rows of 90000 66 -> 73 us, 10 rows of 10^6 271 -> 177), and rows of two leaves do not gain enough for what
+    // crowded ones lose (1000 rows of 8200, full range 0.91, 40 copies of each key 1.28, Zipf 1.61; of 12000 0.71, Zipf 1.19).
+    const bool enough = KB == 8 || pairs || ((size_t)seg_len * nseg >= 1000000 && seg_len >= 10000) || split_override() > 0;
     if (!(pairs && out != nullptr) && split_override() != 0 && enough) {
       const SplitPlan plan = split_plan(seg_len, nseg, pairs, lay.off_seghist - lay.off_lookback);
       if (plan.ok) {

@@ -157,6 +157,14 @@ def test_sent_back_with_the_sample(dtype, op, n):
     assert _check(a, op) == RADIX
 
 
+@pytest.mark.parametrize("dtype", ["int32", "float32", "int64"])
+def test_rows_of_two_leaves(dtype):
+    """Sorts of 4-byte keys in rows below 10000 keep the passes, others do not."""
+    for n in (9_999, 10_000):
+        tried = _check(_values("normal", n * 200, np.dtype(dtype), 2).reshape(200, n), "sort")
+        assert tried == (OPEN if n < 10_000 and dtype != "int64" else SPLIT)
+
+
 @pytest.mark.parametrize("dtype,rows,n,copies", [("float64", 1, 250_007, 60), ("float32", 1, 700_001, 400), ("float32", 1, 5_000_011, 60),
                                                  ("int64", 1, 24_000_017, 60), ("float32", 1, 32_000_003, 40), ("float32", 60, 20_011, 80)])
 def test_copies_send_argsorts_back(dtype, rows, n, copies):
