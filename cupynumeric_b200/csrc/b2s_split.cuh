@@ -65,6 +65,7 @@ struct SplitLevel {
   unsigned int radix_if;      // bit k: keys that differ in k bytes are left to the radix passes
   unsigned int rounds;        // of samples
   unsigned int most_copies;   // of a key, above which the radix passes are faster
+  unsigned int leaf_cap;      // `cap` of the last split
   SplitMarks* marks;
   const void* src_keys;
   const uint32_t* src_pos;    // null: the place inside the segment
@@ -180,6 +181,74 @@ __device__ __forceinline__ void with_mode(unsigned int mode, F f)
   else f(std::integral_constant<unsigned int, PAIRS ? MAP_POS : MAP_TOP>{});
 }
 
+// MAP_LOG: where, from m.lo on, cell q + 1 starts (2^64 - 1 also for what lies beyond).
+__device__ __forceinline__ unsigned long long log_from(const SplitMap& m, unsigned int q)
+{
+  return q == 0 ? 0ull : __float2ull_ru(__uint_as_float((q + m.mult) << m.shift));
+}
+
+// The last image of that cell.
+__device__ __forceinline__ unsigned long long log_last(const SplitMap& m, unsigned int q)
+{
+  const unsigned long long next = log_from(m, q + 1);
+  return next == ~0ull ? next : next - 1;
+}
+
+// The only image of a cell, where it has one.
+template <int KB, int FORM, bool PAIRS>
+__device__ __forceinline__ bool cell_value(const SplitMap& m, unsigned int c, unsigned int ci, unsigned long long* image)
+{
+  if (FORM != FORM_INT && !PAIRS && c == ci + 2) {
+    *image = KB == 8 ? ~0ull : 0xFFFFFFFFull;
+    return true;
+  }
+  if (c < 1 || c > ci) return false;
+  if (m.mode == MAP_LIN && m.shift == 0) {
+    *image = m.lo + (c - 1);
+    return true;
+  }
+  if (m.mode == MAP_TOP && c == (unsigned int)(m.top >> m.shift) + 2) {
+    *image = m.lo + m.top;
+    return true;
+  }
+  if (m.mode == MAP_LOG) {
+    const unsigned long long z = log_from(m, c - 1);
+    if (log_last(m, c - 1) != z) return false;
+    *image = m.lo + z;
+    return true;
+  }
+  return false;
+}
+
+// The images that cells c0 .. c1 - 1 can hold, where the mapping tells.
+__device__ __forceinline__ bool cell_bounds(const SplitMap& m, unsigned int c0, unsigned int c1, unsigned int ci, unsigned long long* lo, unsigned long long* span)
+{
+  if (c0 < 1 || c1 - 1 > ci) return false;
+  unsigned long long a, b;  // first and last image, from m.lo on
+  // (cells of a mapping may reach beyond the range, and beyond 64 bits)
+  auto step = [&](unsigned int c) { return c > (m.range >> m.shift) ? m.range : ((unsigned long long)c << m.shift) - 1; };   // the last of c linear cells
+  if (m.mode == MAP_LIN) {
+    a = (unsigned long long)(c0 - 1) << m.shift;
+    b = step(c1 - 1);
+  } else if (m.mode == MAP_TOP) {
+    // (cells from the one of lo + top on are two further up, with it and after it)
+    const unsigned int t = (unsigned int)(m.top >> m.shift) + 1;
+    a = c0 <= t ? (unsigned long long)(c0 - 1) << m.shift : c0 == t + 1 ? m.top : c0 == t + 2 ? m.top + 1 : (unsigned long long)(c0 - 3) << m.shift;
+    b = c1 <= t ? step(c1 - 1) : c1 == t + 1 ? m.top - 1 : c1 == t + 2 ? m.top : step(c1 - 3);
+    if (c1 == t + 1 && m.top == 0) return false;
+  } else if (m.mode == MAP_LOG) {
+    a = log_from(m, c0 - 1);
+    b = log_last(m, c1 - 2);
+  } else {
+    return false;
+  }
+  b     = min(b, m.range);
+  if (a > b) return false;
+  *lo   = m.lo + a;
+  *span = b - a;
+  return true;
+}
+
 // Places of a tile: which segment, where in it.
 struct TileRange {
   unsigned int first, end;
@@ -197,7 +266,7 @@ __device__ __forceinline__ TileRange my_tiles(unsigned int ntiles)
 // what lies outside their range: with 1024 per segment of the second split one sort of 2^27 keys in a few had a cell
 // of outsiders that no bucket holds.
 template <int KB, int FORM, bool PAIRS, int SAMPLES>
-__global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl, SplitLevel L, unsigned int decide, typename KeyOf<KB>::type flip)
+__global__ void __launch_bounds__(SPLIT_THREADS, KB == 8 && FORM == FORM_FLOAT ? 1 : 2) split_sample_kernel(Ctrl* ctrl, SplitLevel L, unsigned int decide, typename KeyOf<KB>::type flip)
 {
   using K = typename KeyOf<KB>::type;
   extern __shared__ unsigned int sh_cells[];
@@ -238,6 +307,18 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
     img[j] = i < ns ? src[at[j]] : (K)0;
     if (PAIRS && L.src_pos != nullptr) at[j] = i < ns ? L.src_pos[begin + at[j]] : 0u;
   }
+  // one more key of every stretch per round (of argsorts), from parts of it that do not meet; on their way into the L2 early, since each
+  // round waits for its own (2^28 uint64 keys: three rounds 40 us without)
+  const unsigned int part = PAIRS && L.rounds > 1 ? len / SAMPLES / (L.rounds - 1) : 0;
+  auto further = [&](unsigned int i, unsigned int r) {
+    return (unsigned int)(((unsigned long long)i * len) / SAMPLES) + (r - 1) * part + __umulhi((i + r) * 2654435761u, part);
+  };
+  if (PAIRS && decide) {
+    for (unsigned int r = 1; r < L.rounds; ++r) {
+#pragma unroll
+      for (int j = 0; j < PER; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + further(j * SPLIT_THREADS + tid, r)));
+    }
+  }
   auto mine = [&](int j) { return j * SPLIT_THREADS + tid < ns; };
   K lo = (K)~(K)0, hi = 0;
   unsigned int flags = 0, odd = 0;
@@ -277,9 +358,11 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
   if (lo > hi) lo = hi = (K)~(K)0;  // no finite ones: taken for NaNs
   const unsigned int nan = split_nan_cells(FORM, PAIRS, L.cells), ci = L.cells - 2 - nan;
   const K lo_seen = lo, hi_seen = hi;
-  if ((unsigned long long)(hi - lo) >= ci) {
-    // some room for the keys outside the sampled range, which would all lie in one cell
-    const K room = (K)((hi - lo) >> 6);
+  const bool narrow = (unsigned long long)(hi - lo) < ci;
+  if (!narrow || (FORM == FORM_INT && !PAIRS)) {
+    // some room for the keys outside the sampled range, which would all lie in one cell; a narrow range of integers has cells to
+    // spare (10^7 keys around one place, a hundredth elsewhere: rare values of the crowd that 2048 samples missed filled that cell)
+    const K room = narrow ? (K)((ci - 1 - (unsigned int)(hi - lo)) / 2) : (K)((hi - lo) >> 6);
     const K least = FORM != FORM_INT ? (K)((K)FIN_LO << (8 * KB - 32)) : (K)0, most_ = FORM != FORM_INT ? (K)~least : (K)~(K)0;
     lo = lo - least > room ? (K)(lo - room) : least;
     hi = most_ - hi > room ? (K)(hi + room) : most_;
@@ -435,6 +518,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
       flags = __reduce_or_sync(0xFFFFFFFFu, flags);
       if (lane == 0 && flags) atomicOr(&sh_marks.flags, flags);
     }
+    // What a leaf, or a later split, cannot take apart would be found out late: the fullest cell, if its samples say so by three
+    // standard deviations.  (A cell of one value is filled in, one of a few is counted.)
+    const unsigned int cell = most & 0xFFFFu;
+    const float k_ = (float)(most >> 16), sure = k_ - 3.0f * sqrtf(k_), leaf = (float)L.leaf_cap * (float)ns / (float)len;
+    constexpr float NEXT = SPLIT_BINS * 15 / 16;   // leaves of a segment
+    // of the integers of a sort those in that cell
+    unsigned int in_fullest = 0;
+    if (!PAIRS && FORM == FORM_INT && !L.last && sure > NEXT * leaf) {
+      with_mode<FORM, PAIRS>(m.mode, [&](auto md) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j) in_fullest |= cell_of<KB, FORM, PAIRS, decltype(md)::value>(img[j], at[j], m, ci) == cell ? 1u << j : 0u;
+      });
+    }
     unsigned int same = 0, bytes = 0;
     auto print = [&](K image) {
       if (FORM != FORM_INT && image == (K)~(K)0) return;
@@ -450,25 +546,17 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
         const unsigned long long d = (unsigned long long)(img[j] ^ lo_seen);
 #pragma unroll
         for (int k = 0; k < KB; ++k) bytes |= (d >> (8 * k) & 0xFFu) ? 1u << k : 0u;
-        if (PAIRS || FORM != FORM_INT) print(img[j]);
+        if (PAIRS || FORM != FORM_INT || (in_fullest >> j & 1u)) print(img[j]);
       }
     }
     if (PAIRS) {
-      // one more key of every stretch per round, from parts of it that do not meet
       for (unsigned int r = 1; r < L.rounds; ++r) {
-        const unsigned int part = len / SAMPLES / (L.rounds - 1);
         K more[PER];
-        bool other[PER];
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-          const unsigned int i = j * SPLIT_THREADS + tid;
-          const unsigned int p = (unsigned int)(((unsigned long long)i * len) / SAMPLES) + (r - 1) * part + __umulhi((i + r) * 2654435761u, part);
-          other[j]             = p != place(i);
-          more[j]              = src[p];
-        }
+        for (int j = 0; j < PER; ++j) more[j] = src[further(j * SPLIT_THREADS + tid, r)];
 #pragma unroll
         for (int j = 0; j < PER; ++j)
-          if (other[j]) print(split_image<KB, FORM>(more[j], flip));
+          if (further(j * SPLIT_THREADS + tid, r) != place(j * SPLIT_THREADS + tid)) print(split_image<KB, FORM>(more[j], flip));
       }
     }
     same  = __reduce_add_sync(0xFFFFFFFFu, same);
@@ -488,12 +576,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_sample_kernel(Ctrl* ctrl,
       // (of an argsort equal keys have to be taken apart; in a sort of floats, whose cells cannot be seen to hold one value, they
       // fill cells that nothing splits)
       if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && eq >= 6 && copies > L.most_copies) route = ROUTE_RADIX;
-      if (PAIRS) {
-        // a cell that holds more than the next split takes apart could not be handled later
-        const unsigned long long est = (unsigned long long)(most >> 16) * len / ns;
-        const unsigned long long lim = L.last ? 4ull * L.cap : 1ull << 21;
-        if ((most >> 16) > 16 && est > lim) route = ROUTE_RADIX;
+      if (m.mode == MAP_TOP) {
+        // (the fullest cell is the value's own)
+      } else if (PAIRS) {
+        if (sure > (L.last ? 4.0f : NEXT) * leaf) route = ROUTE_RADIX;
+      } else if (!L.last) {
+        if (sure - (FORM == FORM_INT ? 2.0f * (float)eq : 0.0f) > NEXT * leaf && !(FORM != FORM_INT && cell == ci + 2)) route = ROUTE_RADIX;
+      } else if (sure > leaf) {
+        unsigned long long first, span;
+        const bool known = cell_bounds(m, cell, cell + 1, ci, &first, &span);
+        if (!(FORM != FORM_INT && cell == ci + 2) && (!known || span > (sure > COUNT_MOST * leaf ? 0u : COUNT_SPAN))) route = ROUTE_RADIX;
       }
+      // (a short row of few leaves has its tail in one of them, whose cells are linear)
+      if (KB == 4 && decide == 1 && m.mode == MAP_LOG && len < 6 * L.cap) route = ROUTE_RADIX;
       if (decide == 2 && (L.radix_if >> __popc(sh_n[1]) & 1u)) route = ROUTE_RADIX;
       atomicMax(&ctrl->route, route);
     }
@@ -606,67 +701,6 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
   }
 }
 
-// The only image of a cell, where it has one.
-template <int KB, int FORM, bool PAIRS>
-__device__ __forceinline__ bool cell_value(const SplitMap& m, unsigned int c, unsigned int ci, unsigned long long* image)
-{
-  if (FORM != FORM_INT && !PAIRS && c == ci + 2) {
-    *image = KB == 8 ? ~0ull : 0xFFFFFFFFull;
-    return true;
-  }
-  if (c < 1 || c > ci) return false;
-  if (m.mode == MAP_LIN && m.shift == 0) {
-    *image = m.lo + (c - 1);
-    return true;
-  }
-  if (m.mode == MAP_TOP && c == (unsigned int)(m.top >> m.shift) + 2) {
-    *image = m.lo + m.top;
-    return true;
-  }
-  if (m.mode == MAP_LOG) {
-    if (c == 1) {
-      *image = m.lo;
-      return true;
-    }
-    const float a = __uint_as_float((c - 1 + m.mult) << m.shift), b = __uint_as_float((c + m.mult) << m.shift);
-    if (b > 16777216.0f) return false;  // (below, a cell's ends are exact)
-    const float ca = ceilf(a);
-    if (ceilf(b) - ca != 1.0f) return false;
-    *image = m.lo + (unsigned long long)ca;
-    return true;
-  }
-  return false;
-}
-
-// The images that cells c0 .. c1 - 1 can hold, where the mapping tells.
-__device__ __forceinline__ bool cell_bounds(const SplitMap& m, unsigned int c0, unsigned int c1, unsigned int ci, unsigned long long* lo, unsigned long long* span)
-{
-  if (c0 < 1 || c1 - 1 > ci) return false;
-  unsigned long long a, b;  // first image, and the one behind the last, from m.lo on
-  if (m.mode == MAP_LIN) {
-    a = (unsigned long long)(c0 - 1) << m.shift;
-    b = (unsigned long long)(c1 - 1) << m.shift;
-  } else if (m.mode == MAP_TOP) {
-    // (cells from the one of lo + top on are two further up, with it and after it)
-    const unsigned int t = (unsigned int)(m.top >> m.shift) + 1;
-    auto from = [&](unsigned int c) {
-      return c <= t ? (unsigned long long)(c - 1) << m.shift : c == t + 1 ? m.top : c == t + 2 ? m.top + 1 : (unsigned long long)(c - 3) << m.shift;
-    };
-    a = from(c0);
-    b = from(c1);
-  } else if (m.mode == MAP_LOG) {
-    a = c0 == 1 ? 0 : (unsigned long long)ceilf(__uint_as_float((c0 - 1 + m.mult) << m.shift));
-    b = (unsigned long long)ceilf(__uint_as_float((c1 - 1 + m.mult) << m.shift));
-  } else {
-    return false;
-  }
-  b     = min(b - 1, m.range);
-  if (a > b) return false;
-  *lo   = m.lo + a;
-  *span = b - a;
-  return true;
-}
-
 // ---- pack: one block per segment cuts its cells into buckets ----
 // Latency of a handful of dependent steps on chip: 8 to 9 us, up to 50 where many values are filled in.  Walking from bucket to
 // bucket costs 35 cycles each with one lookup per step (220 with the four it takes to tell what a bucket is, hence
@@ -689,8 +723,9 @@ split_pack_kernel(Ctrl* ctrl, SplitLevel L, SplitLeaf* leaves, SplitSeg* next_se
   __shared__ unsigned int bin_cell[SPLIT_BINS], bin_end[SPLIT_BINS], bin_tile[SPLIT_BINS], bin_tiles[SPLIT_BINS];
   const unsigned int seg = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   chain_wait();
+  const bool mixed = FORM == FORM_FLOAT && !PAIRS && marks_mixed(L.marks->nan, L.marks->flags);
   if (__syncthreads_or(ld_relaxed(&ctrl->route) != ROUTE_SPLIT)) return;  // (other blocks may be changing it)
-  if (FORM == FORM_FLOAT && !PAIRS && marks_mixed(L.marks->nan, L.marks->flags)) {
+  if (mixed) {
     if (tid == 0) atomicMax(&ctrl->route, (unsigned int)ROUTE_LATE);
     return;
   }
@@ -861,7 +896,7 @@ split_pack_kernel(Ctrl* ctrl, SplitLevel L, SplitLeaf* leaves, SplitSeg* next_se
       if (cell_bounds(s.map, c0, c1, ci, &leaf.lo, &leaf.span)) leaf.len |= LEAF_BOUNDED;
       if (len > L.cap) {
         // more than fits the chip: keys of a few values are counted, others are left to the radix passes
-        fail = PAIRS || !(leaf.len & LEAF_BOUNDED) || leaf.span > COUNT_SPAN;
+        fail = PAIRS || !(leaf.len & LEAF_BOUNDED) || leaf.span > COUNT_SPAN || len > COUNT_MOST * L.cap;
         leaf.len |= LEAF_COUNT;
       }
     }
@@ -1332,13 +1367,22 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
       unsigned int* count = reinterpret_cast<unsigned int*>(cnt);
       const K* from       = static_cast<const K*>(A.keys) + leaf.begin;
       K* to               = static_cast<K*>(A.out) + leaf.begin;
-      for (unsigned int i = tid; i <= COUNT_SPAN; i += THREADS) count[i] = 0;
+      const unsigned int values = (unsigned int)leaf.span + 1;
+      for (unsigned int i = tid; i < (values + 31) / 32 * 32; i += THREADS) count[i] = 0;
       __syncthreads();
-      for (unsigned int i = tid; i < n; i += THREADS) atomicAdd(&count[(unsigned int)(split_image<KB, FORM>(from[i], flip) - (K)leaf.lo)], 1u);
+      constexpr unsigned int AHEAD = 8;
+      for (unsigned int i = tid; i < n; i += AHEAD * THREADS) {
+        K k[AHEAD];
+#pragma unroll
+        for (unsigned int j = 0; j < AHEAD; ++j) k[j] = i + j * THREADS < n ? from[i + j * THREADS] : (K)0;
+#pragma unroll
+        for (unsigned int j = 0; j < AHEAD; ++j)
+          if (i + j * THREADS < n) atomicAdd(&count[(unsigned int)(split_image<KB, FORM>(k[j], flip) - (K)leaf.lo)], 1u);
+      }
       __syncthreads();
       if (warp == 0) {   // counts -> ends
         unsigned int run = 0;
-        for (unsigned int i = lane; i <= COUNT_SPAN; i += 32) {
+        for (unsigned int i = lane; i < (values + 31) / 32 * 32; i += 32) {
           unsigned int incl = count[i];
 #pragma unroll
           for (int o = 1; o < 32; o <<= 1) {
@@ -1350,15 +1394,14 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
         }
       }
       __syncthreads();
-      for (unsigned int i = tid; i < n; i += THREADS) {
-        unsigned int a = 0, b = COUNT_SPAN;   // the first value that ends behind i
-        while (a < b) {
-          const unsigned int mid = (a + b) >> 1;
-          if (count[mid] > i) b = mid; else a = mid + 1;
-        }
-        const K o = (K)((K)leaf.lo + a);
-        if constexpr (FORM != FORM_INT) to[i] = marked_raw<KB>(o, A.marks);
-        else to[i] = (K)(o ^ flip);
+      for (unsigned int v = warp; v < values; v += THREADS / 32) {   // a warp writes the copies of a value
+        const unsigned int first = v ? count[v - 1] : 0u, end = count[v];
+        if (first == end) continue;
+        const K o = (K)((K)leaf.lo + v);
+        K raw;
+        if constexpr (FORM != FORM_INT) raw = marked_raw<KB>(o, A.marks);
+        else raw = (K)(o ^ flip);
+        for (unsigned int i = first + lane; i < end; i += 32) to[i] = raw;
       }
       __syncthreads();
       continue;
@@ -1564,6 +1607,7 @@ inline cudaError_t split_form(typename KeyOf<KB>::type flip, const SplitPlan& pl
     L.pos_n         = job.seg_len;
     L.radix_if      = plan.radix_if;
     L.rounds        = l == 0 ? split_rounds(job.seg_len, job.nseg, PAIRS) : 1;
+    L.leaf_cap      = plan.lev[plan.levels - 1].cap;
     L.most_copies   = split_most_copies(KB, PAIRS, job.nseg, plan);
     L.marks         = reinterpret_cast<SplitMarks*>(job.tables + plan.off_marks);
     L.src_keys      = l == 0 ? job.in : job.tmp_keys[0];

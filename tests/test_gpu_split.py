@@ -157,6 +157,46 @@ def test_sent_back_with_the_sample(dtype, op, n):
     assert _check(a, op) == RADIX
 
 
+def _crowds(how: str, n: int, dtype: np.dtype) -> np.ndarray:
+    rng, bits = np.random.default_rng(n), 8 * dtype.itemsize - 1
+    if how in ("signed", "negative"):          # every magnitude, in both directions or downwards only
+        a = np.exp2(rng.uniform(0, bits, n))
+        return (a * np.where(rng.random(n) < 0.5, 1.0, -1.0) if how == "signed" else -a).astype(dtype)
+    a = np.rint(rng.standard_normal(n) * 3)     # crowded around one place, or two, with outliers on both sides
+    if how == "two":
+        a += np.where(rng.random(n) < 0.5, 2.0**29, -(2.0**28))
+    out = rng.random(n) < 0.01
+    a[out] = rng.integers(-(2**20), 2**20, n)[out] if how == "one" else rng.integers(-(2**30), 2**30, n)[out]
+    return a.astype(dtype)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 300_007), (1, 2_100_019), (3, 400_009), (37, 20_011)])
+@pytest.mark.parametrize("dtype", ["int32", "int64"])
+def test_crowds_inside_the_range(split_all, dtype, rows, n):
+    """Integers whose crowd lies at neither end of their range: a second split fills in or takes apart what is crowded around a place;
+    what it could not, or a leaf, goes back with the sample.  No block is left with most of the keys."""
+    for how in ("signed", "negative", "one", "two"):
+        a = _crowds(how, rows * n, np.dtype(dtype))
+        got = _check(a.reshape(rows, n) if rows > 1 else a, "sort")
+        if n > 2_000_000:
+            assert got == SPLIT or how in ("signed", "negative"), how
+        else:
+            assert got in (SPLIT, RADIX), how
+
+
+@pytest.mark.parametrize("width,count,split", [(2048, 100_000, True), (2048, 140_000, False), (4096, 60_000, False)])
+def test_a_bucket_of_few_values(split_all, width, count, split):
+    """A cell of a row with no more values and keys than one block counts, or with more of either."""
+    rng, n = np.random.default_rng(width), 1_000_003
+    rows = np.empty((2, n), np.int64)
+    edge = width * 1000 - ((width * 1980 - 1) >> 6) % width     # of a cell: the range gets a 64th of itself as room
+    for r in rows:
+        r[:] = rng.integers(0, width * 1980, n)
+        r[:2] = 0, width * 1980 - 1
+        r[rng.permutation(n - 2)[:count] + 2] = edge + rng.integers(0, width, count)
+    assert (_check(rows, "sort") == SPLIT) == split
+
+
 @pytest.mark.parametrize("dtype", ["int32", "float32", "int64"])
 def test_rows_of_two_leaves(dtype):
     """Sorts of 4-byte keys in rows below 10000 keep the passes, others do not."""
