@@ -38,9 +38,9 @@ constexpr unsigned short LUT_DROP = 0xFFFF;
 constexpr int SPLIT_THREADS       = 512;
 constexpr int SPLIT_SAMPLES       = 4096;  // of a segment of the input
 constexpr int SPLIT_SAMPLES_NEXT  = 2048;  // of a bucket of the first split
-// Places for the samples' fingerprints by how often the samples are drawn: of keys of an argsort, whose copies decide (below),
-// more samples from 8 * 10^6 keys on, where 16 copies of each value are too few pairs among 4096.
-inline unsigned int split_rounds(unsigned int len, unsigned int nseg, bool pairs) { return !pairs || nseg != 1 || len <= 8000000u ? 1 : len <= 32000000u ? 2 : 4; }
+// Places for the samples' fingerprints by how often the samples are drawn: of argsorts, whose copies decide (below), twice from
+// 1.6 * 10^7 keys on, where a dozen copies of each value are too few pairs among 4096.  (Four rounds cost 2^27 uint64 keys 15 us.)
+inline unsigned int split_rounds(unsigned int len, unsigned int nseg, bool pairs) { return pairs && nseg == 1 && len > 16000000u ? 2 : 1; }
 __host__ __device__ constexpr unsigned int split_prints(unsigned int rounds) { return rounds == 1 ? 8192 : 32768; }
 
 template <int KB, bool PAIRS> struct SplitCfg {
@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, KB == 8 && FORM == FORM_FLOAT ?
     img[j] = i < ns ? src[at[j]] : (K)0;
     if (PAIRS && L.src_pos != nullptr) at[j] = i < ns ? L.src_pos[begin + at[j]] : 0u;
   }
-  // one more key of every stretch per round (of argsorts), from parts of it that do not meet; on their way into the L2 early, since each
-  // round waits for its own (2^28 uint64 keys: three rounds 40 us without)
+  // one more key of every stretch per round (of argsorts), from parts of it that do not meet; on their way into the L2 early, since a round
+  // waits for its own
   const unsigned int part = PAIRS && L.rounds > 1 ? len / SAMPLES / (L.rounds - 1) : 0;
   auto further = [&](unsigned int i, unsigned int r) {
     return (unsigned int)(((unsigned long long)i * len) / SAMPLES) + (r - 1) * part + __umulhi((i + r) * 2654435761u, part);
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, KB == 8 && FORM == FORM_FLOAT ?
     // What a leaf, or a later split, cannot take apart would be found out late: the fullest cell, if its samples say so by three
     // standard deviations.  (A cell of one value is filled in, one of a few is counted.)
     const unsigned int cell = most & 0xFFFFu;
-    const float k_ = (float)(most >> 16), sure = k_ - 3.0f * sqrtf(k_), leaf = (float)L.leaf_cap * (float)ns / (float)len;
+    const float k_ = (float)(most >> 16), sure = k_ - 3.0f * sqrtf(k_), leaf = (float)L.leaf_cap * __fdividef((float)ns, (float)len);
     constexpr float NEXT = SPLIT_BINS * 15 / 16;   // leaves of a segment
     // of the integers of a sort those in that cell
     unsigned int in_fullest = 0;
@@ -570,12 +570,13 @@ __global__ void __launch_bounds__(SPLIT_THREADS, KB == 8 && FORM == FORM_FLOAT ?
       unsigned int route = FORM == FORM_FLOAT && !PAIRS && marks_mixed(sh_marks.nan, sh_marks.flags) ? ROUTE_RADIX : ROUTE_SPLIT;
       // A sample finds its copies among those before it: half of the square, as long as few have any; then what counts is how many
       // others there are.
-      const unsigned int drawn    = ns * L.rounds, eq = sh_n[0];
-      unsigned long long copies   = (unsigned long long)eq * 2 * len / ((unsigned long long)drawn * drawn);
-      if (2 * eq > drawn) copies  = max(copies, (unsigned long long)(len / max(drawn - eq, 1u)));
+      const unsigned int eq = sh_n[0];
+      const float drawn     = (float)(ns * L.rounds);
+      float copies          = 2.0f * (float)eq * __fdividef((float)len, drawn * drawn);
+      if (2.0f * (float)eq > drawn) copies = fmaxf(copies, __fdividef((float)len, fmaxf(drawn - (float)eq, 1.0f)));
       // (of an argsort equal keys have to be taken apart; in a sort of floats, whose cells cannot be seen to hold one value, they
       // fill cells that nothing splits)
-      if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && eq >= 6 && copies > L.most_copies) route = ROUTE_RADIX;
+      if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && eq >= 6 && copies > (float)L.most_copies) route = ROUTE_RADIX;
       if (m.mode == MAP_TOP) {
         // (the fullest cell is the value's own)
       } else if (PAIRS) {
@@ -1394,14 +1395,26 @@ split_leaf_kernel(const Ctrl* ctrl, LeafArgs A, typename KeyOf<KB>::type flip)
         }
       }
       __syncthreads();
-      for (unsigned int v = warp; v < values; v += THREADS / 32) {   // a warp writes the copies of a value
-        const unsigned int first = v ? count[v - 1] : 0u, end = count[v];
-        if (first == end) continue;
+      auto raw_of = [&](unsigned int v) -> K {
         const K o = (K)((K)leaf.lo + v);
-        K raw;
-        if constexpr (FORM != FORM_INT) raw = marked_raw<KB>(o, A.marks);
-        else raw = (K)(o ^ flip);
-        for (unsigned int i = first + lane; i < end; i += 32) to[i] = raw;
+        if constexpr (FORM != FORM_INT) return marked_raw<KB>(o, A.marks);
+        else return (K)(o ^ flip);
+      };
+      if (n > 32 * values) {
+        for (unsigned int v = warp; v < values; v += THREADS / 32) {   // a warp writes the copies of a value
+          const unsigned int first = v ? count[v - 1] : 0u, end = count[v];
+          const K raw = raw_of(v);
+          for (unsigned int i = first + lane; i < end; i += 32) to[i] = raw;
+        }
+      } else {
+        for (unsigned int i = tid; i < n; i += THREADS) {
+          unsigned int a = 0, b = values - 1;   // the first value that ends behind i
+          while (a < b) {
+            const unsigned int mid = (a + b) >> 1;
+            if (count[mid] > i) b = mid; else a = mid + 1;
+          }
+          to[i] = raw_of(a);
+        }
       }
       __syncthreads();
       continue;

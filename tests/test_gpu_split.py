@@ -206,7 +206,7 @@ def test_rows_of_two_leaves(dtype):
 
 
 @pytest.mark.parametrize("dtype,rows,n,copies", [("float64", 1, 250_007, 60), ("float32", 1, 700_001, 400), ("float32", 1, 5_000_011, 60),
-                                                 ("int64", 1, 24_000_017, 60), ("float32", 1, 32_000_003, 40), ("float32", 60, 20_011, 80)])
+                                                 ("int64", 1, 24_000_017, 60), ("float32", 1, 16_000_003, 40), ("float32", 60, 20_011, 80)])
 def test_copies_send_argsorts_back(dtype, rows, n, copies):
     """Evenly used values: two copies of each stay with the splits, many go back with the sample, which draws more keys of long arrays."""
     rng = np.random.default_rng(n)
