@@ -264,9 +264,10 @@ __device__ __forceinline__ TileRange my_tiles(unsigned int ntiles)
 // ---- sample: one block per segment ----
 // Latency of scattered loads: 7 to 13 us for an array, 33 us for the 187 segments of 2^28 keys.  More samples would narrow
 // what lies outside their range: with 1024 per segment of the second split one sort of 2^27 keys in a few had a cell
-// of outsiders that no bucket holds.
+// of outsiders that no bucket holds.  Two blocks per SM at 64 registers (1000 rows of 12000 float64 88 -> 70 us); argsorts of float64
+// would spill (2 * 10^6 keys 138.9 -> 140.7).
 template <int KB, int FORM, bool PAIRS, int SAMPLES>
-__global__ void __launch_bounds__(SPLIT_THREADS, KB == 8 && FORM == FORM_FLOAT ? 1 : 2) split_sample_kernel(Ctrl* ctrl, SplitLevel L, unsigned int decide, typename KeyOf<KB>::type flip)
+__global__ void __launch_bounds__(SPLIT_THREADS, KB == 8 && FORM == FORM_FLOAT && PAIRS ? 1 : 2) split_sample_kernel(Ctrl* ctrl, SplitLevel L, unsigned int decide, typename KeyOf<KB>::type flip)
 {
   using K = typename KeyOf<KB>::type;
   extern __shared__ unsigned int sh_cells[];
