@@ -102,27 +102,39 @@ def split_all(monkeypatch):
     monkeypatch.setenv("B2S_SPLIT", "8193")
 
 
+def _tried(route: int, how: str, dtype: np.dtype, op: str) -> None:
+    """The splits were tried, spread keys stayed with them, and what needs the input order of equal images did not."""
+    assert route != OPEN
+    if how == "normal":
+        assert route == SPLIT
+    if how == "patterns" and dtype.kind == "f" and op == "sort":
+        assert route in (RADIX, LATE)
+
+
 @pytest.mark.parametrize("how", HOW)
 @pytest.mark.parametrize("op", ["sort", "argsort"])
 @pytest.mark.parametrize("dtype", ["int32", "uint32", "float32", "int64", "uint64", "float64"])
 def test_two_splits(split_all, dtype, op, how):
-    # (more keys than one split takes apart)
-    _check(_values(how, 2_100_019, np.dtype(dtype), 11), op)
+    # (more keys than one split takes apart, and of 4-byte argsorts so many that the tables fit)
+    t = np.dtype(dtype)
+    n = 5_000_011 if op == "argsort" and t.itemsize == 4 else 2_100_019
+    _tried(_check(_values(how, n, t, 11), op), how, t, op)
 
 
 @pytest.mark.parametrize("how", HOW)
 @pytest.mark.parametrize("op", ["sort", "argsort"])
 @pytest.mark.parametrize("dtype", ["int32", "float32", "uint64", "float64"])
 def test_one_split(split_all, dtype, op, how):
-    _check(_values(how, 300_007, np.dtype(dtype), 13), op)
+    _tried(_check(_values(how, 300_007, np.dtype(dtype), 13), op), how, np.dtype(dtype), op)
 
 
 @pytest.mark.parametrize("how", HOW)
 @pytest.mark.parametrize("op", ["sort", "argsort"])
 @pytest.mark.parametrize("dtype", ["int32", "float32", "uint64", "float64"])
 def test_long_rows(dtype, op, how):
-    n, rows = 20_011, 37
-    _check(_values(how, n * rows, np.dtype(dtype), 12).reshape(rows, n), op)
+    t = np.dtype(dtype)
+    n, rows = 20_011, 60   # (sorts of 4-byte keys: from 10^6 on)
+    _tried(_check(_values(how, n * rows, t, 12).reshape(rows, n), op), how, t, op)
 
 
 # around the lengths where the buckets' size, the number of splits and the tables change: 200 buckets of 2048, 4096, 6144
@@ -130,10 +142,81 @@ def test_long_rows(dtype, op, how):
 @pytest.mark.parametrize("n", [8193, 8704, 16384, 30011, 409_600, 409_601, 819_201, 1_100_003, 1_228_801, 1_638_401])
 @pytest.mark.parametrize("dtype", ["int32", "float32", "int64", "float64"])
 def test_lengths(split_all, dtype, n):
+    t = np.dtype(dtype)
     for op in ("sort", "argsort"):
-        _check(_values("nans", n, np.dtype(dtype), n), op)
+        route = _check(_values("nans", n, t, n), op)
+        # (the tables of two splits of 4-byte pairs do not fit the look-back room of so few keys)
+        assert (route == OPEN) == (t.itemsize == 4 and op == "argsort" and n > 1_228_800)
     if n < 100_000:
-        _check(_values("nans", n * 3, np.dtype(dtype), n).reshape(3, n), "argsort")
+        # (nor those of few rows of up to 16384 4-byte pairs)
+        route = _check(_values("nans", n * 3, t, n).reshape(3, n), "argsort")
+        assert (route == OPEN) == (t.itemsize == 4 and n <= 16384)
+
+
+@pytest.mark.parametrize("dtype,op,n", [("int32", "sort", 39_000_017), ("int32", "sort", 60_000_011), ("int64", "sort", 60_000_011), ("float64", "sort", 60_000_011),
+                                        ("float32", "argsort", 39_000_017), ("int64", "argsort", 93_000_017), ("float64", "argsort", 93_000_017)])
+def test_long_plans(dtype, op, n):
+    """Plans of 8192 cells, and leaves of 8192, with positions 6144, keys after two splits, for each mapping; against torch's sort."""
+    import cupynumeric_b200 as num
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    t = getattr(torch, dtype)
+    bits = 8 * t.itemsize
+    if t.is_floating_point:
+        draws = [torch.rand(n, dtype=t, device="cuda", generator=gen), torch.randn(n, dtype=t, device="cuda", generator=gen)]
+        draws[1][7::1001] = float("nan")
+    else:
+        raw = torch.randint(0, 256, (n * t.itemsize,), dtype=torch.uint8, device="cuda", generator=gen).view(t)
+        u = torch.rand(n, dtype=torch.float64, device="cuda", generator=gen)
+        draws = [raw, (1 - u).pow(-5.0).clamp(max=2.0 ** min(bits - 2, 40)).to(t)] if op == "sort" else [raw]   # (Zipf argsorts go back)
+        if op == "sort":
+            draws.append(torch.where(u < 0.5, torch.full((), 12345, dtype=t, device="cuda"), raw))     # a spike
+    for k, a in enumerate(draws):
+        want = torch.sort(a, stable=True)
+        got = num.sort(num.array(a)) if op == "sort" else num.argsort(num.array(a), kind="stable")
+        assert _route() == SPLIT, k
+        if op == "argsort":
+            assert torch.equal(got.torch(), want.indices)
+        else:
+            i = torch.int32 if bits == 32 else torch.int64
+            assert torch.equal(got.torch().view(i), want.values.view(i))
+        del want, got
+
+
+@pytest.mark.parametrize("names", [("float64", "int32"), ("float32", "int64"), ("int64", "float64", "int8")], ids="-".join)
+def test_first_keys_of_lexsort(split_all, names):
+    """Positions as 32 bits straight out of the leaves, for the keys behind."""
+    import cupynumeric_b200 as num
+
+    rng, n = np.random.default_rng(6), 300_007
+    cols = [_values("normal", n, np.dtype(d), 5) if i == 0 else rng.integers(0, 90, n).astype(d) for i, d in enumerate(names)]
+    cols[0][1::2] = cols[0][: n // 2]     # (two copies of each)
+    assert np.array_equal(num.lexsort(cols).to_numpy(), np.lexsort(cols))
+
+
+@pytest.mark.parametrize("n", [300_007, 3_000_017])
+def test_payloads_of_complex_argsorts(n):
+    """The real parts are sorted behind the imaginary ones, whose order is the payload that the leaves look up."""
+    import cupynumeric_b200 as num
+
+    rng = np.random.default_rng(n)
+    a = rng.permutation(np.repeat(rng.standard_normal(n // 2 + 1), 2)[:n]) + 1j * rng.permutation(np.repeat(rng.standard_normal(n // 3 + 1), 3)[:n])
+    assert np.array_equal(num.argsort(a, kind="stable").to_numpy(), np.argsort(a, kind="stable"))
+
+
+@pytest.mark.parametrize("dtype", ["float64", "uint64"])
+def test_payloads_of_distributed_argsorts(split_all, dtype):
+    """What a rank received carries positions of the whole array."""
+    from tests.test_gpu_dist_threads import run_ranks
+
+    t = np.dtype(dtype)
+    a = _values("normal", 700_001, t, 9)
+    a[1::2] = a[:350_000]
+    shards = np.split(a, [250_000, 460_000])
+    parts = [part for status, part, _, _ in run_ranks(shards, True) if status == 0]
+    assert len(parts) == 3 and min(p.size for p in parts) > 200_000
+    assert np.array_equal(np.concatenate(parts), np.argsort(a, kind="stable"))
 
 
 @pytest.mark.parametrize("dtype,n", [("float32", 6_000_011), ("int64", 24_000_017)])
