@@ -47,7 +47,8 @@ L2_BYTES = 126 << 20
 # adds the k-way merge); nvlink_bytes: bytes per key that cross NVLink per direction, before the
 # (P-1)/P factor; sweep_bytes: algorithmic bytes per key of one launch of the dominant kernel.  Only what runs is
 # counted.  c2 runs a histogram and four radix passes; the others with a split_move_kernel two splits, each counted and moved, and the
-# leaves: c1 4 + 8 + 4 + 8 + 8; c4, of whose keys 0.39 are moved and the others filled in, 8 + 11.1 + 3.1 + 6.2 + 11.1;
+# leaves: c1 4 + 8 + 4 + 8 + 8; c4, of whose keys 0.39 are moved and the others filled in, 8 + 11.1 + 3.1 + 6.2 + 11.1, on one GPU:
+# on several the ranks hold key ranges of which very different parts are moved, and no figure by bytes is given (None);
 # c5 8 + 20 + 8 + 24 + 20.
 CONFIGS = {
     "c1": dict(label="1-D int32 sort, N=2^{log2} per GPU, keys uniform over the full int32 range", dtype="i32", log2=24,
@@ -60,7 +61,7 @@ CONFIGS = {
                log2=28, argsort=False, hbm_bytes=(16.0, 16.0), nvlink_bytes=0.0, sweep_bytes=16.0,
                kernel="segmerge_kernel", multi="rows"),
     "c4": dict(label="1-D int64 distributed sort, 2^{log2} keys per GPU, Zipf(1.2) clipped to [0,2^40)", dtype="i64",
-               log2=28, argsort=False, hbm_bytes=(39.5, 55.5), nvlink_bytes=8.0, sweep_bytes=8.65,
+               log2=28, argsort=False, hbm_bytes=(39.5, None), nvlink_bytes=8.0, sweep_bytes=8.65,
                kernel="split_move_kernel", multi="distributed"),
     "c5": dict(label="1-D uint64 distributed stable argsort -> int64, 2^{log2} keys per GPU, ascending with 1% pair swaps",
                dtype="u64", log2=28, argsort=True, hbm_bytes=(80.0, 104.0), nvlink_bytes=16.0, sweep_bytes=22.0,
@@ -537,18 +538,19 @@ class Bench:
         total_keys = n_local * nranks
         gkeys = total_keys / (ms * 1e-3) / 1e9
         hbm_bytes = c["hbm_bytes"][1 if multi else 0]
-        t_hbm = hbm_bytes * n_local / (self.peak * 1e9)
+        t_hbm = (hbm_bytes or 0.0) * n_local / (self.peak * 1e9)
         t_nvl = c["nvlink_bytes"] * (nranks - 1) / nranks * n_local / (NVLINK_GBS * 1e9) if multi else 0.0
         floor = max(t_hbm, t_nvl)
         rec.update({
             "keys_per_gpu": n_local, "ms_per_step": ms, "gkeys_per_s": gkeys,
             "verified": {"ok": bool(small_ok and full_ok), "oracle_bit_exact_at_reduced_size": bool(small_ok),
                          "full_size_properties": detail},
-            "roofline": {"bound": "hbm" if t_hbm >= t_nvl else "nvlink", "hbm_bytes_per_key": hbm_bytes,
+            "roofline": {"bound": None if not hbm_bytes else "hbm" if t_hbm >= t_nvl else "nvlink", "hbm_bytes_per_key": hbm_bytes,
                          "nvlink_bytes_per_key_per_direction": c["nvlink_bytes"] * (nranks - 1) / nranks if multi else 0.0,
-                         "floor_ms": floor * 1e3, "frac": floor * 1e3 / ms, "hbm_peak_gbs": self.peak,
+                         "floor_ms": floor * 1e3 if hbm_bytes else None, "frac": floor * 1e3 / ms if hbm_bytes else None,
+                         "hbm_peak_gbs": self.peak,
                          "peak_source": f"of {self.peak_kind}", "nvlink_gbs": NVLINK_GBS,
-                         "frac_of_8TBs": (max(hbm_bytes * n_local / 8e12, t_nvl)) * 1e3 / ms},
+                         "frac_of_8TBs": (max(hbm_bytes * n_local / 8e12, t_nvl)) * 1e3 / ms if hbm_bytes else None},
             "kernels": kernels, "kernels_of_rank": kernels_rank, "gpu_launches_per_step": launches / args.steps,
             "l2": "input smaller than L2: a 256 MB buffer is written between timed steps" if flush
                   else "input larger than the 126 MB L2, no flush needed",
@@ -556,7 +558,7 @@ class Bench:
         if multi:
             rec["exchange"] = os.environ.get("B2S_DIST_P2P", "1") != "0" and "peer" or "nccl"
         dom = {"onesweep_kernel": "sweep", "split_move_kernel": "sweep", "segmerge_kernel": "segsort"}[c["kernel"]]
-        if dom in kernels:
+        if dom in kernels and hbm_bytes:
             avg_ms = kernels[dom]["avg_working_launch_ms"]
             achieved = c["sweep_bytes"] * n_local / (avg_ms * 1e-3) / 1e9
             traffic = ncu_traffic_bytes_per_key().get(name)

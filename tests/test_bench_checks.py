@@ -95,3 +95,11 @@ def test_reference_arm_prints_one_line(capsys, monkeypatch):
     line = json.loads(capsys.readouterr().out.strip().splitlines()[-1])
     assert line["impl"] == "reference" and line["cpu_baseline"]["cores"] == bench.host_threads()
     assert line["steps"] == 2 and line["e2e"]["h2d_bytes_per_step"] == 0
+
+
+def test_no_figures_by_bytes_that_describe_no_rank():
+    """How much of the Zipf keys is moved depends on a rank's key range: bytes per key are those of one GPU alone."""
+    import bench
+
+    assert bench.CONFIGS["c4"]["hbm_bytes"] == (39.5, None)
+    assert all(b is not None for name, c in bench.CONFIGS.items() if name != "c4" for b in c["hbm_bytes"])
