@@ -120,7 +120,7 @@ inline cudaError_t launch_sweeps(Ctrl* ctrl, unsigned int* lookback, unsigned in
 }
 
 // Testing aid and comparisons: B2S_SPLIT=0 leaves every sort to the radix passes, another number is the length from which
-// 1-D sorts are tried by the splitting kernels, whatever the keys.
+// 1-D sorts are tried by the splitting kernels, whatever bytes of the keys differ; rows are tried then at every length.
 inline long long split_override()
 {
   const char* e = std::getenv("B2S_SPLIT");
@@ -138,13 +138,21 @@ inline long long split_override()
 //   float64 argsort                2 * 10^5 87 -> 70, 4 103 -> 75, 80 * 10^6 4587 -> 2536
 //   uint64 argsort, almost in order  3 * 10^7 940 -> 769, 2^28 8094 -> 6225
 //   int64 sort, Zipf               3 * 10^7 921 -> 468, 2^28 7174 -> 3120
-// Whether bytes are constant is not known before the sample; keys that are sent back have paid for it and for the
-// launches (about 15 us for one split, 25 for two).  Integers, whose upper bytes often are constant, are tried only
-// where that is a small part or the splits win all the same.  So int32 argsorts are not tried (full range 4 * 10^7
-// 1002 -> 843 us, but a hundred values 5 * 10^7 346 -> 373), and 8-byte integers not below 2.4 * 10^7 (full range sort 10^7
-// 601 -> 309, but Zipf 8 * 10^6 317 -> 344, almost in order 214 -> 236).  Float64 keys that hold whole numbers differ in
-// five bytes; many copies crowd their cells, which the splits find out late (unique of ids, 5 * 10^6:
-// 334 -> 450 us, sent back by the sample 361).  Of int64 sorts two differing bytes go back (65536 values, 8 * 10^7 1110 -> 1655),
+// Whether bytes are constant is not known before the sample; keys that are sent back have paid for it and for the launches: 13
+// to 17 us for one split, 22 to 30 for two.  On both sides of the borders, passes -> splits, and what goes back:
+//   int32 sort 16       full range 10^7 264 -> 197 and 14 * 10^6 335 -> 241, but of 65536 values 154 -> 176 and 185 -> 208; 16 * 10^6
+//                       365 -> 264, 205 -> 227: a tenth.  A hundred values stay, one byte differing: 16 134 -> 134, 40 259 -> 237, 160 * 10^6
+//                       856 -> 683; two and three go back (65536 values, 16 * 10^6 by splits 234 and more)
+//   int32 argsort none  full range 16 * 10^6 494 -> 370, 40 1012 -> 819, but Zipf 453 -> 492, 942 -> 980, 2^24 values 774 -> 829
+//   int64 24            sort, full range 8 * 10^6 513 -> 250, 12 702 -> 335, 20 1071 -> 490, but Zipf 8 377 -> 502 (12 514 -> 270), 65536
+//                       values, which go back, 8 166 -> 191, 20 338 -> 363, 24 397 -> 417
+//   float32 sort 0.9    one split 0.7 * 10^6 60 -> 59, 0.85 66 -> 61, 1.3 74 -> 65; two (5) 1.7 85 -> 93, 2.5 98 -> 115, 3.5 124 -> 140, 4.5 169 -> 152
+//                       (scores 164 -> 163), 5 179 -> 168
+//   float32 argsort 0.6 one split 0.3 * 10^6 55 -> 55, 0.45 63 -> 55, 0.6 98 -> 59; to 10^8: 0.9 * 10^8 2062 -> 1832, 1.6 3540 -> 3229 (with
+//                       NaNs and copies 3377), 2.7 5769 -> 5497 (5736)
+//   float64 0.2         sort 10^5 76 -> 64, 2 * 10^5 83 -> 64; what goes back 54 -> 68
+// Float64 keys that hold whole numbers differ in five bytes; many copies crowd their cells (unique of ids, 5 * 10^6: 334 us, by
+// splits 450, sent back by the sample 361).  Of int64 sorts two differing bytes go back (65536 values, 8 * 10^7 1110 -> 1655),
 // one and three do not (a hundred values 670 -> 644, 2^24 values 2.4 * 10^7 544 -> 503, 8 1559 -> 1629).
 // Argsorts of keys that are alike as far as the sample sees need few passes, and the splits, which cut them by position, give up
 // late: they go back (one value, 2.4 * 10^7 int64 148 us by the passes, by the splits 519; 8 * 10^6 float64 73, 935).  Sorts of such
@@ -160,7 +168,7 @@ inline SplitPlan split_plan_1d(size_t n, bool pairs, bool keys_too, size_t room)
   if (KB == 4) least = !FLOAT ? (pairs ? SIZE_MAX : 16000000) : p.levels != 1 ? 5000000 : pairs ? 600000 : 900000;
   else least = FLOAT ? 200000 : 24000000;
   if (n < (over > 0 ? (size_t)over : least)) p.ok = false;
-  // (float32 argsort of 2^28 5.80 -> 5.85 ms)
+  // (above, the gain shrinks to that of the noise for keys with NaNs and copies)
   if (KB == 4 && pairs && n > 100000000 && over < 0) p.ok = false;
   // each byte in which the keys differ is a radix pass
   if (over <= 0) p.radix_if = KB == 4 ? (pairs ? 0xFu : p.levels == 1 ? 0xEu : 0xCu) : FLOAT ? (pairs ? 0x3Fu : 0x3Eu) : pairs ? 0xFu : 0x4u;

@@ -45,8 +45,8 @@ __host__ __device__ constexpr unsigned int split_prints(unsigned int rounds) { r
 
 template <int KB, bool PAIRS> struct SplitCfg {
   // (two blocks per SM, each with its tile, the counters and the table of up to 8192 cells)
-  // Keys per thread, by sweeps: more spill, fewer make shorter runs (int64 14 -> 12: a split of 2^25 keys 176 -> 160 us; float32
-  // with positions 14 -> 12: the second split of 2^25 179 -> 160).
+  // Keys per thread, by sweeps: more spill more, fewer make shorter runs (int64 14 -> 12: a split of 2^25 keys 176 -> 160 us; float32
+  // with positions 14 -> 12: the second split of 2^25 179 -> 160).  These spill 48 to 104 bytes of a thread's each way in the moves.
   static constexpr int ITEMS = KB == 8 && PAIRS ? 9 : KB == 8 || PAIRS ? 12 : 16;
   static constexpr int TILE  = SPLIT_THREADS * ITEMS;
 };
@@ -577,7 +577,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, KB == 8 && FORM == FORM_FLOAT &
       if (2.0f * (float)eq > drawn) copies = fmaxf(copies, __fdividef((float)len, fmaxf(drawn - (float)eq, 1.0f)));
       // (of an argsort equal keys have to be taken apart; in a sort of floats, whose cells cannot be seen to hold one value, they
       // fill cells that nothing splits)
-      if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && eq >= 6 && copies > (float)L.most_copies) route = ROUTE_RADIX;
+      const bool each = decide == 1 && !PAIRS && m.mode == MAP_LIN && m.shift == 0;   // (a row of few values has a cell for each)
+      if ((PAIRS || FORM != FORM_INT) && m.mode != MAP_POS && !each && eq >= 6 && copies > (float)L.most_copies) route = ROUTE_RADIX;
       if (m.mode == MAP_TOP) {
         // (the fullest cell is the value's own)
       } else if (PAIRS) {

@@ -39,8 +39,9 @@ struct SplitSeg {
 constexpr unsigned int LEAF_FILL = 1u << 31, LEAF_BOUNDED = 1u << 30, LEAF_COUNT = 1u << 29;
 constexpr unsigned int LEAF_LEN   = LEAF_COUNT - 1;   // (two-split plans take fewer keys, rows are shorter)
 constexpr unsigned int COUNT_SPAN = 2047;
-// (one block counts a bucket: 10^6 keys of a few values took it 1 ms while all others were done after 0.1)
-constexpr unsigned int COUNT_MOST = 16;               // times `cap`
+// (one block counts a bucket: at this length, 96 keys per thread, it takes about as long as sending short rows back; 10^6 keys took
+// it 1 ms while all others were done after 0.1)
+constexpr unsigned int COUNT_MOST = 6;                // times `cap`
 struct SplitLeaf {
   unsigned int begin, len;
   unsigned long long lo, span;

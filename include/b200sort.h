@@ -82,7 +82,8 @@ int b2s_workspace_bytes(int dtype, size_t volume, size_t segment, int argsort, s
  *   idx_out   NULL for sort; for argsort receives int64 positions along the sort axis:
  *             1-D (ndim_is_1 != 0): index_offset + i ;  N-D: i % segment + index_offset
  *             (src/cupynumeric/sort/sort.cu:1851-1862, sort.h:83-92)
- *   ws        device scratch of at least b2s_workspace_bytes(...) bytes, 256-byte aligned
+ *   ws        device scratch of at least b2s_workspace_bytes(...) bytes, 256-byte aligned; calls that are not
+ *             ordered (other streams, other host threads) need one each
  *
  * Replaces local_sort<CODE> -> cub_local_sort / thrust_local_sort
  * (src/cupynumeric/sort/sort.cu:63-96, cub_sort.cuh:36-193, thrust_sort.cuh:37-124) together
@@ -336,7 +337,9 @@ int b2s_partition_1d(int dtype, const void* keys_in, void* keys_out, int64_t* id
  * being the least significant (numpy.lexsort's convention): `volume` elements per key in
  * `volume / segment` rows; idx_out receives int64 positions inside each row.  One stable argsort per
  * key with the order so far carried through it; no step leaves the library.  `ws`:
- * b2s_lexsort_workspace_bytes(...) bytes, 256-byte aligned.  Replaces the chain of ARGSORT tasks
+ * b2s_lexsort_workspace_bytes(...) bytes, 256-byte aligned: 35 to 46 bytes per row of short and 4-byte keys,
+ * 57 where neighbouring keys are sorted as one of eight bytes (57 for 8-byte keys anyway); a smaller one down to what the widest
+ * key takes by itself is accepted, and the keys are sorted one by one then.  Replaces the chain of ARGSORT tasks
  * and gathers of cupynumeric/_module/ssc_sorting.py:423-444. */
 int b2s_lexsort_workspace_bytes(int nkeys, const int* dtypes, size_t volume, size_t segment, size_t* bytes);
 int b2s_lexsort(int nkeys, const int* dtypes, const void* const* keys, int64_t* idx_out, size_t volume, size_t segment,

@@ -267,7 +267,7 @@ def test_crowds_inside_the_range(split_all, dtype, rows, n):
             assert got in (SPLIT, RADIX), how
 
 
-@pytest.mark.parametrize("width,count,split", [(2048, 100_000, True), (2048, 140_000, False), (4096, 60_000, False)])
+@pytest.mark.parametrize("width,count,split", [(2048, 45_000, True), (2048, 55_000, False), (4096, 45_000, False)])
 def test_a_bucket_of_few_values(split_all, width, count, split):
     """A cell of a row with no more values and keys than one block counts, or with more of either."""
     rng, n = np.random.default_rng(width), 1_000_003
@@ -278,6 +278,12 @@ def test_a_bucket_of_few_values(split_all, width, count, split):
         r[:2] = 0, width * 1980 - 1
         r[rng.permutation(n - 2)[:count] + 2] = edge + rng.integers(0, width, count)
     assert (_check(rows, "sort") == SPLIT) == split
+
+
+@pytest.mark.parametrize("dtype", ["int32", "float32", "int64"])
+def test_rows_of_one_value(dtype):
+    """A cell of its own, filled in: no copies that crowd anything."""
+    assert _check(np.full((200, 12_000), 3, np.dtype(dtype)), "sort") == SPLIT
 
 
 @pytest.mark.parametrize("dtype", ["int32", "float32", "int64"])
