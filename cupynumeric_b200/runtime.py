@@ -27,7 +27,8 @@ class Scratch:
 
 
 class Runtime:
-    KEPT = 8       # workspaces kept per process, least recently used first out
+    KEPT = 8       # workspaces kept per process, least recently used first out,
+    KEPT_BYTES = 16 << 30   # and what the others may hold when one is made
     STICKY = 64    # status words kept per process
 
     def __init__(self) -> None:
@@ -82,7 +83,7 @@ class Runtime:
     def _renew(self, key: tuple[int, int, int], nbytes: int) -> Scratch:
         with self._lock:
             self._kept.pop(key, None)
-            while len(self._kept) >= self.KEPT:
+            while len(self._kept) >= self.KEPT or sum(k.nbytes for k in self._kept.values()) > self.KEPT_BYTES:
                 del self._kept[min(self._kept, key=lambda k: self._kept[k].used)]
             try:
                 ws = self._bytes(nbytes)

@@ -80,6 +80,13 @@ def test_what_is_kept_is_bounded_and_given_back(run):
         run.workspace((1 << 20) + 1)
 
 
+def test_what_the_others_hold_is_bounded_too(run, monkeypatch):
+    monkeypatch.setattr(Runtime, "KEPT_BYTES", 3 << 20)
+    for run.stream in range(4):
+        run.workspace(2 << 20)
+    assert sorted(k[1] for k in run._kept) == [2, 3]
+
+
 @pytest.mark.parametrize("streams", [2, 66])
 def test_a_failure_on_any_stream_is_raised_once(run, streams):
     for run.stream in range(streams):
