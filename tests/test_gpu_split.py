@@ -359,6 +359,26 @@ def test_in_place_and_other_streams(split_all):
     assert np.array_equal(y.to_numpy(), np.sort(b))
 
 
+def test_two_threads_on_one_stream(split_all):
+    """Their kernels are enqueued in any order between each other."""
+    import threading
+
+    import cupynumeric_b200 as num
+
+    inputs = [_values("normal", 300_007, np.dtype("float64"), k) for k in (1, 2)]
+    dev = [num.array(torch.from_numpy(a).cuda()) for a in inputs]
+    torch.cuda.synchronize()
+    out = [[], []]
+    threads = [threading.Thread(target=lambda i=i: out[i].extend(num.argsort(dev[i], kind="stable") for _ in range(20))) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        want = np.argsort(inputs[i], kind="stable")
+        assert len(out[i]) == 20 and all(np.array_equal(o.to_numpy(), want) for o in out[i])
+
+
 def test_under_capture(split_all):
     """The launches and their chaining can be captured and replayed on other keys."""
     import ctypes
