@@ -105,7 +105,10 @@ __device__ __forceinline__ void mark(typename KeyOf<KB>::type raw, typename KeyO
 {
   if (image != (typename KeyOf<KB>::type)~(typename KeyOf<KB>::type)0) {
     flags |= MARK_NEG_ZERO;
-  } else if (*reinterpret_cast<volatile unsigned long long*>(&block->nan) != (unsigned long long)raw) {
+    return;
+  }
+  flags |= MARK_OTHER;
+  if (*reinterpret_cast<volatile unsigned long long*>(&block->nan) != (unsigned long long)raw) {
     const unsigned long long old = atomicCAS(&block->nan, 0ull, (unsigned long long)raw);
     if (old != 0 && old != (unsigned long long)raw) flags |= MARK_MIXED;
   }
@@ -690,16 +693,18 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 3) split_cells_kernel(Ctrl* ctr
   }
   flush();
   if (FORM == FORM_FLOAT && !PAIRS) {
-    flags = __reduce_or_sync(0xFFFFFFFFu, flags);
-    if ((tid & 31) == 0 && flags) atomicOr(&sh_marks.flags, flags);
-    __syncthreads();
-    if (tid == 0) {
-      flags = sh_marks.flags;
-      if (sh_marks.nan != 0) {
-        const unsigned long long old = atomicCAS(&L.marks->nan, 0ull, sh_marks.nan);
-        if (old != 0 && old != sh_marks.nan) flags |= MARK_MIXED;
+    if (__syncthreads_or(flags)) {
+      flags = __reduce_or_sync(0xFFFFFFFFu, flags);
+      if ((tid & 31) == 0 && flags) atomicOr(&sh_marks.flags, flags);
+      __syncthreads();
+      if (tid == 0) {
+        flags = sh_marks.flags;
+        if (sh_marks.nan != 0) {
+          const unsigned long long old = atomicCAS(&L.marks->nan, 0ull, sh_marks.nan);
+          if (old != 0 && old != sh_marks.nan) flags |= MARK_MIXED;
+        }
+        atomicOr(&L.marks->flags, flags);
       }
-      if (flags & ~ld_relaxed(&L.marks->flags)) atomicOr(&L.marks->flags, flags);
     }
   }
 }

@@ -48,7 +48,7 @@ struct SplitLeaf {
 };
 
 // Bit patterns among the float keys of a sort without positions whose image stands for several.
-enum : unsigned int { MARK_ZERO = 1, MARK_NEG_ZERO = 2, MARK_NAN = 4 /* the canonical one */, MARK_MIXED = 8 /* several others */ };
+enum : unsigned int { MARK_ZERO = 1, MARK_NEG_ZERO = 2, MARK_NAN = 4 /* the canonical one */, MARK_MIXED = 8 /* several others */, MARK_OTHER = 16 /* others */ };
 struct SplitMarks {
   unsigned long long nan;  // NaNs of another pattern; 0: none
   unsigned int flags;
